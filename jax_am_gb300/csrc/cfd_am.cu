@@ -9,15 +9,15 @@
 //
 // BiCGSTAB follows jax.scipy.sparse.linalg.bicgstab (preconditioned
 // van der Vorst with JAX's stopping rule |r|^2 <= max(tol^2 |b|^2, atol^2),
-// its early exit on |s|^2 and its breakdown codes).  One iteration is six
-// launches: two elementwise updates, two stencil applications with fused dot
-// products, one elementwise update with two fused dot products, and a
-// single-block scalar step that advances rho, alpha, omega, k and the stop
-// flag.  Dot products are per-block partial sums reduced in a fixed order, so
-// results do not depend on scheduling.  The host enqueues iterations in
-// chunks and reads the stop flag after each chunk; launches after the stop
-// return at once, so the iteration count is exactly JAX's.  No kernel waits
-// on another.
+// its early exit on |s|^2 and its breakdown codes).  A system whose vectors
+// fit the SMs (up to about 311,000 cells: the flow box of every driver) is
+// solved in one cooperative launch (k_solve).  Larger ones take five launches
+// an iteration: two elementwise updates, two stencil applications with fused
+// dot products, and one update that also does the scalar step; the host
+// enqueues them in chunks and reads the stop flag after each chunk (launches
+// after the stop return at once, so the iteration count is exactly JAX's).
+// Dot products are per-block partial sums reduced in a fixed order, the same in
+// both forms, so results do not depend on scheduling or on the form.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -174,6 +174,7 @@ struct Work {
   double* velL;  // 3 nL (flow step)
   double* P;     // kSlots * kMaxBlocks partials
   KState* st;
+  struct SolveTail* tail;
 };
 
 // Blocks for n cells: about four cells per thread, at most four blocks per
@@ -379,8 +380,443 @@ __global__ void k_e(long long n, KState* st, double* P, double* x, double* r, co
   }
 }
 
+// ---- a whole solve in one launch ---------------------------------------------
+// Small systems (the flow box: 288,144 cells in the standalone driver's case)
+// spend the five launches of an iteration on launch latency, on re-reading
+// the vectors from L2 and on reduction trees.  Here one cooperative launch
+// runs the solve: a thread owns its cells from start to end and keeps their x,
+// r, rhat, p, q, s and t on the SM; only phat and shat, which the stencil
+// reads at neighbouring cells, go through memory (L2).
+//
+// Results are those of the kernels above, bit for bit: a thread owns the
+// cells it owns there (two of their 256-thread blocks per block, grid-stride),
+// and every sum is added in the same order -- within a warp by halving
+// offsets, then over the eight warps, then over the blocks.  The trees are
+// evaluated packed, with one addition per level on several sums at a time (the
+// lanes that a halving tree leaves idle carry another sum): a float64 addition
+// takes the pipe 16 cycles per warp whatever its active lanes.
+//
+// Three more warps do the waiting, one per sum: they add the warps' sums, post
+// the block's partials, collect everybody's, add them (every block does, in the
+// same order) and hand the scalars to the 16 working warps, which meanwhile
+// run what does not need them (the x update, the products of <s, s>).
+// A partial is one 16-byte word of value and sequence number, and so is every
+// cell of phat and shat: a reader waits on the word that it needs, so a dot
+// product and an exchange cost one trip through L2 each, with no flags, fences
+// or atomics.
+//
+// Bound: the float64 pipe (27 float64 operations per cell and iteration, 2
+// lanes a clock per SM: 2119 warp instructions of 16 cycles per SM and
+// iteration, 65 % of the time).  The driver's pressure solve (767 iterations)
+// takes 25 us an iteration against 47 us with the five launches.
+//
+// The blocks wait on one another, so the launch is cooperative (all of them
+// resident, at most one per SM), and each wait is bounded: one that runs out
+// sets the abort word, and every block returns.
+constexpr int kSolveCells = 4;      // cells per thread, at most
+constexpr int kSolveWork = 512;     // working threads: two 256-thread blocks of the kernels above
+constexpr int kSolveThreads = kSolveWork + 96;
+constexpr int kSolveBlocks = 320;   // 256-thread blocks of the reduction order, at most
+constexpr long long kSolveWaitCycles = 4000000000LL;  // about two seconds
+constexpr int kTailAt = 192;  // bytes of the 256-byte reserve that the solver state may take
+
+struct SolveTail {   // behind the solver state, in its reserve
+  double norm;       // Newton residual norm^2
+  int abort, pad;
+  long long k[4];    // iteration counts of the step's solves
+};
+static_assert(sizeof(KState) <= kTailAt && kTailAt + sizeof(SolveTail) <= 256,
+              "solver state and tail outgrew their reserve");
+
+struct __align__(16) Posted {  // a partial sum and the number of its reduction
+  double value;
+  unsigned long long seq;
+};
+struct SolveBoard {  // in the partial-sum area; zeroed before each solve
+  // <rhat, q>; <s, s>, <t, s>, <t, t>; <r, r>, <rhat, r>.  A block may be one
+  // reduction ahead of another that still reads its last partial, so the three
+  // reductions of an iteration have places of their own.
+  Posted part[6][kSolveBlocks];
+};
+static_assert(sizeof(SolveBoard) + 16 <= sizeof(double) * kSlots * kMaxBlocks,
+              "board outgrew its area");
+
+struct SolveArgs {
+  int nx, ny, nz, n;
+  int nb;              // 256-thread blocks of the reduction order
+  const double* diag;  // n own coefficients, or NULL: diag0 everywhere
+  const double* rows;  // six planes of n neighbour coefficients, or NULL: off[] everywhere
+  double diag0, off[6];
+  const double* dinv;  // Jacobi reciprocals or NULL
+  const double* b;
+  double* x;
+  Posted* phat;
+  Posted* shat;
+  SolveBoard* board;
+  SolveTail* tail;
+  long long* k_out;
+  double tol, atol;
+  long long maxiter;
+};
+
+// One level of a packed tree: value a goes on in the lanes without bit o, b in
+// those with it.
+__device__ __forceinline__ double fold(double a, double b, int o, int lane) {
+  const bool up = lane & o;
+  return (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, o);
+}
+
+// Sums over the warp of D values per lane (D = 1, 2 or 3), by offsets 16, 8,
+// .. 1; value i ends in the lane sum_lane<D>(i) (and those below it).
+template <int D>
+__device__ __forceinline__ double warp_sums(const double (&v)[D], int lane) {
+  double t;
+  if constexpr (D == 1) {
+    t = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+    t += __shfl_xor_sync(0xffffffffu, t, 8);
+  } else if constexpr (D == 2) {
+    t = fold(v[0], v[1], 16, lane);
+    t += __shfl_xor_sync(0xffffffffu, t, 8);
+  } else {
+    const double u = v[2] + __shfl_xor_sync(0xffffffffu, v[2], 16);
+    t = fold(fold(v[0], v[1], 16, lane), u, 8, lane);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+template <int D>
+__device__ __forceinline__ int sum_lane(int i) {
+  return D == 1 ? 0 : (i == 2 ? 8 : 16 * i);
+}
+
+// Named barriers between the working warps and the waiting ones.
+enum { kBarSums = 1, kBarTotals, kBarGo, kBarNext };
+template <int COUNT>
+__device__ __forceinline__ void bar_arrive(int id) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(COUNT) : "memory");
+}
+template <int COUNT>
+__device__ __forceinline__ void bar_wait(int id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(COUNT) : "memory");
+}
+
+__device__ __forceinline__ void post(Posted* p, double value, unsigned long long seq) {
+  asm volatile(
+      "{ .reg .b128 v; mov.b128 v, {%1, %2}; st.relaxed.gpu.global.b128 [%0], v; }" ::"l"(p),
+      "l"(__double_as_longlong(value)), "l"(seq)
+      : "memory");
+}
+__device__ __forceinline__ bool posted(const Posted* p, unsigned long long seq, double& value) {
+  long long v;
+  unsigned long long s;
+  asm volatile("{ .reg .b128 v; ld.relaxed.gpu.global.b128 v, [%2]; mov.b128 {%0, %1}, v; }"
+               : "=l"(v), "=l"(s)
+               : "l"(p)
+               : "memory");
+  value = __longlong_as_double(v);
+  return s == seq;
+}
+
+// ---- the waiting warps
+struct SolveShared {
+  double sums[3][2][8];  // the warps' sums: value, half, warp
+  double total[3];
+  double alpha, omega, beta;
+  int stop, early;
+  int late;  // a working warp's wait ran out
+};
+
+__device__ __forceinline__ bool solve_late(const SolveArgs& a, bool& late, long long t0) {
+  if (clock64() - t0 < kSolveWaitCycles) return false;
+  atomicExch(&a.tail->abort, 1);
+  late = true;
+  return true;
+}
+
+// Waiting warp i: value i of D sums (places PART ..).  The warps' sums of this
+// block, posted; then everybody's, added as total() adds them: a thread of 256
+// takes every 256th, then the block's tree.  False, in all three waiting warps,
+// when a wait of theirs ran out.
+template <int D, int PART>
+__device__ __forceinline__ bool solve_reduce(const SolveArgs& a, SolveShared& sh,
+                                             unsigned long long seq, int i, int lane,
+                                             bool& late) {
+  bar_wait<kSolveThreads>(kBarSums);
+  if (sh.late) late = true;
+  if (i < D) {
+    Posted* part = a.board->part[PART + i];
+    const int half = (lane >> 3) & 1, vb = 2 * (int)blockIdx.x + half;
+    double s = sh.sums[i][half][lane & 7];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((lane & 23) == 0 && vb < a.nb) post(part + vb, s, seq);
+    constexpr int kParts = kSolveBlocks / 32;
+    static_assert(kParts >= 8 && kParts <= 16, "a thread of 256 takes one or two partials");
+    double v[kParts];
+    const long long t0 = clock64();
+    bool all;
+    do {
+      all = true;
+#pragma unroll
+      for (int w = 0; w < kParts; ++w) {
+        v[w] = 0.0;
+        if (w * 32 + lane < a.nb) all &= posted(part + w * 32 + lane, seq, v[w]);
+      }
+    } while (!__all_sync(0xffffffffu, all || solve_late(a, late, t0)));
+#pragma unroll
+    for (int w = 8; w < kParts; ++w)
+      if (w * 32 < a.nb) v[w - 8] += v[w];
+    // eight warps' trees at a time: warp w ends in the lanes whose bits 4, 3
+    // and 2 are bits 0, 1 and 2 of w
+    double t = fold(fold(fold(v[0], v[1], 16, lane), fold(v[2], v[3], 16, lane), 8, lane),
+                    fold(fold(v[4], v[5], 16, lane), fold(v[6], v[7], 16, lane), 8, lane), 4,
+                    lane);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    t += __shfl_xor_sync(0xffffffffu, t, 4);   // w and w + 4
+    t += __shfl_xor_sync(0xffffffffu, t, 8);   // w + 2
+    t += __shfl_xor_sync(0xffffffffu, t, 16);  // w + 1
+    if (lane == 0) sh.total[i] = t;
+  }
+  int any;
+  asm volatile(
+      "{ .reg .pred p, q; setp.ne.s32 p, %1, 0; bar.red.or.pred q, %2, 96, p; selp.s32 %0, 1, 0, q; }"
+      : "=r"(any)
+      : "r"((int)late), "r"((int)kBarTotals)
+      : "memory");
+  return any == 0;
+}
+
+__device__ __forceinline__ void solve_wait(const SolveArgs& a, SolveShared& sh, int i, int lane) {
+  double rho = 1.0, alpha = 1.0, omega = 1.0, rho_new = 0.0, atol2 = 0.0;
+  long long it = 0;
+  unsigned long long seq = 0;
+  bool late = false;
+  bool ok = solve_reduce<1, 4>(a, sh, ++seq, i, lane, late);
+  __threadfence();  // every block has cleared its words of phat and shat
+  if (i == 0) {
+    const double bs = sh.total[0];
+    const double a2 = a.tol * a.tol * bs, b2 = a.atol * a.atol;
+    atol2 = a2 > b2 ? a2 : b2;
+    rho_new = bs;
+    if (lane == 0) sh.stop = !ok || !(bs > atol2 && 0 < a.maxiter);
+  }
+  for (;;) {
+    if (i == 0) {
+      if (lane == 0) {
+        sh.beta = rho_new / rho * alpha / omega;
+        sh.omega = omega;
+      }
+      __syncwarp();
+      bar_arrive<kSolveWork + 32>(kBarGo);
+    }
+    bar_wait<96>(kBarNext);
+    if (sh.stop) break;
+    ok = solve_reduce<1, 0>(a, sh, ++seq, i, lane, late);
+    if (i == 0) {
+      alpha = rho_new / sh.total[0];
+      if (lane == 0) {
+        sh.alpha = alpha;
+        if (!ok) sh.stop = 1;
+      }
+      __syncwarp();
+      bar_arrive<kSolveWork + 32>(kBarGo);
+    }
+    if (!ok) break;
+    ok = solve_reduce<3, 1>(a, sh, ++seq, i, lane, late);  // <s, s>, <t, s>, <t, t>
+    if (i == 0) {
+      omega = sh.total[1] / sh.total[2];
+      if (lane == 0) {
+        sh.omega = omega;
+        sh.early = sh.total[0] < atol2;
+        if (!ok) sh.stop = 1;
+      }
+      __syncwarp();
+      bar_arrive<kSolveWork + 32>(kBarGo);
+    }
+    if (!ok) break;
+    ok = solve_reduce<2, 4>(a, sh, ++seq, i, lane, late);  // <r, r>, <rhat, r>
+    if (i == 0) {
+      it = (omega == 0.0 || alpha == 0.0) ? -11 : it + 1;
+      if (rho_new == 0.0) it = -10;
+      rho = rho_new;
+      rho_new = sh.total[1];
+      if (lane == 0) sh.stop = !ok || !(sh.total[0] > atol2 && it < a.maxiter && it >= 0);
+    }
+  }
+  if (blockIdx.x == 0 && i == 0 && lane == 0) *a.k_out = it;
+}
+
+// ROWS: neighbour coefficients per cell; PREC: Jacobi reciprocals.
+template <bool ROWS, bool PREC>
+__global__ void __launch_bounds__(kSolveThreads, 1) k_solve(const __grid_constant__ SolveArgs a) {
+  __shared__ SolveShared sh;
+  // off the critical path, and 19 warps leave a thread 96 registers
+  __shared__ double x[kSolveCells][kSolveWork], rhat[kSolveCells][kSolveWork];
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) sh.late = 0;
+  __syncthreads();
+  if (threadIdx.x >= kSolveWork) {
+    solve_wait(a, sh, (threadIdx.x - kSolveWork) >> 5, lane);
+    return;
+  }
+
+  // ---- the working warps
+  const int warp = (threadIdx.x >> 5) & 7, half = threadIdx.x >> 8;
+  const int stride = a.nb * kThreads;
+  const int vb = 2 * (int)blockIdx.x + half;
+  const int c0 = vb * kThreads + (threadIdx.x & 255);
+  const int off[6] = {-a.ny * a.nz, a.ny * a.nz, -a.nz, a.nz, -1, 1};
+  unsigned inner = 0;  // six bits per cell: the neighbour exists (else the cell itself)
+  bool on[kSolveCells];
+  double r[kSolveCells], p[kSolveCells], q[kSolveCells], s[kSolveCells], t[kSolveCells];
+  const int me = threadIdx.x;
+  auto put = [&](const auto& v) {  // this warp's sums of D values
+    constexpr int D = sizeof(v) / sizeof(double);
+    const double u = warp_sums<D>(v, lane);
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+      if (lane == sum_lane<D>(i)) sh.sums[i][half][warp] = u;
+    bar_arrive<kSolveThreads>(kBarSums);
+  };
+  unsigned long long turn = 0;  // the iteration: the number of its phat and shat
+  double bb[1] = {0.0};
+#pragma unroll
+  for (int k = 0; k < kSolveCells; ++k) {
+    const int c = c0 + k * stride;
+    on[k] = vb < a.nb && c < a.n;
+    const double v = on[k] ? a.b[c] : 0.0;
+    x[k][me] = 0.0;
+    rhat[k][me] = v;
+    r[k] = p[k] = q[k] = v;
+    s[k] = t[k] = 0.0;
+    if (on[k]) {
+      bb[0] += v * v;
+      const int row = c / a.nz, kz = c - row * a.nz, i = row / a.ny, j = row - i * a.ny;
+      const unsigned m = (i > 0 ? 1u : 0u) | (i < a.nx - 1 ? 2u : 0u) | (j > 0 ? 4u : 0u) |
+                         (j < a.ny - 1 ? 8u : 0u) | (kz > 0 ? 16u : 0u) |
+                         (kz < a.nz - 1 ? 32u : 0u);
+      inner |= m << (8 * k);
+      post(a.phat + c, 0.0, 0);  // what an earlier solve left may carry our numbers
+      post(a.shat + c, 0.0, 0);
+    }
+  }
+  __threadfence();
+  auto hat = [&](double v, int k) {  // M v
+    return PREC ? __ldg(a.dinv + c0 + k * stride) * v : v;
+  };
+  // A u at cell k, u0 its own value: the products of the cell and of its first
+  // neighbour fused as the compiler fuses apply_row's (u0's inside the fma)
+  auto row = [&](const Posted* u, double u0, int k) {
+    const int c = c0 + k * stride;
+    double nbv[6], w[6];
+    long long since = 0;
+    for (;;) {
+      bool all = true;
+#pragma unroll
+      for (int f = 0; f < 6; ++f)
+        all &= posted(u + c + ((inner >> (8 * k + f)) & 1u ? off[f] : 0), turn, nbv[f]);
+      if (all) break;
+      bool late = false;
+      if (since == 0) since = clock64();
+      else if (solve_late(a, late, since)) {
+        *(volatile int*)&sh.late = 1;
+        break;
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < 6; ++f) w[f] = ROWS ? __ldg(a.rows + (long long)f * a.n + c) : a.off[f];
+    double acc = __fma_rn(a.diag ? __ldg(a.diag + c) : a.diag0, u0, __dmul_rn(w[0], nbv[0]));
+#pragma unroll
+    for (int f = 1; f < 6; ++f) acc = __fma_rn(w[f], nbv[f], acc);
+    return acc;
+  };
+  put(bb);
+  bar_wait<kSolveWork + 32>(kBarGo);
+  while (!sh.stop) {
+    {  // p = r + beta (p - omega q); phat = M p
+      const double beta = sh.beta, om = sh.omega;
+      ++turn;
+#pragma unroll
+      for (int k = 0; k < kSolveCells; ++k)
+        if (on[k]) {
+          p[k] = r[k] + beta * (p[k] - om * q[k]);
+          post(a.phat + c0 + k * stride, hat(p[k], k), turn);
+        }
+    }
+    {  // q = A phat; <rhat, q>
+      double rq[1] = {0.0};
+#pragma unroll
+      for (int k = 0; k < kSolveCells; ++k)
+        if (on[k]) {
+          q[k] = row(a.phat, hat(p[k], k), k);
+          rq[0] += rhat[k][me] * q[k];
+        }
+      put(rq);
+    }
+    bar_wait<kSolveWork + 32>(kBarGo);
+    if (sh.stop) break;
+    const double al = sh.alpha;
+    // s = r - alpha q; shat = M s
+#pragma unroll
+    for (int k = 0; k < kSolveCells; ++k)
+      if (on[k]) {
+        s[k] = r[k] - al * q[k];
+        post(a.shat + c0 + k * stride, hat(s[k], k), turn);
+      }
+    double d[3] = {0.0, 0.0, 0.0};  // <s, s>, <t, s>, <t, t>
+#pragma unroll
+    for (int k = 0; k < kSolveCells; ++k)
+      if (on[k]) d[0] += s[k] * s[k];
+    // t = A shat
+#pragma unroll
+    for (int k = 0; k < kSolveCells; ++k)
+      if (on[k]) {
+        t[k] = row(a.shat, hat(s[k], k), k);
+        d[1] += t[k] * s[k];
+        d[2] += t[k] * t[k];
+      }
+    put(d);
+    bar_wait<kSolveWork + 32>(kBarGo);
+    if (sh.stop) break;
+    {  // r (early exit when <s, s> is below the tolerance); <r, r>, <rhat, r>
+      const double om = sh.omega;
+      const bool early = sh.early;  // the same in every thread
+      double e[2] = {0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < kSolveCells; ++k)
+        if (on[k]) {
+          r[k] = early ? s[k] : s[k] - om * t[k];
+          e[0] += r[k] * r[k];
+          e[1] += rhat[k][me] * r[k];
+        }
+      put(e);
+      if (early) {
+#pragma unroll
+        for (int k = 0; k < kSolveCells; ++k)
+          if (on[k]) x[k][me] = __fma_rn(al, hat(p[k], k), x[k][me]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < kSolveCells; ++k)
+          if (on[k]) x[k][me] += __fma_rn(al, hat(p[k], k), __dmul_rn(om, hat(s[k], k)));
+      }
+    }
+    bar_wait<kSolveWork + 32>(kBarGo);
+  }
+#pragma unroll
+  for (int k = 0; k < kSolveCells; ++k)
+    if (on[k]) a.x[c0 + k * stride] = x[k][me];
+}
+
 static cudaError_t read_state(const KState* dst, KState* host, cudaStream_t s) {
   cudaError_t e = cudaMemcpyAsync(host, dst, sizeof(KState), cudaMemcpyDeviceToHost, s);
+  if (e != cudaSuccess) return e;
+  return cudaStreamSynchronize(s);
+}
+
+static cudaError_t read_tail(const SolveTail* dst, SolveTail* host, cudaStream_t s) {
+  cudaError_t e = cudaMemcpyAsync(host, dst, sizeof(SolveTail), cudaMemcpyDeviceToHost, s);
   if (e != cudaSuccess) return e;
   return cudaStreamSynchronize(s);
 }
@@ -451,6 +887,55 @@ static cudaGraphExec_t chunk_graph(const Dims& d, const double* vals, const doub
   g_graph_execs[g_graph_count] = exec;
   ++g_graph_count;
   return exec;
+}
+
+// Whether k_solve takes a system of n cells: its reduction order has at most
+// two 256-thread blocks per SM, with at most kSolveCells cells per thread.
+// Above that the per-iteration launches are the better ones: the vectors no
+// longer fit the registers of one wave of blocks.
+static bool solve_fits(long long n) {
+  const long long nb = nblocks(n);
+  return nb <= std::min(2LL * device_info().sm_count, (long long)kSolveBlocks) &&
+         n <= nb * kThreads * kSolveCells;
+}
+
+// Enqueue k_solve: x = 0 start, k lands in tail->k[slot] (no host wait).
+static int solve_resident(const Dims& d, const double* diag, double diag0, const double* rows,
+                          const double* off, const double* dinv, const double* b, double* x,
+                          double tol, double atol, long long maxiter, const Work& w, int slot,
+                          cudaStream_t s) {
+  SolveArgs a{};
+  a.nx = d.nx;
+  a.ny = d.ny;
+  a.nz = d.nz;
+  a.n = (int)d.n;
+  a.nb = nblocks(d.n);
+  a.diag = diag;
+  a.diag0 = diag0;
+  a.rows = rows;
+  for (int f = 0; f < 6; ++f) a.off[f] = off ? off[f] : 0.0;
+  a.dinv = dinv;
+  a.b = b;
+  a.x = x;
+  // phat, q, s, shat and t lie one behind the other: the two arrays of 16-byte
+  // words take four of them, aligned
+  a.phat = reinterpret_cast<Posted*>(((uintptr_t)w.phat + 15) & ~(uintptr_t)15);
+  a.shat = a.phat + d.n;
+  a.board = reinterpret_cast<SolveBoard*>(((uintptr_t)w.P + 15) & ~(uintptr_t)15);
+  a.tail = w.tail;
+  a.k_out = &w.tail->k[slot];
+  a.tol = tol;
+  a.atol = atol;
+  a.maxiter = maxiter;
+  cudaError_t e = cudaMemsetAsync(a.board, 0, sizeof(SolveBoard), s);
+  if (e != cudaSuccess) return record_cuda(e);
+  void* args[] = {&a};
+  const void* fn = rows ? (const void*)k_solve<true, true>
+                   : dinv ? (const void*)k_solve<false, true>
+                          : (const void*)k_solve<false, false>;
+  e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)((a.nb + 1) / 2)), dim3(kSolveThreads), args,
+                                  0, s);
+  return e == cudaSuccess ? PFG_OK : record_cuda(e);
 }
 
 // Solve vals x = b (dinv: Jacobi reciprocals or NULL); *iters = JAX's k.
@@ -618,7 +1103,7 @@ __device__ __forceinline__ double fluid_frac(double T, double Ts, double Tl) {
 // (cfd_am.py:530-536, 426-472, solver_linear :748-778)
 __global__ void k_momentum(Dims d, FlowK F, int comp, const double* T, const double* vel0,
                            const double* conv, const double* gp, double* b, double* vals,
-                           double* diag) {
+                           double* diag, bool rows) {
   const pfg_cfd_flow& f = F.f;
   GRID_LOOP(c, d.n) {
     int i, j, k;
@@ -647,7 +1132,7 @@ __global__ void k_momentum(Dims d, FlowK F, int comp, const double* T, const dou
       const double gq = d.g[q];
       v0 += gq * f.visco;
       const double vq = -gq * f.visco;
-      vals[(1 + q) * d.n + c] = vq;
+      if (rows) vals[(1 + q) * d.n + c] = vq;
       if (on_face(d, i, j, k, q)) {
         dg += vq;
         // Dirichlet walls: all faces but the top for u and v (cfd_am.py:304-310)
@@ -823,6 +1308,7 @@ static bool carve(void* ws, int64_t bytes, long long n, long long nl, Work& w) {
   w.velL = p; p += 3 * nl;
   w.P = p; p += (long long)kSlots * kMaxBlocks;
   w.st = reinterpret_cast<KState*>(p);
+  w.tail = reinterpret_cast<SolveTail*>(p + kTailAt / 8);
   return true;
 }
 
@@ -861,36 +1347,41 @@ extern "C" int pfg_cfd_energy_solve(const pfg_cfd_grid* g, const pfg_cfd_energy*
   K.Ly = g->ly;
   K.Lz = g->lz;
   const int nb = nblocks(n);
-  // the Newton residual norm^2 sits after the solver state, inside the 256-byte reserve
-  static_assert(sizeof(KState) <= 192, "solver state outgrew its reserve");
-  double* norm = reinterpret_cast<double*>(w.st) + 24;
+  double* norm = &w.tail->norm;
+  const bool resident = solve_fits(n);
+  cudaError_t ce = cudaMemsetAsync(w.tail, 0, sizeof(SolveTail), s);
+  if (ce != cudaSuccess) return record_cuda(ce);
   k_copy<<<nb, kThreads, 0, s>>>(n, T0, T_out);
   k_energy_residual<<<nb, kThreads, 0, s>>>(d, K, T_out, T0, conv_T, w.b, w.P);
   k_norm<<<1, kThreads, 0, s>>>(w.P, nb, norm);
-  cudaError_t ce = cudaGetLastError();
+  ce = cudaGetLastError();
   if (ce != cudaSuccess) return record_cuda(ce);
-  double bb0 = 0.0;
-  ce = cudaMemcpyAsync(&bb0, norm, sizeof(double), cudaMemcpyDeviceToHost, s);
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+  SolveTail h{};
+  ce = read_tail(w.tail, &h, s);
   if (ce != cudaSuccess) return record_cuda(ce);
-  const double res_init = std::sqrt(bb0);
-  double bb = bb0;
+  const double res_init = std::sqrt(h.norm);
+  double bb = h.norm;
   int it = 0;
   long long lin = 0;
   while (std::sqrt(bb) / res_init > e->newton_tol && it < e->max_newton) {
     k_energy_jacobian<<<nb, kThreads, 0, s>>>(d, K, T_out, T0, w.vals, w.diag);
     long long k = 0;
-    st = krylov(d, w.vals, w.diag, w.b, w.x, 1e-5, 0.0, 10 * n, w, s, &k);
+    if (resident)
+      st = solve_resident(d, w.vals, 0.0, w.vals + n, nullptr, w.diag, w.b, w.x, 1e-5, 0.0, 10 * n,
+                          w, 0, s);
+    else
+      st = krylov(d, w.vals, w.diag, w.b, w.x, 1e-5, 0.0, 10 * n, w, s, &k);
     if (st) return st;
-    lin += k;
     k_axpy<<<nb, kThreads, 0, s>>>(n, T_out, w.x);
     k_energy_residual<<<nb, kThreads, 0, s>>>(d, K, T_out, T0, conv_T, w.b, w.P);
     k_norm<<<1, kThreads, 0, s>>>(w.P, nb, norm);
     ce = cudaGetLastError();
     if (ce != cudaSuccess) return record_cuda(ce);
-    ce = cudaMemcpyAsync(&bb, norm, sizeof(double), cudaMemcpyDeviceToHost, s);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+    ce = read_tail(w.tail, &h, s);
     if (ce != cudaSuccess) return record_cuda(ce);
+    if (h.abort) return PFG_ERR_TIMEOUT;
+    bb = h.norm;
+    lin += resident ? h.k[0] : k;
     ++it;
   }
   if (stats) {
@@ -938,21 +1429,50 @@ extern "C" int pfg_cfd_flow_step(const pfg_cfd_grid* global, const pfg_cfd_grid*
   F.ldx = local->dx;
   F.ldy = local->dy;
   const int nb = nblocks(nl);
+  const bool resident = solve_fits(nl);
+  // the neighbour coefficients are the same in every cell
+  double off_m[6], off_p[6], diag_p = 0.0;
+  for (int q = 0; q < 6; ++q) {
+    off_m[q] = -d.g[q] * f->visco;
+    off_p[q] = -d.g[q];
+    diag_p += d.g[q];
+  }
+  cudaError_t ce = cudaMemsetAsync(w.tail, 0, sizeof(SolveTail), s);
+  if (ce != cudaSuccess) return record_cuda(ce);
+  SolveTail h{};
   for (int comp = 0; comp < 3; ++comp) {
-    k_momentum<<<nb, kThreads, 0, s>>>(d, F, comp, T, vel, conv, grad_p0, w.b, w.vals, w.diag);
-    long long k = 0;
-    st = krylov(d, w.vals, w.diag, w.b, w.velL + comp * nl, 1e-10, 0.0, 10000, w, s, &k);
+    double* u = w.velL + comp * nl;
+    k_momentum<<<nb, kThreads, 0, s>>>(d, F, comp, T, vel, conv, grad_p0, w.b, w.vals, w.diag,
+                                       !resident);
+    if (resident)
+      st = solve_resident(d, w.vals, 0.0, nullptr, off_m, w.diag, w.b, u, 1e-10, 0.0, 10000, w,
+                          comp, s);
+    else
+      st = krylov(d, w.vals, w.diag, w.b, u, 1e-10, 0.0, 10000, w, s, &h.k[comp]);
     if (st) return st;
-    if (stats) stats->momentum_krylov[comp] = k;
   }
   k_pressure_rhs<<<nb, kThreads, 0, s>>>(d, F, w.velL, w.b, local->dz);
-  k_pressure_vals<<<nb, kThreads, 0, s>>>(d, w.vals);
-  long long k = 0;
-  st = krylov(d, w.vals, nullptr, w.b, w.x, 1e-10, 0.0, 10000, w, s, &k);
+  if (resident) {
+    st = solve_resident(d, nullptr, diag_p, nullptr, off_p, nullptr, w.b, w.x, 1e-10, 0.0, 10000,
+                        w, 3, s);
+  } else {
+    k_pressure_vals<<<nb, kThreads, 0, s>>>(d, w.vals);
+    st = krylov(d, w.vals, nullptr, w.b, w.x, 1e-10, 0.0, 10000, w, s, &h.k[3]);
+  }
   if (st) return st;
-  if (stats) stats->pressure_krylov = k;
   k_project<<<nb, kThreads, 0, s>>>(d, F, w.x, w.velL, vel, grad_p0, local->dz);
   k_convective<<<nb, kThreads, 0, s>>>(d, F, global->dx, global->dy, global->dz, T, vel, conv_T,
                                        conv);
-  return record_cuda(cudaGetLastError());
+  ce = cudaGetLastError();
+  if (ce != cudaSuccess) return record_cuda(ce);
+  if (resident) {  // the one host wait of the step
+    ce = read_tail(w.tail, &h, s);
+    if (ce != cudaSuccess) return record_cuda(ce);
+    if (h.abort) return PFG_ERR_TIMEOUT;
+  }
+  if (stats) {
+    for (int comp = 0; comp < 3; ++comp) stats->momentum_krylov[comp] = h.k[comp];
+    stats->pressure_krylov = h.k[3];
+  }
+  return PFG_OK;
 }

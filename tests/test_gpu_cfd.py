@@ -228,3 +228,32 @@ def test_am3d_edge_shapes(N, NL, heat_source):
         for f in FIELDS:
             ok, err, scale = close(getattr(s, f), getattr(o, f), 1e-7)
             assert ok, (N, NL, step, f, err, scale)
+
+
+@pytest.mark.parametrize("N,NL,cells_per_thread", [
+    ([16, 8, 8], [16, 8, 8], 4),     # 1024 cells: one whole block
+    ([18, 9, 7], [16, 9, 7], 4),     # two blocks; one block of 1008 cells
+    ([17, 11, 11], [13, 11, 9], 4),  # three blocks (half a CTA idle); two
+    ([17, 11, 11], [13, 11, 9], 8),  # more cells per thread: a launch per operation
+])
+def test_am3d_solver_block_edges(N, NL, cells_per_thread):
+    """The one-launch solve at the edges of its blocks, and the launches per
+    operation that larger systems take, against the oracle: two steps."""
+    from jax_am_gb300 import _lib
+    h = 5e-6
+    args = dict(CASES["surface"], P=40.0, speed=2.5, X0=[4e-5, 3e-5, N[2] * h])
+    cp, k = (0.2441, 338.39, 300.0, 1563.0), (0.0163105, 4.5847, 300.0, 1563.0)
+    lib = _lib.load()
+    assert lib.pfg_tune(6, cells_per_thread) == 0
+    try:
+        s = gpu_solver(args, N, NL, h, cp, k)
+        o = oracle_solver(args, N, NL, h, cp, k)
+        for step in range(2):
+            s.time_integration()
+            o.time_integration()
+            torch.cuda.synchronize()
+            for f in FIELDS:
+                ok, err, scale = close(getattr(s, f), getattr(o, f), 1e-7)
+                assert ok, (N, NL, step, f, err, scale)
+    finally:
+        lib.pfg_tune(6, 0)
