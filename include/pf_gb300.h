@@ -424,6 +424,10 @@ int64_t pfg_grain_scratch_bytes(const pfg_pf_params* p);
 int pfg_grains(const pfg_pf_params* p, const int32_t* ori, const float* T, int T_ghosted,
                int32_t* grain_of_cell, pfg_grain* grains, int64_t max_grains, int64_t* num_grains,
                void* scratch, int64_t scratch_bytes, void* stream);
+/* Renumber a grain_of_cell array in place: labels[i] = rank[labels[i]], -1
+ * stays.  rank: device int32 per grain number (the caller's order of the
+ * records). */
+int pfg_grain_relabel(int64_t num_cells, const int32_t* rank, int32_t* labels, void* stream);
 
 /* ---- diagnostics ----------------------------------------------------------
  * The metrics PFSolver.inspect_sol prints (allen_cahn.py:165-180) plus the

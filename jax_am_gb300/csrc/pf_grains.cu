@@ -8,19 +8,27 @@
 // cell index); each grain's volume and PCA aspect ratio follow from its cells'
 // centres.
 //
-// Here the components come from a lock-free union-find over the cell grid:
-//  1. every solid cell starts as its own root (liquid cells are -1);
-//  2. each solid cell unites with its +x, +y, +z neighbours of the same
-//     orientation (Playne and Hawick's merge: find both roots, hang the larger
-//     root under the smaller with atomicMin, retry if that root moved);
+// Here the components come from a two-level lock-free union-find:
+//  1. a block labels a tile of 32 x 8 x 8 cells in shared memory: a row's runs
+//     of one orientation come from a ballot, runs of adjacent rows unite
+//     (Playne and Hawick's merge: find both roots, hang the larger under the
+//     smaller with atomicMin, retry if that root moved) where they first touch;
+//     every cell's label is its tile root (-1 in liquid);
+//  2. the cells on tile faces unite their tiles' roots in global memory;
 //  3. every cell's label is replaced by its root.
 // A root is therefore the smallest cell index of its component -- the cell at
 // which the reference's search starts that grain.  Roots are then numbered in
-// increasing index order (a block-wise scan), and one pass adds each cell's
-// count and first and second coordinate moments into its grain's record
-// (exact 64-bit integers, aggregated per warp before the atomics).  The
-// caller orders the records by (orientation, first cell) to obtain the
-// reference's order, and computes volumes and aspect ratios from the moments.
+// increasing index order (a block-wise scan), and one pass adds each tile's
+// count and first and second coordinate moments into its grains' records
+// (exact integers: per run in closed form, per tile in shared memory, then one
+// 64-bit atomic per grain of the tile and moment).  The caller orders the
+// records by (orientation, first cell) to obtain the reference's order, and
+// computes volumes and aspect ratios from the moments.
+//
+// Bound: latency and L2.  A cell-by-cell merge in global memory took 2306 us of
+// 2946 us at 8M cells (1,500 grains: every cell of a grain chases and updates
+// the same few roots); within a tile the chains are short and in shared memory:
+// 330 us in all (tiles 168, faces 47, roots 33, moments 48).
 //
 // Termination: a label only ever decreases and never drops below its own
 // root's index, and a non-root always points to a smaller index, so every find
@@ -53,20 +61,42 @@ struct GrainArgs {
   int64_t* num_grains;
 };
 
+// Tiles: 32 cells along x (a warp's row), 8 along y and z.
+constexpr int kTileX = 32, kTileY = 8, kTileZ = 8;
+constexpr int kTileRows = kTileY * kTileZ, kTileCells = kTileX * kTileRows;
+static_assert(kGrainThreads == kTileY * 32, "a warp takes one y of every z plane of the tile");
+
+struct Tile {
+  int x0, y0, z0;
+};
+__device__ __forceinline__ Tile tile_of(const GrainArgs& a, int t) {
+  const int tx = (a.nx + kTileX - 1) / kTileX, ty = (a.ny + kTileY - 1) / kTileY;
+  const int q = t / tx;
+  return Tile{(t - q * tx) * kTileX, (q % ty) * kTileY, (q / ty) * kTileZ};
+}
+
+template <bool GLOBAL>
+__device__ __forceinline__ int load_label(const int32_t* L, int x) {
+  if constexpr (GLOBAL) return __ldcg(L + x);
+  else return *(volatile const int32_t*)(L + x);
+}
+
+template <bool GLOBAL>
 __device__ __forceinline__ int find_root(const int32_t* L, int x) {
-  int y = __ldcg(L + x);
+  int y = load_label<GLOBAL>(L, x);
   while (y != x) {
     x = y;
-    y = __ldcg(L + x);
+    y = load_label<GLOBAL>(L, x);
   }
   return x;
 }
 
+template <bool GLOBAL>
 __device__ __forceinline__ void merge(int32_t* L, int a, int b) {
   bool done;
   do {
-    a = find_root(L, a);
-    b = find_root(L, b);
+    a = find_root<GLOBAL>(L, a);
+    b = find_root<GLOBAL>(L, b);
     if (a < b) {
       const int old = atomicMin(L + b, a);
       done = (old == b);
@@ -81,39 +111,98 @@ __device__ __forceinline__ void merge(int32_t* L, int a, int b) {
   } while (!done);
 }
 
-__global__ void __launch_bounds__(kGrainThreads) grain_init_kernel(const GrainArgs a) {
-  const int N = a.nx * a.ny * a.nz;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    float T;
-    if (a.T_ghosted) {
-      const int xy = a.nx * a.ny;
-      const int z = i / xy, r = i - z * xy, y = r / a.nx, x = r - y * a.nx;
-      T = a.T[((int64_t)(z + 1) * (a.ny + 2) + (y + 1)) * (a.nx + 2) + x + 1];
-    } else {
-      T = a.T[i];
+// Labels of one tile: every cell's is the global index of its tile root.
+__global__ void __launch_bounds__(kGrainThreads) grain_tile_kernel(const GrainArgs a) {
+  __shared__ int32_t s_ori[kTileCells], s_L[kTileCells];
+  __shared__ unsigned s_start[kTileRows];  // where a row's runs start (liquid cells too)
+  const int lane = threadIdx.x & 31, yl = threadIdx.x >> 5;
+  const Tile t = tile_of(a, blockIdx.x);
+  const int x = t.x0 + lane, y = t.y0 + yl, xy = a.nx * a.ny;
+  const bool col = x < a.nx && y < a.ny;
+#pragma unroll
+  for (int zl = 0; zl < kTileZ; ++zl) {
+    const int z = t.z0 + zl, r = zl * kTileY + yl;
+    int o = 0;
+    bool solid = false;
+    if (col && z < a.nz) {
+      const int i = z * xy + y * a.nx + x;
+      const float T = a.T_ghosted
+                          ? a.T[((int64_t)(z + 1) * (a.ny + 2) + (y + 1)) * (a.nx + 2) + x + 1]
+                          : a.T[i];
+      o = a.ori[i];
+      solid = T < a.T_liq;  // NaN T is not solid, as in the reference's compare
     }
-    a.L[i] = (T < a.T_liq) ? i : -1;  // NaN T is not solid, as in the reference's compare
+    const int o_left = __shfl_up_sync(0xffffffffu, o, 1);
+    const unsigned solids = __ballot_sync(0xffffffffu, solid);
+    const bool joins = lane > 0 && solid && (solids >> (lane - 1) & 1u) && o == o_left;
+    const unsigned starts = ~__ballot_sync(0xffffffffu, joins);
+    const int head = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
+    s_ori[r * 32 + lane] = o;
+    s_L[r * 32 + lane] = solid ? r * 32 + head : -1;
+    if (lane == 0) s_start[r] = starts;
+  }
+  __syncthreads();
+  // Two rows' runs unite at the first cell of each overlap: where either run
+  // starts.
+#pragma unroll
+  for (int zl = 0; zl < kTileZ; ++zl) {
+    const int r = zl * kTileY + yl, c = r * 32 + lane;
+    if (s_L[c] < 0) continue;
+    if (yl > 0 && s_L[c - 32] >= 0 && s_ori[c - 32] == s_ori[c] &&
+        ((s_start[r] | s_start[r - 1]) >> lane & 1u))
+      merge<false>(s_L, c, c - 32);
+    if (zl > 0 && s_L[c - 32 * kTileY] >= 0 && s_ori[c - 32 * kTileY] == s_ori[c] &&
+        ((s_start[r] | s_start[r - kTileY]) >> lane & 1u))
+      merge<false>(s_L, c, c - 32 * kTileY);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int zl = 0; zl < kTileZ; ++zl) {
+    const int z = t.z0 + zl, c = (zl * kTileY + yl) * 32 + lane;
+    if (!col || z >= a.nz) continue;
+    int g = -1;
+    if (s_L[c] >= 0) {
+      const int q = find_root<false>(s_L, c);
+      g = (t.z0 + q / (32 * kTileY)) * xy + (t.y0 + q / 32 % kTileY) * a.nx + t.x0 + q % 32;
+    }
+    a.L[z * xy + y * a.nx + x] = g;
   }
 }
 
-__global__ void __launch_bounds__(kGrainThreads) grain_merge_kernel(const GrainArgs a) {
-  const int N = a.nx * a.ny * a.nz;
+// Unite across tile faces.  Along x, a face's pairs of cells unite one by one;
+// across y and z faces a pair whose left neighbours are a pair of the same two
+// tile components has nothing to add.
+__global__ void __launch_bounds__(kGrainThreads) grain_faces_kernel(const GrainArgs a) {
   const int xy = a.nx * a.ny;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    if (__ldcg(a.L + i) < 0) continue;
-    const int z = i / xy, r = i - z * xy, y = r / a.nx, x = r - y * a.nx;
-    const int o = a.ori[i];
-    if (x + 1 < a.nx && __ldcg(a.L + i + 1) >= 0 && a.ori[i + 1] == o) merge(a.L, i, i + 1);
-    if (y + 1 < a.ny && __ldcg(a.L + i + a.nx) >= 0 && a.ori[i + a.nx] == o)
-      merge(a.L, i, i + a.nx);
-    if (z + 1 < a.nz && __ldcg(a.L + i + xy) >= 0 && a.ori[i + xy] == o) merge(a.L, i, i + xy);
-  }
-}
-
-__global__ void __launch_bounds__(kGrainThreads) grain_compress_kernel(const GrainArgs a) {
-  const int N = a.nx * a.ny * a.nz;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    if (__ldcg(a.L + i) >= 0) a.L[i] = find_root(a.L, i);
+  const int64_t fx = (int64_t)((a.nx - 1) / kTileX) * a.ny * a.nz;
+  const int64_t fy = (int64_t)((a.ny - 1) / kTileY) * a.nx * a.nz;
+  const int64_t fz = (int64_t)((a.nz - 1) / kTileZ) * xy;
+  for (int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; f < fx + fy + fz;
+       f += (int64_t)gridDim.x * blockDim.x) {
+    int i, j, x;
+    if (f < fz) {
+      const int p = (int)(f / xy), r = (int)(f - (int64_t)p * xy);
+      i = (p + 1) * kTileZ * xy + r;
+      j = i - xy;
+      x = r % a.nx;
+    } else if (f < fz + fy) {
+      const int64_t g = f - fz;
+      const int row = (int)(g / a.nx), k = (a.ny - 1) / kTileY;
+      x = (int)(g - (int64_t)row * a.nx);
+      i = (row / k) * xy + (row % k + 1) * kTileY * a.nx + x;
+      j = i - a.nx;
+    } else {
+      const int64_t g = f - fz - fy;
+      const int k = (a.nx - 1) / kTileX, row = (int)(g / k);
+      x = (int)(g - (int64_t)row * k + 1) * kTileX;
+      i = row * a.nx + x;
+      j = i - 1;
+      x = 0;
+    }
+    const int li = __ldcg(a.L + i), lj = __ldcg(a.L + j);
+    if (li < 0 || lj < 0 || a.ori[i] != a.ori[j]) continue;
+    if (x % kTileX && __ldcg(a.L + i - 1) == li && __ldcg(a.L + j - 1) == lj) continue;
+    merge<true>(a.L, li, lj);
   }
 }
 
@@ -145,19 +234,33 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* total) {
   return before + inc - v;
 }
 
-// roots per chunk of kScanChunk cells
-__global__ void __launch_bounds__(kGrainThreads) grain_count_kernel(const GrainArgs a) {
+// every cell's label becomes its root; roots per chunk of kScanChunk cells
+__global__ void __launch_bounds__(kGrainThreads) grain_roots_kernel(const GrainArgs a) {
   const int N = a.nx * a.ny * a.nz;
-  const int base = blockIdx.x * kScanChunk + threadIdx.x * kScanItems;
+  const int base = blockIdx.x * kScanChunk + threadIdx.x;
   int c = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    const int i = base + k;
-    if (i < N && a.L[i] == i) ++c;
+    const int i = base + k * kGrainThreads;
+    if (i >= N) continue;
+    const int l = __ldcg(a.L + i);
+    if (l < 0) continue;
+    if (l == i) {
+      ++c;
+    } else {
+      const int r = find_root<true>(a.L, l);
+      if (r != l) a.L[i] = r;
+    }
   }
-  int total;
-  block_exclusive_scan(c, &total);
-  if (threadIdx.x == 0) a.chunk[blockIdx.x] = total;
+  c = __reduce_add_sync(0xffffffffu, c);
+  __shared__ int s_c[kGrainThreads / 32];
+  if ((threadIdx.x & 31) == 0) s_c[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int total = 0;
+    for (int w = 0; w < kGrainThreads / 32; ++w) total += s_c[w];
+    a.chunk[blockIdx.x] = total;
+  }
 }
 
 // exclusive offsets of the chunk counts (one block) and the grain count
@@ -175,9 +278,13 @@ __global__ void __launch_bounds__(kGrainThreads) grain_offsets_kernel(const Grai
   if (threadIdx.x == 0) *a.num_grains = carry;
 }
 
-// number the roots and start their records
-__global__ void __launch_bounds__(kGrainThreads) grain_number_kernel(const GrainArgs a) {
+// number the roots and start their records (a thread scans consecutive cells)
+__global__ void __launch_bounds__(kGrainThreads) grain_number_kernel(const GrainArgs a,
+                                                                     int nchunks) {
   const int N = a.nx * a.ny * a.nz;
+  const int first = a.chunk[blockIdx.x];
+  const int next = (int)blockIdx.x + 1 < nchunks ? a.chunk[blockIdx.x + 1] : (int)*a.num_grains;
+  if (first == next) return;  // no root here (most chunks)
   const int base = blockIdx.x * kScanChunk + threadIdx.x * kScanItems;
   int c = 0;
 #pragma unroll
@@ -186,7 +293,7 @@ __global__ void __launch_bounds__(kGrainThreads) grain_number_kernel(const Grain
     if (i < N && a.L[i] == i) ++c;
   }
   int total;
-  int g = a.chunk[blockIdx.x] + block_exclusive_scan(c, &total);
+  int g = first + block_exclusive_scan(c, &total);
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     const int i = base + k;
@@ -206,57 +313,99 @@ __global__ void __launch_bounds__(kGrainThreads) grain_number_kernel(const Grain
   }
 }
 
-// per-cell grain number and the grains' moments
+// The moments of a set of cells as sums over (1, x, y, z, xx, yy, zz, xy, xz, yz),
+// moved by (X, Y, Z): the records hold whole-grid coordinates, a tile's table
+// its own.
+template <typename I>
+__device__ __forceinline__ long long moved_moment(const I* v, int m, long long X, long long Y,
+                                                  long long Z) {
+  const long long c = v[0], x = v[1], y = v[2], z = v[3];
+  switch (m) {
+    case 0: return c;
+    case 1: return x + c * X;
+    case 2: return y + c * Y;
+    case 3: return z + c * Z;
+    case 4: return v[4] + 2 * x * X + c * X * X;
+    case 5: return v[5] + 2 * y * Y + c * Y * Y;
+    case 6: return v[6] + 2 * z * Z + c * Z * Z;
+    case 7: return v[7] + x * Y + y * X + c * X * Y;
+    case 8: return v[8] + x * Z + z * X + c * X * Z;
+    default: return v[9] + y * Z + z * Y + c * Y * Z;
+  }
+}
+
+// Per-cell grain numbers and the grains' moments, a tile per block.  A row's
+// runs add their closed-form moments to a small table of the tile's grains in
+// shared memory (tile coordinates: below 2^21, so 32 bits hold them); the
+// table goes to the records with one atomic per grain and moment.  A run
+// whose grain finds no place in the table adds to the record itself.
+constexpr int kMoments = 10, kTable = 128, kProbes = 16;
 __global__ void __launch_bounds__(kGrainThreads) grain_moments_kernel(const GrainArgs a) {
-  const int N = a.nx * a.ny * a.nz;
-  const int xy = a.nx * a.ny;
-  const int lane = threadIdx.x & 31;
-  const int stride = gridDim.x * blockDim.x;
-  // the loop bound is uniform across the warp so that every lane takes part
-  // in the warp-wide aggregation below
-  const int first = blockIdx.x * blockDim.x + (threadIdx.x & ~31);
-  for (int w0 = first; w0 < N; w0 += stride) {
-    const int i = w0 + lane;
+  __shared__ int s_key[kTable];
+  __shared__ int s_sum[kTable][kMoments + 1];
+  const int lane = threadIdx.x & 31, yl = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < kTable; i += kGrainThreads) s_key[i] = -1;
+  for (int i = threadIdx.x; i < kTable * (kMoments + 1); i += kGrainThreads)
+    (&s_sum[0][0])[i] = 0;
+  __syncthreads();
+  const Tile t = tile_of(a, blockIdx.x);
+  const int x = t.x0 + lane, y = t.y0 + yl, xy = a.nx * a.ny;
+  const bool col = x < a.nx && y < a.ny;
+  auto record = [&](int g) { return reinterpret_cast<unsigned long long*>(&a.grains[g].cells); };
+#pragma unroll
+  for (int zl = 0; zl < kTileZ; ++zl) {
+    const int z = t.z0 + zl;
     int g = -1;
-    long long v[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (i < N) {
+    if (col && z < a.nz) {
+      const int i = z * xy + y * a.nx + x;
       const int root = __ldcg(a.L + i);
-      if (root >= 0) {
-        g = a.id[root];
-        const long long z = i / xy, r = i - z * xy, y = r / a.nx, x = r - y * a.nx;
-        v[0] = 1;
-        v[1] = x; v[2] = y; v[3] = z;
-        v[4] = x * x; v[5] = y * y; v[6] = z * z;
-        v[7] = x * y; v[8] = x * z; v[9] = y * z;
-      }
+      if (root >= 0) g = __ldg(a.id + root);
       if (a.out_of_cell) a.out_of_cell[i] = g;
     }
-    // one group of lanes with the same grain at a time
-    unsigned pending = __ballot_sync(0xffffffffu, g >= 0);
-    while (pending) {
-      const int leader = __ffs(pending) - 1;
-      const int gl = __shfl_sync(0xffffffffu, g, leader);
-      const bool mine = (g == gl);
-      pending &= ~__ballot_sync(0xffffffffu, mine);
-      long long s[10];
-#pragma unroll
-      for (int k = 0; k < 10; ++k) {
-        long long t = mine ? v[k] : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        s[k] = t;
-      }
-      if (lane == leader && gl < a.max_grains) {
-        pfg_grain& G = a.grains[gl];
-        unsigned long long* p = reinterpret_cast<unsigned long long*>(&G.cells);
-        atomicAdd(p, (unsigned long long)s[0]);
-        for (int d = 0; d < 3; ++d)
-          atomicAdd(reinterpret_cast<unsigned long long*>(&G.sum[d]), (unsigned long long)s[1 + d]);
-        for (int d = 0; d < 6; ++d)
-          atomicAdd(reinterpret_cast<unsigned long long*>(&G.sum2[d]),
-                    (unsigned long long)s[4 + d]);
-      }
+    const int left = __shfl_up_sync(0xffffffffu, g, 1);
+    const bool start = lane == 0 || g != left;
+    const unsigned starts = __ballot_sync(0xffffffffu, start);
+    if (!start || g < 0 || g >= a.max_grains) continue;
+    const unsigned later = lane == 31 ? 0u : starts & (0xfffffffeu << lane);
+    const int end = later ? __ffs(later) - 1 : 32;  // the run is lane .. end - 1
+    const int c = end - lane, b = end - 1;
+    const int sx = c * (lane + b) / 2;
+    const int sxx = (b * (b + 1) * (2 * b + 1) - (lane - 1) * lane * (2 * lane - 1)) / 6;
+    const int v[kMoments] = {c,           sx,      c * yl,  c * zl,      sxx,
+                             c * yl * yl, c * zl * zl, sx * yl, sx * zl, c * yl * zl};
+    int at = (int)(((unsigned)g * 2654435761u) >> 25);  // 7 bits: the table's size
+    bool placed = false;
+    for (int probe = 0; probe < kProbes && !placed; ++probe) {
+      const int old = atomicCAS(&s_key[at], -1, g);
+      placed = old == -1 || old == g;
+      if (!placed) at = (at + 1) & (kTable - 1);
     }
+    if (placed) {
+#pragma unroll
+      for (int m = 0; m < kMoments; ++m) atomicAdd(&s_sum[at][m], v[m]);
+    } else {
+      for (int m = 0; m < kMoments; ++m)
+        atomicAdd(record(g) + m, (unsigned long long)moved_moment(v, m, t.x0, t.y0, t.z0));
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kTable * kMoments; i += kGrainThreads) {
+    const int e = i / kMoments, m = i - e * kMoments, g = s_key[e];
+    if (g >= 0)
+      atomicAdd(record(g) + m,
+                (unsigned long long)moved_moment(s_sum[e], m, t.x0, t.y0, t.z0));
+  }
+}
+static_assert(kTable == 128, "the table's hash takes 7 bits");
+
+// labels[i] = rank[labels[i]] in place (-1 stays)
+__global__ void __launch_bounds__(kGrainThreads) grain_relabel_kernel(int64_t N,
+                                                                      const int32_t* rank,
+                                                                      int32_t* labels) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int g = labels[i];
+    if (g >= 0) labels[i] = __ldg(rank + g);
   }
 }
 
@@ -312,12 +461,25 @@ extern "C" int pfg_grains(const pfg_pf_params* p, const int32_t* ori, const floa
   a.num_grains = num_grains;
   const int grid = grain_grid(N);
   const int nchunks = (int)chunk_count(N);
-  grain_init_kernel<<<grid, kGrainThreads, 0, s>>>(a);
-  grain_merge_kernel<<<grid, kGrainThreads, 0, s>>>(a);
-  grain_compress_kernel<<<grid, kGrainThreads, 0, s>>>(a);
-  grain_count_kernel<<<nchunks, kGrainThreads, 0, s>>>(a);
+  // tile counts stay below 2^31: at least one cell per tile
+  const unsigned tiles = (unsigned)((p->nx + kTileX - 1) / kTileX) *
+                         (unsigned)((p->ny + kTileY - 1) / kTileY) *
+                         (unsigned)((p->nz + kTileZ - 1) / kTileZ);
+  grain_tile_kernel<<<tiles, kGrainThreads, 0, s>>>(a);
+  grain_faces_kernel<<<grid, kGrainThreads, 0, s>>>(a);
+  grain_roots_kernel<<<nchunks, kGrainThreads, 0, s>>>(a);
   grain_offsets_kernel<<<1, kGrainThreads, 0, s>>>(a, nchunks);
-  grain_number_kernel<<<nchunks, kGrainThreads, 0, s>>>(a);
-  grain_moments_kernel<<<grid, kGrainThreads, 0, s>>>(a);
+  grain_number_kernel<<<nchunks, kGrainThreads, 0, s>>>(a, nchunks);
+  grain_moments_kernel<<<tiles, kGrainThreads, 0, s>>>(a);
+  return record_cuda(cudaGetLastError());
+}
+
+extern "C" int pfg_grain_relabel(int64_t num_cells, const int32_t* rank, int32_t* labels,
+                                 void* stream) {
+  if (num_cells < 1) return PFG_ERR_SHAPE;
+  if (!rank || !labels) return PFG_ERR_NULL;
+  if (!device_info().ok) return PFG_ERR_NO_DEVICE;
+  grain_relabel_kernel<<<grain_grid(num_cells), kGrainThreads, 0,
+                         static_cast<cudaStream_t>(stream)>>>(num_cells, rank, labels);
   return record_cuda(cudaGetLastError());
 }

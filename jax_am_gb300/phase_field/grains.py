@@ -54,25 +54,40 @@ def _cell_volume(pf_args):
 
 
 def aspect_ratios(records):
-    """Aspect ratios from the grains' integer moments: the covariance of
-    the cell centres (ddof = 1, exact integer numerators), its eigenvalues in
-    descending order, 2 sqrt(ev0) / (sqrt(ev1) + sqrt(ev2)); 1 below 5 cells
-    (utils.py:286-310).  Cell-centre scaling (h, the volume weights) cancels."""
-    K = len(records)
-    ar = np.ones(K)
-    big = [k for k in range(K) if records[k][0] >= 5]
-    if not big:
+    """Aspect ratios of grains given as (cells, sums, sums2) records of their
+    integer moments (see ``_aspect_ratios``)."""
+    if not len(records):
+        return np.ones(0)
+    c, s, s2 = (np.array([r[k] for r in records], dtype=np.int64) for k in range(3))
+    return _aspect_ratios(c, s, s2)
+
+
+def _aspect_ratios(cells, sums, sums2):
+    """Aspect ratios from the grains' integer moments ((K,), (K, 3) and (K, 6)
+    int64): the covariance of the cell centres (ddof = 1, exact integer
+    numerators), its eigenvalues in descending order, 2 sqrt(ev0) / (sqrt(ev1)
+    + sqrt(ev2)); 1 below 5 cells (utils.py:286-310).  Cell-centre scaling (h,
+    the volume weights) cancels."""
+    ar = np.ones(len(cells))
+    big = np.flatnonzero(cells >= 5)
+    if not len(big):
         return ar
-    cov = np.zeros((len(big), 3, 3))
-    pairs = ((0, 0, 0), (1, 1, 1), (2, 2, 2), (0, 1, 3), (0, 2, 4), (1, 2, 5))
-    for j, k in enumerate(big):
-        c, s, s2 = records[k]
-        c = int(c)
-        den = c * (c - 1)
-        for a, b, m in pairs:
-            # exact: (c * sum(ab) - sum(a) sum(b)) / (c (c - 1)), big Python ints
-            v = (c * int(s2[m]) - int(s[a]) * int(s[b])) / den
-            cov[j, a, b] = cov[j, b, a] = v
+    c, s, s2 = cells[big], sums[big], sums2[big]
+    # c * sum(ab) - sum(a) sum(b) over c (c - 1), correctly rounded: integers
+    # below 2^53 are exact in int64 and float64, the few others take Python's
+    limit = 2.0 ** 53
+    exact = (c.astype(np.float64) * np.maximum(s2.max(axis=1), c) < limit) & (
+        s.max(axis=1).astype(np.float64) ** 2 < limit)
+    a, b = (0, 1, 2, 0, 0, 1), (0, 1, 2, 1, 2, 2)
+    with np.errstate(over="ignore"):
+        v = (c[:, None] * s2 - s[:, a] * s[:, b]) / (c * (c - 1)).astype(np.float64)[:, None]
+    for j in np.flatnonzero(~exact):
+        cj = int(c[j])
+        for m in range(6):
+            v[j, m] = (cj * int(s2[j, m]) - int(s[j, a[m]]) * int(s[j, b[m]])) / (cj * (cj - 1))
+    cov = np.empty((len(big), 3, 3))
+    cov[:, a, b] = v
+    cov[:, b, a] = v
     ev = np.linalg.eigvalsh(cov)[:, ::-1]
     ln = np.sqrt(np.maximum(ev, 0.0))
     with np.errstate(divide="ignore", invalid="ignore"):
@@ -95,8 +110,9 @@ def segment_grains(pf_args, ori_inds, T, T_ghosted=False, max_grains=None):
     ori = ori.to("cuda", torch.int32).reshape(-1).contiguous()
     if ori.numel() != N:
         raise ValueError(f"ori_inds has {ori.numel()} entries, expected {N}")
-    n = int(ori.max().item()) + 1 if N else 1
-    n = max(n, int(pf_args.get("num_oris", n)))
+    n = int(pf_args.get("num_oris", 0))
+    if n < 1:  # not given: from the map
+        n = max(n, int(ori.max().item()) + 1 if N else 1)
     args = dict(pf_args, num_oris=min(n, _lib.MAX_ORIS))
     for key, default in (("gas_const", 8.3), ("Qg", 1.4e5), ("L0", 3.5e3), ("kappa_g", 2.77e-6),
                          ("m_g", 2.4e5), ("anisotropy", 0.0), ("ad_hoc", 1.0)):
@@ -129,18 +145,20 @@ def segment_grains(pf_args, ori_inds, T, T_ghosted=False, max_grains=None):
     first, ori_g = raw[:, 0], (raw[:, 1] & 0xFFFFFFFF).astype(np.int64)
     cells, sums, sums2 = raw[:, 2], raw[:, 3:6], raw[:, 6:12]
     order = np.lexsort((first, ori_g))  # by orientation, then smallest cell index
-    rank = np.empty(K, dtype=np.int64)
-    rank[order] = np.arange(K)
-    rank_t = torch.as_tensor(rank, dtype=torch.int32, device="cuda")
-    lab = torch.where(labels >= 0, rank_t[labels.clamp(min=0).long()] if K else labels, labels)
-    records = [(cells[k], sums[k], sums2[k]) for k in order]
+    rank = np.empty(K, dtype=np.int32)
+    rank[order] = np.arange(K, dtype=np.int32)
+    if K:
+        rank_t = torch.from_numpy(rank).to("cuda")
+        st = lib.pfg_grain_relabel(N, _lib.ptr(rank_t), _lib.ptr(labels), stream)
+        _lib.check(st, "pfg_grain_relabel")
+    cells, sums, sums2 = cells[order], sums[order], sums2[order]
     return {
-        "labels": lab,
+        "labels": labels,
         "ori": ori_g[order].astype(np.int64),
         "first_cell": first[order],
-        "cells": cells[order],
-        "volumes": cells[order] * _cell_volume(pf_args),
-        "aspect_ratios": aspect_ratios(records),
+        "cells": cells,
+        "volumes": cells * _cell_volume(pf_args),
+        "aspect_ratios": _aspect_ratios(cells, sums, sums2),
     }
 
 

@@ -73,6 +73,40 @@ def test_grains_match_oracle(shape, n, seeds, liquid):
     _check_aspect_ratios(res["aspect_ratios"], ars)
 
 
+@pytest.mark.parametrize("shape,pattern", [((33, 9, 9), "noise"), ((32, 8, 8), "speckle"),
+                                           ((65, 17, 16), "snake"), ((31, 25, 7), "comb")])
+def test_grains_across_tiles(shape, pattern):
+    """At the edges of the 32 x 8 x 8 cell tiles: noise (short runs), a speckle
+    with more grains in a tile than its table holds, one grain that winds
+    through every tile, and teeth that meet only at a far row."""
+    from jax_am_gb300.phase_field.grains import segment_grains
+    rng = np.random.default_rng(11)
+    Nx, Ny, Nz = shape
+    zz, yy, xx = np.meshgrid(np.arange(Nz), np.arange(Ny), np.arange(Nx), indexing="ij")
+    if pattern == "noise":
+        ori = rng.integers(0, 3, (Nz, Ny, Nx))
+    elif pattern == "speckle":
+        ori = rng.integers(0, 40, (Nz, Ny, Nx))
+    elif pattern == "snake":  # odd rows and planes joined at alternating ends
+        row, plane = (yy % 2 == 0), (zz % 2 == 0)
+        turn_y = (yy % 2 == 1) & (xx == np.where(yy % 4 == 1, Nx - 1, 0))
+        turn_z = (zz % 2 == 1) & (xx == 0) & (yy == np.where(zz % 4 == 1, Ny - 1, 0))
+        ori = np.where(plane & (row | turn_y) | turn_z, 1, 0)
+    else:
+        ori = np.where((xx % 2 == 0) | (yy == Ny - 1), 1, 2)
+    T = rng.uniform(1400.0, 1600.0, ori.shape).astype(np.float32)
+    if pattern == "noise":
+        T[rng.random(T.shape) < 0.1] = 1700.0
+    ori, T = ori.ravel().astype(np.int32), T.ravel()
+    res = segment_grains(_args(Nx, Ny, Nz), ori, T)
+    labels, K = O.grain_components(ori, T, 1623.0, Nx, Ny, Nz)
+    vols, ars = O.grain_volumes_and_aspect_ratios(labels, K, Nx, Ny, Nz, 1e-6)
+    assert pattern != "speckle" or K > 128
+    np.testing.assert_array_equal(res["labels"].cpu().numpy(), labels)
+    np.testing.assert_allclose(res["volumes"], vols, rtol=1e-12)
+    _check_aspect_ratios(res["aspect_ratios"], ars)
+
+
 def test_ghosted_temperature_and_small_capacity():
     """The ghosted heat state gives the same grains as the per-cell T, and a
     grain array too small for the first call is regrown."""
