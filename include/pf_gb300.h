@@ -260,6 +260,19 @@ int pfg_pf_step_quench(const pfg_pf_params* p, const pfg_quench* q, const float*
 int pfg_pf_step_point_source(const pfg_pf_params* p, const pfg_point_sources* src,
                              const float* eta_in, float* eta_out, const pfg_clock* clk_in,
                              pfg_clock* clk_out, float dt, void* stream);
+/* The same two steps, and the interpolated one below, with their start given
+ * by value: a host loop that knows the time (or the source record) keeps no
+ * clock on the device. */
+int pfg_pf_step_quench_at(const pfg_pf_params* p, const pfg_quench* q, const float* eta_in,
+                          float* eta_out, double t, float dt, void* stream);
+int pfg_pf_step_point_source_at(const pfg_pf_params* p, const pfg_point_sources* src,
+                                const float* eta_in, float* eta_out, int64_t record, float dt,
+                                void* stream);
+int pfg_pf_step_interp_at(const pfg_pf_params* p, const pfg_interp* w, const float* T_past,
+                          const float* T_future, const float* eta_in, float* eta_out, double t,
+                          float dt, void* stream);
+/* Set a device clock (enqueued on the stream, no host wait). */
+int pfg_clock_set(pfg_clock* clk, double t, int64_t step, void* stream);
 /* The (nz, ny, nx) temperature that pfg_pf_step_point_source uses for a step
  * starting at clk (what the drivers pass to inspect_sol and write_sols). */
 int pfg_point_source_T(const pfg_pf_params* p, const pfg_point_sources* src,

@@ -167,6 +167,13 @@ _PROTOS = {
                                       _P, _P, _P, _F, _P]),
     "pfg_pf_step_interp": (_I, [ctypes.POINTER(PfParams), ctypes.POINTER(Interp), _P, _P, _P, _P,
                                 _P, _P, _F, _P]),
+    "pfg_pf_step_quench_at": (_I, [ctypes.POINTER(PfParams), ctypes.POINTER(Quench), _P, _P,
+                                   ctypes.c_double, _F, _P]),
+    "pfg_pf_step_point_source_at": (_I, [ctypes.POINTER(PfParams), ctypes.POINTER(PointSources),
+                                         _P, _P, ctypes.c_int64, _F, _P]),
+    "pfg_pf_step_interp_at": (_I, [ctypes.POINTER(PfParams), ctypes.POINTER(Interp), _P, _P, _P,
+                                   _P, ctypes.c_double, _F, _P]),
+    "pfg_clock_set": (_I, [_P, ctypes.c_double, ctypes.c_int64, _P]),
     "pfg_transpose_xyz": (_I, [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, _P, _P, _P]),
     "pfg_cfd_workspace_bytes": (ctypes.c_int64, [ctypes.POINTER(CfdGrid), ctypes.POINTER(CfdGrid)]),
     "pfg_cfd_energy_solve": (_I, [ctypes.POINTER(CfdGrid), ctypes.POINTER(CfdEnergy), _P, _P, _P,

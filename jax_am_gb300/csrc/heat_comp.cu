@@ -36,7 +36,7 @@ heat_comp_kernel(const __grid_constant__ StepArgs a) {
     if (threadIdx.x == 0) {
       // the beam centre and power at mid-step, the centre also as double-float
       double xd, yd;
-      laser_at_d(a.hp, a.clk_in->t + 0.5 * (double)a.dt, &xd, &yd, &s_beam[2]);
+      laser_at_d(a.hp, start_time(a) + 0.5 * (double)a.dt, &xd, &yd, &s_beam[2]);
       s_beam[0] = (float)xd;
       s_beam[1] = (float)yd;
       s_beam[3] = (float)(xd - (double)s_beam[0]);

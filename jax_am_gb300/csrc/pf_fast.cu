@@ -31,11 +31,8 @@ __global__ void __launch_bounds__(kThreads, 2) pf_warp_kernel(const __grid_const
   extern __shared__ __align__(16) float smem[];
   double t0 = 0.0;
   if constexpr (TSRC != kTArray) {
-    t0 = a.clk_in->t;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && a.clk_out) {
-      a.clk_out->t = t0 + (double)a.dt;
-      a.clk_out->step = a.clk_in->step + 1;
-    }
+    t0 = start_time(a);
+    if (blockIdx.x == 0 && threadIdx.x == 0) end_step(a, t0);
   }
   warp_unit<VEC, ANISO, TSRC>(a, blockIdx.x, t0, smem);
 }

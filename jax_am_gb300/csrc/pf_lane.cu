@@ -166,15 +166,12 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     double t = 0.0;
     if constexpr (TSRC != kTArray) {
-      t = a.clk_in->t;
-      if (blockIdx.x == 0 && a.clk_out) {
-        a.clk_out->t = t + (double)a.dt;
-        a.clk_out->step = a.clk_in->step + 1;
-      }
+      t = start_time(a);
+      if (blockIdx.x == 0) end_step(a, t);
     }
     s_t0 = t;
     if constexpr (TSRC == kTQuench) s_Tq[0] = quench_T(a, zb, t);
-    s_step = (TSRC != kTArray) ? a.clk_in->step : 0;
+    s_step = (TSRC != kTArray) ? start_step(a) : 0;
     if constexpr (HEAT) {
       // beam centre and power at mid-step; the centre also as double-float
       double xd, yd;

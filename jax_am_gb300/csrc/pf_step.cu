@@ -140,14 +140,11 @@ pf_zmarch_kernel(const __grid_constant__ StepArgs a) {
   float xl = 0.f, yl = 0.f, P = 0.f;
   double t0 = 0.0;
   pfg_point_source prec{};
-  if constexpr (TSRC == kTPoint) prec = point_record(a.ps, a.clk_in->step);
+  if constexpr (TSRC == kTPoint) prec = point_record(a.ps, start_step(a));
   if constexpr (TSRC != kTArray) {
-    t0 = a.clk_in->t;
+    t0 = start_time(a);
     if constexpr (TSRC == kTHeat) laser_at(a.hp, t0 + 0.5 * (double)a.dt, &xl, &yl, &P);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && a.clk_out) {
-      a.clk_out->t = t0 + (double)a.dt;
-      a.clk_out->step = a.clk_in->step + 1;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) end_step(a, t0);
   }
 
   const int S = a.stages;
@@ -610,20 +607,41 @@ extern "C" int pfg_pf_step(const pfg_pf_params* p, const float* eta_in, float* e
   return record_cuda(dispatch<kTArray>(a, *p, dt, static_cast<cudaStream_t>(stream)));
 }
 
+// A step whose start is a clock on the device (clk_in, clk_out) or a value.
+template <int TSRC>
+static int step_from(StepArgs& a, const pfg_pf_params* p, const float* eta_in, float* eta_out,
+                     const pfg_clock* clk_in, pfg_clock* clk_out, pfg_clock start, float dt,
+                     void* stream) {
+  if (!eta_in || !eta_out) return PFG_ERR_NULL;
+  if (!aligned16(eta_in) || !aligned16(eta_out)) return PFG_ERR_ALIGN;
+  if (!device_info().ok) return PFG_ERR_NO_DEVICE;
+  a.eta_in = eta_in; a.eta_out = eta_out; a.T_out = nullptr;
+  a.clk_in = clk_in; a.clk_out = clk_out;
+  a.start = start;
+  return record_cuda(dispatch<TSRC>(a, *p, dt, static_cast<cudaStream_t>(stream)));
+}
+
 extern "C" int pfg_pf_step_quench(const pfg_pf_params* p, const pfg_quench* q,
                                   const float* eta_in, float* eta_out, const pfg_clock* clk_in,
                                   pfg_clock* clk_out, float dt, void* stream) {
   int st = check_pf_params(p);
   if (st) return st;
-  if (!q || !eta_in || !eta_out || !clk_in) return PFG_ERR_NULL;
+  if (!q || !clk_in) return PFG_ERR_NULL;
   if (clk_in == clk_out) return PFG_ERR_PARAM;
-  if (!aligned16(eta_in) || !aligned16(eta_out)) return PFG_ERR_ALIGN;
-  if (!device_info().ok) return PFG_ERR_NO_DEVICE;
   StepArgs a{};
-  a.eta_in = eta_in; a.eta_out = eta_out; a.T = nullptr; a.T_out = nullptr;
-  a.clk_in = clk_in; a.clk_out = clk_out;
   a.q = *q;
-  return record_cuda(dispatch<kTQuench>(a, *p, dt, static_cast<cudaStream_t>(stream)));
+  return step_from<kTQuench>(a, p, eta_in, eta_out, clk_in, clk_out, pfg_clock{}, dt, stream);
+}
+
+extern "C" int pfg_pf_step_quench_at(const pfg_pf_params* p, const pfg_quench* q,
+                                     const float* eta_in, float* eta_out, double t, float dt,
+                                     void* stream) {
+  int st = check_pf_params(p);
+  if (st) return st;
+  if (!q) return PFG_ERR_NULL;
+  StepArgs a{};
+  a.q = *q;
+  return step_from<kTQuench>(a, p, eta_in, eta_out, nullptr, nullptr, pfg_clock{t, 0}, dt, stream);
 }
 
 extern "C" int pfg_pf_step_point_source(const pfg_pf_params* p, const pfg_point_sources* src,
@@ -634,15 +652,34 @@ extern "C" int pfg_pf_step_point_source(const pfg_pf_params* p, const pfg_point_
   if (st) return st;
   st = check_point_sources(src);
   if (st) return st;
-  if (!eta_in || !eta_out || !clk_in) return PFG_ERR_NULL;
+  if (!clk_in) return PFG_ERR_NULL;
   if (clk_in == clk_out) return PFG_ERR_PARAM;
-  if (!aligned16(eta_in) || !aligned16(eta_out)) return PFG_ERR_ALIGN;
-  if (!device_info().ok) return PFG_ERR_NO_DEVICE;
   StepArgs a{};
-  a.eta_in = eta_in; a.eta_out = eta_out; a.T = nullptr; a.T_out = nullptr;
-  a.clk_in = clk_in; a.clk_out = clk_out;
   a.ps = make_point_consts(*src, *p);
-  return record_cuda(dispatch<kTPoint>(a, *p, dt, static_cast<cudaStream_t>(stream)));
+  return step_from<kTPoint>(a, p, eta_in, eta_out, clk_in, clk_out, pfg_clock{}, dt, stream);
+}
+
+extern "C" int pfg_pf_step_point_source_at(const pfg_pf_params* p, const pfg_point_sources* src,
+                                           const float* eta_in, float* eta_out, int64_t record,
+                                           float dt, void* stream) {
+  int st = check_pf_params(p);
+  if (st) return st;
+  st = check_point_sources(src);
+  if (st) return st;
+  StepArgs a{};
+  a.ps = make_point_consts(*src, *p);
+  return step_from<kTPoint>(a, p, eta_in, eta_out, nullptr, nullptr, pfg_clock{0.0, record}, dt,
+                            stream);
+}
+
+static int set_interp(StepArgs& a, const pfg_interp* w, const float* T_past,
+                      const float* T_future) {
+  if (!w || !T_past || !T_future) return PFG_ERR_NULL;
+  if (!(w->dt_coarse > 0.0)) return PFG_ERR_PARAM;
+  a.T = T_past; a.T2 = T_future;
+  a.t_future = w->t_future;
+  a.dt_coarse = w->dt_coarse;
+  return PFG_OK;
 }
 
 extern "C" int pfg_pf_step_interp(const pfg_pf_params* p, const pfg_interp* w,
@@ -651,17 +688,33 @@ extern "C" int pfg_pf_step_interp(const pfg_pf_params* p, const pfg_interp* w,
                                   pfg_clock* clk_out, float dt, void* stream) {
   int st = check_pf_params(p);
   if (st) return st;
-  if (!w || !T_past || !T_future || !eta_in || !eta_out || !clk_in) return PFG_ERR_NULL;
-  if (clk_in == clk_out) return PFG_ERR_PARAM;
-  if (!(w->dt_coarse > 0.0)) return PFG_ERR_PARAM;
-  if (!aligned16(eta_in) || !aligned16(eta_out)) return PFG_ERR_ALIGN;
-  if (!device_info().ok) return PFG_ERR_NO_DEVICE;
   StepArgs a{};
-  a.eta_in = eta_in; a.eta_out = eta_out; a.T = T_past; a.T2 = T_future; a.T_out = nullptr;
-  a.clk_in = clk_in; a.clk_out = clk_out;
-  a.t_future = w->t_future;
-  a.dt_coarse = w->dt_coarse;
-  return record_cuda(dispatch<kTInterp>(a, *p, dt, static_cast<cudaStream_t>(stream)));
+  if (!clk_in) return PFG_ERR_NULL;
+  if (clk_in == clk_out) return PFG_ERR_PARAM;
+  st = set_interp(a, w, T_past, T_future);
+  if (st) return st;
+  return step_from<kTInterp>(a, p, eta_in, eta_out, clk_in, clk_out, pfg_clock{}, dt, stream);
+}
+
+extern "C" int pfg_pf_step_interp_at(const pfg_pf_params* p, const pfg_interp* w,
+                                     const float* T_past, const float* T_future,
+                                     const float* eta_in, float* eta_out, double t, float dt,
+                                     void* stream) {
+  int st = check_pf_params(p);
+  if (st) return st;
+  StepArgs a{};
+  st = set_interp(a, w, T_past, T_future);
+  if (st) return st;
+  return step_from<kTInterp>(a, p, eta_in, eta_out, nullptr, nullptr, pfg_clock{t, 0}, dt, stream);
+}
+
+__global__ void clock_set_kernel(pfg_clock* clk, pfg_clock v) { *clk = v; }
+
+extern "C" int pfg_clock_set(pfg_clock* clk, double t, int64_t step, void* stream) {
+  if (!clk) return PFG_ERR_NULL;
+  if (!device_info().ok) return PFG_ERR_NO_DEVICE;
+  clock_set_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(clk, pfg_clock{t, step});
+  return record_cuda(cudaGetLastError());
 }
 
 // (nx, ny, nz) z-fastest -> (nz, ny, nx) x-fastest, 32 x 32 tiles of (x, z)

@@ -23,8 +23,9 @@ struct __align__(16) StepArgs {
   float* eta_out;
   const float* T;  // per-cell T (pf only) or ghosted Tg (fused)
   float* T_out;    // ghosted Tg_out (fused) or nullptr
-  const pfg_clock* clk_in;
+  const pfg_clock* clk_in;  // the step's start on the device, or NULL: `start`
   pfg_clock* clk_out;
+  pfg_clock start;
   HeatConsts hc;
   HeatDF hd;           // compensated heat update constants (fused, T_lo set)
   const float* T_lo;   // low parts of the compensated ghosted T (or nullptr)
@@ -39,6 +40,20 @@ struct __align__(16) StepArgs {
   float dirs[3 * PFG_MAX_ORIS * 3];
 };
 
+
+// The start of the step.
+__device__ __forceinline__ double start_time(const StepArgs& a) {
+  return a.clk_in ? a.clk_in->t : a.start.t;
+}
+__device__ __forceinline__ int64_t start_step(const StepArgs& a) {
+  return a.clk_in ? a.clk_in->step : a.start.step;
+}
+// Advance the clock (one thread of a launch).
+__device__ __forceinline__ void end_step(const StepArgs& a, double t) {
+  if (!a.clk_out) return;
+  a.clk_out->t = t + (double)a.dt;
+  a.clk_out->step = start_step(a) + 1;
+}
 
 struct TilePlan;
 int set_tune(int key, int value);

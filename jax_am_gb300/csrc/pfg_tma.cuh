@@ -156,14 +156,11 @@ __device__ __forceinline__ void tma_unit(const StepArgs& a, int unit, const floa
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     double t = 0.0;
     if constexpr (TSRC != kTArray) {
-      t = BATCH ? t_batch : a.clk_in->t;
-      if (!BATCH && unit == 0 && a.clk_out) {
-        a.clk_out->t = t + (double)a.dt;
-        a.clk_out->step = a.clk_in->step + 1;
-      }
+      t = BATCH ? t_batch : start_time(a);
+      if (!BATCH && unit == 0) end_step(a, t);
     }
     s_t0 = t;
-    s_step = (TSRC != kTArray && !BATCH) ? a.clk_in->step : 0;
+    s_step = (TSRC != kTArray && !BATCH) ? start_step(a) : 0;
     if constexpr (TSRC == kTHeat) {
       // beam position and power at mid-step, once per CTA
       laser_at(a.hp, t + 0.5 * (double)a.dt, &s_beam[0], &s_beam[1], &s_beam[2]);

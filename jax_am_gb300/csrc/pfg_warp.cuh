@@ -191,7 +191,7 @@ __device__ __forceinline__ void warp_unit(const StepArgs& a, int unit, double t0
   }
   float xl = 0.f, yl = 0.f, Pw = 0.f;  // read after the prologue's barrier
   pfg_point_source prec{};
-  if constexpr (TSRC == kTPoint) prec = point_record(a.ps, a.clk_in->step);
+  if constexpr (TSRC == kTPoint) prec = point_record(a.ps, start_step(a));
   float w_past = 0.f;
   if constexpr (TSRC == kTInterp) w_past = interp_weight(a.t_future, a.dt_coarse, t0 + (double)a.dt);
 

@@ -14,6 +14,7 @@ reference's ``get_force_eta_fn``, whose call is commented out of its
 """
 import ctypes
 import glob
+import math
 import os
 import time
 
@@ -93,8 +94,8 @@ def as_device_f32(x, shape=None, name="array"):
     if x.dtype != torch.float32:
         x = x.float()
     x = x.contiguous()
-    if shape is not None and x.numel() != int(np.prod(shape)):
-        raise ValueError(f"{name} has {x.numel()} entries, expected {int(np.prod(shape))}")
+    if shape is not None and x.numel() != math.prod(shape):
+        raise ValueError(f"{name} has {x.numel()} entries, expected {math.prod(shape)}")
     return x
 
 
@@ -123,7 +124,6 @@ class PFSolver:
         self.params = make_pf_params(pf_args, polycrystal)
         self.N = self.params.nx * self.params.ny * self.params.nz
         self.n = self.params.num_oris
-        self._clock = None
         self._diag_scratch = None
         self._diag_out = None
         self._argmax0 = None
@@ -149,39 +149,27 @@ class PFSolver:
         elif out.data_ptr() == eta.data_ptr():
             raise ValueError("out must not alias eta")
         dt = float(t_crt) - float(t_prev)
+        p, stream = ctypes.byref(self.params), _stream()
+        src, dst = eta.data_ptr(), out.data_ptr()
+        # the step's start goes by value: no clock on the device, no copies
         if isinstance(T, Quench):
-            clk = self._clocks()
-            clk[0].fill_(0)
-            clk[0].view(torch.float64)[0] = float(t_prev)
             q = T.struct(self.params.h_z)
-            st = self.lib.pfg_pf_step_quench(ctypes.byref(self.params), ctypes.byref(q),
-                                              _lib.ptr(eta), _lib.ptr(out), _lib.ptr(clk[0]),
-                                              _lib.ptr(clk[1]), dt, _stream())
+            st = self.lib.pfg_pf_step_quench_at(p, ctypes.byref(q), src, dst, float(t_prev), dt,
+                                                stream)
         elif isinstance(T, InterpolatedT):
             if T.T_past.numel() != self.N:
                 raise ValueError(f"InterpolatedT holds {T.T_past.numel()} cells, expected {self.N}")
-            clk = self._clocks()
-            clk[0].fill_(0)
-            clk[0].view(torch.float64)[0] = float(t_prev)
             w = T.struct()
-            st = self.lib.pfg_pf_step_interp(ctypes.byref(self.params), ctypes.byref(w),
-                                              _lib.ptr(T.T_past), _lib.ptr(T.T_future),
-                                              _lib.ptr(eta), _lib.ptr(out), _lib.ptr(clk[0]),
-                                              _lib.ptr(clk[1]), dt, _stream())
+            st = self.lib.pfg_pf_step_interp_at(p, ctypes.byref(w), T.T_past.data_ptr(),
+                                                T.T_future.data_ptr(), src, dst, float(t_prev),
+                                                dt, stream)
         elif isinstance(T, PointSource):
-            clk = self._clocks()
-            clk[0].fill_(0)
-            clk[0].view(torch.float64)[0] = float(t_prev)
-            clk[0][1] = T.index_at(t_prev)
-            src = T.struct(self.params)
-            st = self.lib.pfg_pf_step_point_source(ctypes.byref(self.params), ctypes.byref(src),
-                                                    _lib.ptr(eta), _lib.ptr(out),
-                                                    _lib.ptr(clk[0]), _lib.ptr(clk[1]), dt,
-                                                    _stream())
+            source = T.struct(self.params)
+            st = self.lib.pfg_pf_step_point_source_at(p, ctypes.byref(source), src, dst,
+                                                      T.index_at(t_prev), dt, stream)
         else:
             T = as_device_f32(T, (self.N,), "T")
-            st = self.lib.pfg_pf_step(ctypes.byref(self.params), _lib.ptr(eta), _lib.ptr(out),
-                                      _lib.ptr(T), dt, _stream())
+            st = self.lib.pfg_pf_step(p, src, dst, T.data_ptr(), dt, stream)
         _lib.check(st, "pfg_pf_step")
         return (out, t_crt), out
 
@@ -256,11 +244,6 @@ class PFSolver:
         return path
 
     # ---- extensions ---------------------------------------------------------
-    def _clocks(self):
-        if self._clock is None:
-            self._clock = torch.zeros((2, 2), dtype=torch.int64, device="cuda")
-        return self._clock
-
     def argmax(self, eta):
         """First-maximum orientation index per cell (int32), from the diagnostics kernel."""
         out = torch.empty(self.N, dtype=torch.int32, device="cuda")

@@ -89,9 +89,8 @@ class _GraphRun:
         return self
 
     def set_time(self, t, step=0):
-        c = self.clk[self.cur]
-        c[1] = int(step)
-        c[0:1].view(torch.float64)[0] = float(t)
+        _lib.check(_lib.load().pfg_clock_set(_lib.ptr(self.clk[self.cur]), float(t), int(step),
+                                             _stream()), "pfg_clock_set")
 
     @property
     def t(self):

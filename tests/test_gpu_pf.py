@@ -324,3 +324,42 @@ def test_liquidus_not_a_float32_value():
                       torch.tensor(T, dtype=torch.float32, device="cuda"), [0.0, 1e-8], 1)
     want = 100.0 * np.mean(T.astype(np.float32).reshape(-1) >= tl32)
     assert abs(d["pct_liquid"] - want) <= 1e-9
+
+
+@pytest.mark.parametrize("shape,n", [((17, 9, 6), 20), ((12, 7, 5), 8), ((9, 5, 4), 7),
+                                     ((5, 4, 3), 33)])
+@pytest.mark.parametrize("source", ["quench", "point", "interp"])
+def test_start_by_value_matches_device_clock(shape, n, source):
+    """A step started by value (what ``PFSolver.stepper`` enqueues) equals the
+    step started by a clock on the device bit for bit, in each kernel."""
+    import ctypes
+    from jax_am_gb300 import _lib
+    from jax_am_gb300.phase_field.allen_cahn import PFSolver, Quench
+    from jax_am_gb300.phase_field.coupling import InterpolatedT
+    from jax_am_gb300.phase_field.point_source import PointSource
+    poly, eta, T, pf_args, oargs, obc = pf_case(shape, n, 0.15, seed=21)
+    s = PFSolver(pf_args, poly)
+    e = torch.tensor(eta, dtype=torch.float32, device="cuda")
+    t, dt = 3.7e-6, float(np.float32(2e-8))
+    if source == "quench":
+        src, entry = Quench(1623.0, 1e6, 0.1, z0=2e-6), "pfg_pf_step_quench"
+        args = [ctypes.byref(src.struct(s.params.h_z))]
+    elif source == "point":
+        ts = np.arange(4) * 1e-6 + 1e-6
+        src = PointSource(ts, ts * 0.8, 3e-6, 5e-6, (1, 0, 0), 25.0, 0.8, 300.0, T_clip=2000.0)
+        entry, args = "pfg_pf_step_point_source", [ctypes.byref(src.struct(s.params))]
+    else:
+        src = InterpolatedT(T, T + 50.0, t + 1e-6, 2e-6)
+        entry = "pfg_pf_step_interp"
+        args = [ctypes.byref(src.struct()), _lib.ptr(src.T_past), _lib.ptr(src.T_future)]
+    (got, _), _ = s.stepper((e, t), t + dt, [src])
+    clk = torch.zeros((2, 2), dtype=torch.int64, device="cuda")
+    step = src.index_at(t) if source == "point" else 0
+    _lib.check(s.lib.pfg_clock_set(_lib.ptr(clk[0]), t, step, None), "pfg_clock_set")
+    ref = torch.empty_like(e)
+    _lib.check(getattr(s.lib, entry)(ctypes.byref(s.params), *args, _lib.ptr(e), _lib.ptr(ref),
+                                     _lib.ptr(clk[0]), _lib.ptr(clk[1]), (t + dt) - t, None), entry)
+    assert torch.equal(got, ref)
+    torch.cuda.synchronize()
+    assert int(clk[1, 1]) == step + 1
+    assert float(clk[1, :1].view(torch.float64)) == t + float(np.float32((t + dt) - t))
