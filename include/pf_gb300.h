@@ -298,6 +298,10 @@ int pfg_transpose_xyz(int32_t nx, int32_t ny, int32_t nz, const float* T_xyz, fl
  * faces of Tg_out are written, edge/corner ghosts are left untouched. */
 int pfg_heat_step(const pfg_heat_params* h, const float* Tg_in, float* Tg_out,
                   float xl, float yl, float power, float dt, void* stream);
+/* The same step writing every element of Tg_out: the edge and corner ghosts are
+ * carried over from Tg_in, so a new buffer needs no copy first. */
+int pfg_heat_step_whole(const pfg_heat_params* h, const float* Tg_in, float* Tg_out,
+                        float xl, float yl, float power, float dt, void* stream);
 
 /* ---- fused heat + phase field -------------------------------------------
  * One pass that reads eta and the ghosted temperature and writes both:

@@ -142,6 +142,7 @@ _PROTOS = {
     "pfg_pf_step_quench": (_I, [ctypes.POINTER(PfParams), ctypes.POINTER(Quench), _P, _P, _P, _P,
                                 _F, _P]),
     "pfg_heat_step": (_I, [ctypes.POINTER(HeatParams), _P, _P, _F, _F, _F, _F, _P]),
+    "pfg_heat_step_whole": (_I, [ctypes.POINTER(HeatParams), _P, _P, _F, _F, _F, _F, _P]),
     "pfg_heat_pf_step": (_I, [ctypes.POINTER(PfParams), ctypes.POINTER(HeatParams), _P, _P, _P,
                               _P, _P, _P, _F, _P]),
     "pfg_heat_pf_step_comp": (_I, [ctypes.POINTER(PfParams), ctypes.POINTER(HeatParams), _P, _P,

@@ -59,9 +59,8 @@ def update_T(T, xl, yl, x, y, P, dx, dy, dz, dt, gamma_args, out=None):
     nx, ny, nz = (s - 2 for s in T.shape)
     key = (id(x), id(y), float(dx), float(dy))
     if key not in _coord_cache:
-        xa = x.detach().cpu().numpy() if torch.is_tensor(x) else np.asarray(x)
-        ya = y.detach().cpu().numpy() if torch.is_tensor(y) else np.asarray(y)
-        xt, yt = xa[:, :, -1], ya[:, :, -1]
+        xt, yt = (a[:, :, -1].detach().cpu().numpy() if torch.is_tensor(a)
+                  else np.asarray(a)[:, :, -1] for a in (x, y))
         ex = xt[0, 0] + float(dx) * np.arange(nx)[:, None]
         ey = yt[0, 0] + float(dy) * np.arange(ny)[None, :]
         if not (np.allclose(xt, ex, rtol=1e-6, atol=1e-12) and np.allclose(yt, ey, rtol=1e-6,
@@ -72,9 +71,10 @@ def update_T(T, xl, yl, x, y, P, dx, dy, dz, dt, gamma_args, out=None):
     x_first, y_first = _coord_cache[key]
     h = make_heat_params(gamma_args, nx, ny, nz, dx, dy, dz, x_first, y_first,
                          layout=_lib.LAYOUT_XYZ)
-    if out is None:
-        out = T.clone()  # edge/corner ghosts are carried over unchanged
-    st = lib.pfg_heat_step(ctypes.byref(h), _lib.ptr(T), _lib.ptr(out), float(xl), float(yl),
+    step = lib.pfg_heat_step
+    if out is None:  # edge/corner ghosts are carried over unchanged
+        out, step = torch.empty_like(T), lib.pfg_heat_step_whole
+    st = step(ctypes.byref(h), _lib.ptr(T), _lib.ptr(out), float(xl), float(yl),
                            float(P), float(dt),
                            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
     _lib.check(st, "pfg_heat_step")

@@ -85,6 +85,36 @@ def test_heat_layouts_agree_and_match_oracle(shape):
         np.testing.assert_array_equal(outs[0][sl[0], sl[1], :], Tx[sl[0], sl[1], :])
 
 
+@pytest.mark.parametrize("shape", [(19, 13, 7), (1, 1, 1), (8, 3, 40), (64, 50, 70)])
+def test_whole_field_entry(shape):
+    """``pfg_heat_step_whole`` (a new buffer, nothing copied first) writes what
+    ``pfg_heat_step`` into a copy of the field gives, every element, in both
+    axis orders; so does ``update_T`` with and without ``out``."""
+    from jax_am_gb300 import _lib
+    from jax_am_gb300.cfd.gamma import make_heat_params, update_T
+    import ctypes
+    nx, ny, nz = shape
+    g = dict(GAMMA_DEFAULTS)
+    rng = np.random.default_rng(17)
+    dx, dy, dz, dt = 1e-6, 1.2e-6, 0.9e-6, 1e-8
+    Tx = f32(rng.uniform(300.0, 2500.0, (nx + 2, ny + 2, nz + 2)))
+    lib = _lib.load()
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for layout, arr in ((_lib.LAYOUT_XYZ, Tx), (_lib.LAYOUT_ZYX, Tx.transpose(2, 1, 0))):
+        h = make_heat_params(g, nx, ny, nz, dx, dy, dz, layout=layout)
+        tin = torch.tensor(np.ascontiguousarray(arr), dtype=torch.float32, device="cuda")
+        ref, got = tin.clone(), torch.full_like(tin, float("nan"))
+        for entry, out in (("pfg_heat_step", ref), ("pfg_heat_step_whole", got)):
+            _lib.check(getattr(lib, entry)(ctypes.byref(h), _lib.ptr(tin), _lib.ptr(out), 5e-6,
+                                           4e-6, 180.0, dt, stream), entry)
+        assert torch.equal(ref, got)
+        if layout == _lib.LAYOUT_XYZ:
+            x, y, _ = np.meshgrid(*(d * (np.arange(n) + 0.5) for d, n in
+                                    ((dx, nx), (dy, ny), (dz, nz))), indexing="ij")
+            args = (5e-6, 4e-6, x, y, 180.0, dx, dy, dz, dt, g)
+            assert torch.equal(update_T(tin, *args), update_T(tin, *args, out=tin.clone()))
+
+
 def test_mushy_zone_edges_match_reference_division():
     """Latent heat enters cp exactly where the reference's float32 liquid
     fraction (clip(T, Ts, Tl) - Ts) / (Tl - Ts) lies strictly inside (0, 1):
