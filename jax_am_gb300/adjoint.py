@@ -43,6 +43,10 @@ class LaserTrackProblem:
         self.C = max(1, int(checkpoint_every))
         self.x_start, self.y = float(x_start), float(y)
         self.t_end = self.steps * self.dt * 2.0 + 1.0  # the track outlasts the run
+        # the device clock at each step: float32 dt summed in float64, in order
+        self.times = [0.0]
+        for _ in range(self.steps):
+            self.times.append(self.times[-1] + self.dt)
         p = self.p
         self.N = p.nx * p.ny * p.nz
         self.n = p.num_oris
@@ -65,19 +69,26 @@ class LaserTrackProblem:
                                        _lib.ptr(clk_in), _lib.ptr(clk_out), self.dt, _stream())
         _lib.check(st, "pfg_heat_pf_step")
 
-    def _run(self, h, eta, T, clk, steps, keep=None):
-        """Advance (eta, T, clk) by `steps` steps in double buffers; keep(k, eta, T)
-        is called with the state before each step."""
-        e = [eta.clone(), torch.empty_like(eta)]
-        t = [T.clone(), T.clone()]
-        c = [clk.clone(), torch.zeros_like(clk)]
-        cur = 0
+    def _advance(self, h, eta, T, k0, steps, keep_every):
+        """Advance (eta, T), the state of step ``k0``, by ``steps`` steps;
+        returns the final state and the kept ones, steps ``k0``, ``k0 +
+        keep_every``, ...  The states that are not kept alternate between two
+        buffers; nothing is copied and the inputs are not written."""
+        clk = torch.empty((2, 2), dtype=torch.int64, device="cuda")
+        _lib.check(self.lib.pfg_clock_set(_lib.ptr(clk[0]), self.times[k0], k0, _stream()),
+                   "pfg_clock_set")
+        kept, free = [], []
+        state, own = (eta, T), False  # own: the state's buffers may be written again
         for k in range(steps):
-            if keep is not None:
-                keep(k, e[cur], t[cur], c[cur])
-            self._step(h, e[cur], e[cur ^ 1], t[cur], t[cur ^ 1], c[cur], c[cur ^ 1])
-            cur ^= 1
-        return e[cur], t[cur], c[cur]
+            if k % keep_every == 0:
+                kept.append(state)
+                own = False
+            out = free.pop() if free else (torch.empty_like(eta), torch.empty_like(T))
+            self._step(h, state[0], out[0], state[1], out[1], clk[k & 1], clk[(k & 1) ^ 1])
+            if own:
+                free.append(state)
+            state, own = out, True
+        return state, kept
 
     def objective(self, eta, lam_seed=None):
         J = torch.zeros(1, dtype=torch.float64, device="cuda")
@@ -91,14 +102,8 @@ class LaserTrackProblem:
         self.P, self.v = float(P), float(v)
         h = self.heat_params(self.P, self.v)
         eta = eta0.to("cuda", torch.float32).reshape(self.N, self.n).contiguous()
-        clk = torch.zeros(2, dtype=torch.int64, device="cuda")
-        ckpt = []
-
-        def keep(k, e, T, c):
-            if k % self.C == 0:
-                ckpt.append((e.clone(), T.clone(), c.clone()))
-
-        eta_f, T_f, _ = self._run(h, eta, self.T_init, clk, self.steps, keep)
+        # the first checkpoint is a copy: the caller may write eta0 before gradient()
+        (eta_f, _), ckpt = self._advance(h, eta.clone(), self.T_init.clone(), 0, self.steps, self.C)
         self._ckpt = ckpt
         self._eta_final = eta_f
         return float(self.objective(eta_f).item())
@@ -116,21 +121,15 @@ class LaserTrackProblem:
         nbytes = int(self.lib.pfg_adjoint_scratch_bytes(ctypes.byref(self.p)))
         scratch = torch.empty(nbytes // 4 + 1, dtype=torch.float32, device="cuda")
         dt = self.dt
-        # the device clock at each step: float32 dt summed in float64, in order
-        times = [0.0]
-        for _ in range(self.steps):
-            times.append(times[-1] + dt)
         for seg in reversed(range(len(self._ckpt))):
             k0 = seg * self.C
             nseg = min(self.C, self.steps - k0)
-            states = []
-            e0, T0, c0 = self._ckpt[seg]
-            self._run(h, e0, T0, c0, nseg,
-                      keep=lambda k, e, T, c: states.append((e.clone(), T.clone())))
+            # the segment's states again (its last step's result is not needed)
+            last, states = self._advance(h, *self._ckpt[seg], k0, nseg - 1, 1)
+            states.append(last)
             for j in reversed(range(nseg)):
-                k = k0 + j
-                t = times[k]
-                e_k, T_k = states[j]
+                t = self.times[k0 + j]
+                e_k, T_k = states.pop()
                 st = self.lib.pfg_adjoint_step(
                     ctypes.byref(self.p), ctypes.byref(h), _lib.ptr(e_k), _lib.ptr(T_k), t, dt,
                     _lib.ptr(lam), _lib.ptr(Tb), _lib.ptr(lam2), _lib.ptr(Tb2), _lib.ptr(scratch),
@@ -139,7 +138,7 @@ class LaserTrackProblem:
                 lam, lam2 = lam2, lam
                 Tb, Tb2 = Tb2, Tb
         g = grads.cpu().numpy()
-        return float(g[0]), float(g[1]), lam.clone()
+        return float(g[0]), float(g[1]), lam
 
 
 class HeatPFObjective(torch.autograd.Function):

@@ -15,6 +15,13 @@
 // the anisotropy term (a depends on e = eta(+d) - eta(-d)) transposes to minus
 // the central difference of v_d = lam Lg kappa' L da/de_d with an odd
 // extension at a Neumann face; periodic axes wrap in both.
+//
+// Without anisotropy (a = 1) u at a neighbour is its lam times one number per
+// cell, so one launch per cell (heat transpose and the cell coefficients) and
+// one per order parameter do the step and no (N, n) field is written but
+// lam_out: at 1M cells, n = 10, 63 us against 230 us with the fields written and
+// gathered.  With anisotropy the fields u, v and loc go through memory (kernels
+// A, B, then C).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -45,6 +52,14 @@ struct AdjArgs {
   float* loc;          // (N, n)
   float* muPF;         // (N) dt * sum_i lam_i dR_i/dT
   float* mask;         // (N) 0 where liquid forcing zeroed the cell, else 1
+  // isotropic step, per cell: Lg kappa' (0 where liquid), Lg m_g / ad_hoc,
+  // 2 (1 - zeta)^2 (-1 where liquid) and d Lg / dT
+  float* q;
+  float* g;
+  float* om2;
+  float* dLg;
+  float* alpha;        // (N) thermal diffusivity k / (rho cp)
+  int tx, ty, zc, tiles_x, tiles_y;  // isotropic step: tile and planes per unit
   double* grads;       // [dJ/dP, dJ/dv]
   float dirs[3 * PFG_MAX_ORIS * 3];
 };
@@ -87,9 +102,27 @@ __device__ __forceinline__ float cell_sum(float v, const AdjLanes& l) {
   return __shfl_sync(0xffffffffu, v, min(lane - l.g, 31));
 }
 
+// The temperature-only quantities of the forward step's arithmetic and their
+// derivatives.
+struct AdjTemp {
+  float om, Lg, dLg, dz;
+  bool liquid;
+};
+__device__ __forceinline__ AdjTemp adj_temp(const PFConsts& pc, float T) {
+  AdjTemp r;
+  const bool clipped = T > 2000.f;
+  const float Tc = clipped ? 2000.f : T;
+  const float xz = Tc / pc.T_liq - 1.f;
+  const float zeta = (xz > 0.f) ? 0.f : (xz < 0.f) ? 1.f : (xz == 0.f) ? 0.5f : xz;
+  r.om = 1.f - zeta;
+  r.Lg = pc.L0 * expf(pc.neg_Qg_over_R / Tc);
+  r.dLg = clipped ? 0.f : r.Lg * (-pc.neg_Qg_over_R) / (Tc * Tc);
+  r.dz = clipped ? 0.f : dzeta_dT(pc, xz);
+  r.liquid = pc.force && T > pc.liquid_limit;
+  return r;
+}
+
 // ---- kernel A: u, v, the local term and the temperature sensitivity --------
-// ANISO = false (A = 0): v is identically zero and is neither written nor read.
-template <bool ANISO>
 __global__ void __launch_bounds__(256) adj_pf_local_kernel(const __grid_constant__ AdjArgs a) {
   const int ncell = a.nx * a.ny * a.nz;  // host checks < 2^31
   const int n = a.n;
@@ -108,15 +141,9 @@ __global__ void __launch_bounds__(256) adj_pf_local_kernel(const __grid_constant
     const int z = cc / xy, r = cc - z * xy, y = r / a.nx, x = r - y * a.nx;
     // temperature-only quantities (as in the forward fast kernels)
     const float T = a.Tg[(int64_t)(z + 1) * gsz + (int64_t)(y + 1) * gsy + x + 1];
-    const bool clipped = T > 2000.f;
-    const float Tc = clipped ? 2000.f : T;
-    const float xz = Tc / a.pc.T_liq - 1.f;
-    const float zeta = (xz > 0.f) ? 0.f : (xz < 0.f) ? 1.f : (xz == 0.f) ? 0.5f : xz;
-    const float om = 1.f - zeta;
-    const float Lg = a.pc.L0 * expf(a.pc.neg_Qg_over_R / Tc);
-    const float dLg = clipped ? 0.f : Lg * (-a.pc.neg_Qg_over_R) / (Tc * Tc);
-    const float dz = clipped ? 0.f : dzeta_dT(a.pc, xz);
-    const bool liquid = a.pc.force && T > a.pc.liquid_limit;
+    const AdjTemp tq = adj_temp(a.pc, T);
+    const float om = tq.om, Lg = tq.Lg, dLg = tq.dLg, dz = tq.dz;
+    const bool liquid = tq.liquid;
     const int64_t base = (int64_t)z * sz + (int64_t)y * sy + (int64_t)x * n;
     // per-cell sums
     float s = 0.f, ld = 0.f;
@@ -156,39 +183,35 @@ __global__ void __launch_bounds__(256) adj_pf_local_kernel(const __grid_constant
         const float L = a.pc.wx * ((vxp - e) + (vxm - e)) + a.pc.wy * ((vyp - e) + (vym - e)) +
                         a.pc.wz * ((vzp - e) + (vzm - e));
         float an = 1.f, dax = 0.f, day = 0.f, daz = 0.f;
-        if (ANISO) {
-          const float ex = vxp - vxm, ey = vyp - vym, ez = vzp - vzm;
-          const float ee = ex * ex + ey * ey + ez * ez;
-          float pbest = 0.f, m = -1.f;
-          int kbest = 0;
+        const float ex = vxp - vxm, ey = vyp - vym, ez = vzp - vzm;
+        const float ee = ex * ex + ey * ey + ez * ez;
+        float pbest = 0.f, m = -1.f;
+        int kbest = 0;
 #pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const float* d = &a.dirs[(k * n + i) * 3];
-            const float pk = d[0] * ex + d[1] * ey + d[2] * ez;
-            if (pk * pk > m) { m = pk * pk; pbest = pk; kbest = k; }
-          }
-          const float c2 = (ee > 0.f) ? m / ee : 1.f;
-          if (c2 < 1.f) {
-            const float s2 = 1.f - c2;
-            an = 1.f + A * (c2 * c2 + s2 * s2);
-            // da/de = A (4 c2 - 2) * 2 (p* d* - c2 e) / ee
-            const float f = A * (4.f * c2 - 2.f) * 2.f / ee;
-            const float* d = &a.dirs[(kbest * n + i) * 3];
-            dax = f * (pbest * d[0] - c2 * ex);
-            day = f * (pbest * d[1] - c2 * ey);
-            daz = f * (pbest * d[2] - c2 * ez);
-          } else {
-            an = 1.f + A;
-          }
+        for (int k = 0; k < 3; ++k) {
+          const float* d = &a.dirs[(k * n + i) * 3];
+          const float pk = d[0] * ex + d[1] * ey + d[2] * ez;
+          if (pk * pk > m) { m = pk * pk; pbest = pk; kbest = k; }
+        }
+        const float c2 = (ee > 0.f) ? m / ee : 1.f;
+        if (c2 < 1.f) {
+          const float s2 = 1.f - c2;
+          an = 1.f + A * (c2 * c2 + s2 * s2);
+          // da/de = A (4 c2 - 2) * 2 (p* d* - c2 e) / ee
+          const float f = A * (4.f * c2 - 2.f) * 2.f / ee;
+          const float* d = &a.dirs[(kbest * n + i) * 3];
+          dax = f * (pbest * d[0] - c2 * ex);
+          day = f * (pbest * d[1] - c2 * ey);
+          daz = f * (pbest * d[2] - c2 * ez);
+        } else {
+          an = 1.f + A;
         }
         const float gg = e * (K - 3.f * e * e);
         const float Q = Lg * kap;
         a.u[base + i] = lam * Q * an;
-        if (ANISO) {
-          a.v[base + i] = lam * Q * L * dax;
-          a.v[Nn + base + i] = lam * Q * L * day;
-          a.v[2 * Nn + base + i] = lam * Q * L * daz;
-        }
+        a.v[base + i] = lam * Q * L * dax;
+        a.v[Nn + base + i] = lam * Q * L * day;
+        a.v[2 * Nn + base + i] = lam * Q * L * daz;
         a.loc[base + i] = liquid ? 0.f : -Lg * mg * (lam * (K - 9.f * e * e) + 8.f * e * ld);
         mu += lam * (dLg * (-mg * gg + kap * an * L) + Lg * mg * 4.f * om * e * dz);
       }
@@ -202,7 +225,6 @@ __global__ void __launch_bounds__(256) adj_pf_local_kernel(const __grid_constant
 }
 
 // ---- kernel B: the adjoint of the stencil terms, gathered per element --------
-template <bool ANISO>
 __global__ void __launch_bounds__(256) adj_pf_gather_kernel(const __grid_constant__ AdjArgs a) {
   const int ncell = a.nx * a.ny * a.nz;
   const int n = a.n;
@@ -241,19 +263,149 @@ __global__ void __launch_bounds__(256) adj_pf_gather_kernel(const __grid_constan
       const float lapu = a.pc.wx * (a.u[off[0] + i] + a.u[off[1] + i] - 2.f * uc) +
                          a.pc.wy * (a.u[off[2] + i] + a.u[off[3] + i] - 2.f * uc) +
                          a.pc.wz * (a.u[off[4] + i] + a.u[off[5] + i] - 2.f * uc);
-      float dvx = 0.f, dvy = 0.f, dvz = 0.f;
-      if (ANISO) {
-        dvx = sgn[1] * a.v[off[1] + i] - sgn[0] * a.v[off[0] + i];
-        dvy = sgn[3] * a.v[Nn + off[3] + i] - sgn[2] * a.v[Nn + off[2] + i];
-        dvz = sgn[5] * a.v[2 * Nn + off[5] + i] - sgn[4] * a.v[2 * Nn + off[4] + i];
-      }
+      const float dvx = sgn[1] * a.v[off[1] + i] - sgn[0] * a.v[off[0] + i];
+      const float dvy = sgn[3] * a.v[Nn + off[3] + i] - sgn[2] * a.v[Nn + off[2] + i];
+      const float dvz = sgn[5] * a.v[2 * Nn + off[5] + i] - sgn[4] * a.v[2 * Nn + off[4] + i];
       a.lam_out[base + i] =
           m * a.lam_in[base + i] + a.dt * (a.loc[base + i] + lapu - (dvx + dvy + dvz));
     }
   }
 }
 
+// ---- the isotropic step of the order parameters --------------------------------
+// A block marches a tile of tx x ty cells (12 warps: two along x, six along y;
+// a warp holds 32 / tpc cells) through zc planes, with the planes below and at
+// the cell in registers; the in-plane neighbours come from L1, where the block
+// has just loaded them as the plane ahead.  The sums over a cell's orientations
+// and every product that the two-launch form stores are rounded as there.
+constexpr int kIsoThreads = 384, kIsoWarpsX = 2, kIsoWarpsY = 6;
+
+// Two consecutive values of a cell (the second absent at the end of an odd n).
+template <bool VEC>
+__device__ __forceinline__ float2 load_two(const float* p, bool second) {
+  if constexpr (VEC) return __ldg(reinterpret_cast<const float2*>(p));
+  else return make_float2(__ldg(p), second ? __ldg(p + 1) : 0.f);
+}
+
+// VEC: n even and the fields 8-byte aligned.
+template <bool VEC>
+__global__ void __launch_bounds__(kIsoThreads, 2)
+adj_pf_iso_kernel(const __grid_constant__ AdjArgs a) {
+  const int n = a.n;
+  const AdjLanes ln = adj_lanes(n);
+  const int warp = threadIdx.x >> 5;
+  const int per_plane = a.tiles_x * a.tiles_y;
+  const int chunk = blockIdx.x / per_plane, tile = blockIdx.x - chunk * per_plane;
+  const int tyi = tile / a.tiles_x, txi = tile - tyi * a.tiles_x;
+  const int xr = txi * a.tx + (warp % kIsoWarpsX) * ln.cpw + ln.cw;
+  const int yr = tyi * a.ty + warp / kIsoWarpsX;
+  const bool valid = ln.active && xr < a.nx && yr < a.ny;
+  const int x = valid ? xr : 0, y = valid ? yr : 0;  // idle lanes shadow cell (0, 0)
+  const int zb = chunk * a.zc, ze = min(zb + a.zc, a.nz);
+  const int i0 = valid ? 2 * ln.g : 0;
+  const bool second = i0 + 1 < n;
+  const int xy = a.nx * a.ny;
+  const int64_t sz = (int64_t)xy * n;
+  const int c0 = y * a.nx + x;
+  // in-plane neighbours: cells, and elements from the cell's
+  const int cxm = y * a.nx + nbr(x, -1, a.nx, a.bcx), cxp = y * a.nx + nbr(x, 1, a.nx, a.bcx);
+  const int cym = nbr(y, -1, a.ny, a.bcy) * a.nx + x, cyp = nbr(y, 1, a.ny, a.bcy) * a.nx + x;
+  const float mg = a.pc.mg_ad, kap = a.pc.kappa_ad;
+  auto u_of = [](float2 l, float q) { return make_float2(__fmul_rn(l.x, q), __fmul_rn(l.y, q)); };
+  const int64_t first = (int64_t)c0 * n + i0;
+  const float* eta = a.eta + first;
+  const float* lam = a.lam_in + first;
+  const int zl = nbr(zb, -1, a.nz, a.bcz);
+  float2 em = load_two<VEC>(eta + zl * sz, second), ec = load_two<VEC>(eta + zb * sz, second);
+  float2 um = u_of(load_two<VEC>(lam + zl * sz, second), a.q[(int64_t)zl * xy + c0]);
+  float2 lc = load_two<VEC>(lam + zb * sz, second);
+  float2 uc = u_of(lc, a.q[(int64_t)zb * xy + c0]);
+  eta += zb * sz;
+  lam += zb * sz;
+  // the host keeps a plane below 2^31 elements
+  const int nxm = (cxm - c0) * n, nxp = (cxp - c0) * n, nym = (cym - c0) * n, nyp = (cyp - c0) * n;
+  int cz = zb * xy + c0;
+  for (int z = zb; z < ze; ++z, eta += sz, lam += sz, cz += xy) {
+    const bool wraps = z + 1 == a.nz;  // the plane above: the next, this one or the first
+    const int64_t up_at = wraps ? (a.bcz ? -(int64_t)(a.nz - 1) * sz : 0) : sz;
+    const float2 ep = load_two<VEC>(eta + up_at, second), lp = load_two<VEC>(lam + up_at, second);
+    const float2 up = u_of(lp, a.q[cz + (wraps ? (a.bcz ? -(a.nz - 1) * xy : 0) : xy)]);
+    const float2 exm = load_two<VEC>(eta + nxm, second), exp_ = load_two<VEC>(eta + nxp, second);
+    const float2 eym = load_two<VEC>(eta + nym, second), eyp = load_two<VEC>(eta + nyp, second);
+    const float* qz = a.q + (cz - c0);
+    const float2 uxm = u_of(load_two<VEC>(lam + nxm, second), qz[cxm]);
+    const float2 uxp = u_of(load_two<VEC>(lam + nxp, second), qz[cxp]);
+    const float2 uym = u_of(load_two<VEC>(lam + nym, second), qz[cym]);
+    const float2 uyp = u_of(load_two<VEC>(lam + nyp, second), qz[cyp]);
+    const float Lgm = a.g[cz], o2 = a.om2[cz], dLg = a.dLg[cz];
+    const bool liquid = o2 < 0.f;
+    // per-cell sums
+    float s = 0.f, ld = 0.f;
+    if (valid) {
+      s = fmaf(ec.x, ec.x, s);
+      ld = fmaf(lc.x, ec.x, ld);
+      if (second) {
+        s = fmaf(ec.y, ec.y, s);
+        ld = fmaf(lc.y, ec.y, ld);
+      }
+    }
+    s = cell_sum(s, ln);
+    ld = cell_sum(ld, ln);
+    const float K = 4.f * s + o2 - 1.f;
+    // d zeta / dT: only at T == T_liquidus exactly (1 - zeta = 1/2)
+    float om = 0.f, dz = 0.f;
+    if (o2 == 0.5f) {
+      const AdjTemp tq = adj_temp(
+          a.pc, a.Tg[((int64_t)(z + 1) * (a.ny + 2) + (y + 1)) * (a.nx + 2) + x + 1]);
+      om = tq.om;
+      dz = tq.dz;
+    }
+    float mu = 0.f;
+    auto element = [&](float e, float vxm, float vxp, float vym, float vyp, float vzm, float vzp,
+                       float l, float u, float u0, float u1, float u2, float u3, float u4,
+                       float u5) {
+      const float lamm = liquid ? 0.f : l;
+      const float L = a.pc.wx * ((vxp - e) + (vxm - e)) + a.pc.wy * ((vyp - e) + (vym - e)) +
+                      a.pc.wz * ((vzp - e) + (vzm - e));
+      const float gg = e * (K - 3.f * e * e);
+      const float loc =
+          liquid ? 0.f : __fmul_rn(-Lgm, fmaf(8.f * e, ld, __fmul_rn(lamm, K - 9.f * e * e)));
+      mu += lamm * (dLg * (-mg * gg + kap * L) + Lgm * 4.f * om * e * dz);
+      const float lapu = a.pc.wx * (u0 + u1 - 2.f * u) + a.pc.wy * (u2 + u3 - 2.f * u) +
+                         a.pc.wz * (u4 + u5 - 2.f * u);
+      return __fadd_rn(liquid ? 0.f : l, __fmul_rn(a.dt, loc + lapu));
+    };
+    float2 out;
+    out.x = element(ec.x, exm.x, exp_.x, eym.x, eyp.x, em.x, ep.x, lc.x, uc.x, uxm.x, uxp.x, uym.x,
+                    uyp.x, um.x, up.x);
+    if (second)
+      out.y = element(ec.y, exm.y, exp_.y, eym.y, eyp.y, em.y, ep.y, lc.y, uc.y, uxm.y, uxp.y,
+                      uym.y, uyp.y, um.y, up.y);
+    if (valid) {
+      float* o = a.lam_out + (lam - a.lam_in);
+      if constexpr (VEC) {
+        *reinterpret_cast<float2*>(o) = out;
+      } else {
+        o[0] = out.x;
+        if (second) o[1] = out.y;
+      }
+    }
+    mu = cell_sum(valid ? mu : 0.f, ln);
+    if (valid && ln.g == 0) {  // on top of the heat transpose's part
+      const int64_t idx = ((int64_t)(z + 1) * (a.ny + 2) + (y + 1)) * (a.nx + 2) + x + 1;
+      a.Tb_out[idx] = a.Tb_out[idx] + __fmul_rn(a.dt, mu);
+    }
+    em = ec;
+    ec = ep;
+    um = uc;
+    lc = lp;
+    uc = up;
+  }
+}
+
 // ---- kernel C: heat transpose, one thread per interior cell -------------------
+// ISO: the isotropic step adds its part of dJ/dT afterwards.  The neighbours'
+// diffusivities (two divisions each) come from the launch before.
 struct HeatLocal {
   float k, dk, cp, dcp, alpha, dalpha;
 };
@@ -270,15 +422,35 @@ __device__ __forceinline__ HeatLocal heat_local(const HeatConsts& H, float T) {
   return r;
 }
 
+// Per-cell numbers of the step: the diffusivity, and with ISO the cell
+// coefficients of the isotropic step.
+template <bool ISO>
+__global__ void __launch_bounds__(256) adj_cell_kernel(const __grid_constant__ AdjArgs a) {
+  const int ncell = a.nx * a.ny * a.nz, xy = a.nx * a.ny;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) {
+    const int z = c / xy, rem = c - z * xy, y = rem / a.nx, x = rem - y * a.nx;
+    const float T = a.Tg[((int64_t)(z + 1) * (a.ny + 2) + (y + 1)) * (a.nx + 2) + x + 1];
+    a.alpha[c] = heat_local(a.hc, T).alpha;
+    if constexpr (ISO) {
+      const AdjTemp tq = adj_temp(a.pc, T);
+      a.q[c] = tq.liquid ? 0.f : tq.Lg * a.pc.kappa_ad;
+      a.g[c] = tq.Lg * a.pc.mg_ad;
+      a.om2[c] = tq.liquid ? -1.f : 2.f * tq.om * tq.om;
+      a.dLg[c] = tq.dLg;
+    }
+  }
+}
+
+template <bool ISO>
 __global__ void __launch_bounds__(256) adj_heat_kernel(const __grid_constant__ AdjArgs a) {
   const HeatConsts& H = a.hc;
-  const long long ncell = (long long)a.nx * a.ny * a.nz;
+  const int ncell = a.nx * a.ny * a.nz;  // host checks (with room for the stride)
+  const int xy = a.nx * a.ny;
   const int64_t sx = 1, sy = a.nx + 2, sz = (int64_t)(a.ny + 2) * (a.nx + 2);
   const float R2 = a.hc.two_over_r2;
   double gP = 0.0, gv = 0.0;
-  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < ncell;
-       c += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(c % a.nx), y = (int)((c / a.nx) % a.ny), z = (int)(c / ((long long)a.nx * a.ny));
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) {
+    const int z = c / xy, rem = c - z * xy, y = rem / a.nx, x = rem - y * a.nx;
     const int64_t idx = (int64_t)(z + 1) * sz + (int64_t)(y + 1) * sy + x + 1;
     const float Tc = a.Tg[idx];
     const HeatLocal hl = heat_local(H, Tc);
@@ -290,6 +462,7 @@ __global__ void __launch_bounds__(256) adj_heat_kernel(const __grid_constant__ A
     const float d[6] = {H.dx, H.dx, H.dy, H.dy, H.dz, H.dz};
     const float r2[6] = {1.f / H.dx2, 1.f / H.dx2, 1.f / H.dy2, 1.f / H.dy2, 1.f / H.dz2, 1.f / H.dz2};
     float Nv[6], dGdT[6], dGdG[6], dGdB[6], B[6];
+#pragma unroll
     for (int f = 0; f < 6; ++f) {
       const float Gold = a.Tg[idx + st[f]];
       dGdT[f] = dGdG[f] = dGdB[f] = 0.f;
@@ -318,6 +491,7 @@ __global__ void __launch_bounds__(256) adj_heat_kernel(const __grid_constant__ A
                       (Nv[4] - 2.f * Tc + Nv[5]) * r2[4];
     float mu = mu_c * (1.f + dt * hl.dalpha * lap -
                        2.f * dt * hl.alpha * (r2[0] + r2[2] + r2[4]));
+#pragma unroll
     for (int f = 0; f < 6; ++f) {
       if (face[f]) {
         const float w = mu_c * dt * hl.alpha * r2[f] + a.Tb_in[idx + st[f]];
@@ -331,12 +505,15 @@ __global__ void __launch_bounds__(256) adj_heat_kernel(const __grid_constant__ A
         }
       } else {
         // this cell is the neighbour m's Laplacian input with weight dt alpha_m / d^2
-        const float Tm = Nv[f];
-        const HeatLocal hm = heat_local(H, Tm);
-        mu += a.Tb_in[idx + st[f]] * dt * hm.alpha * r2[f];
+        const int cs[6] = {-1, 1, -a.nx, a.nx, -xy, xy};
+        mu += a.Tb_in[idx + st[f]] * dt * a.alpha[c + cs[f]] * r2[f];
       }
     }
-    a.Tb_out[idx] = mu + a.muPF[c];
+    if constexpr (ISO) {
+      a.Tb_out[idx] = mu;
+    } else {
+      a.Tb_out[idx] = mu + a.muPF[c];
+    }
   }
   // block reduction of the two gradient components, one atomic per block
   __shared__ double sP[8], sv[8];
@@ -357,27 +534,36 @@ __global__ void __launch_bounds__(256) adj_heat_kernel(const __grid_constant__ A
 }
 
 // ---- objective J = mean over cells of sum_i w_i eta_i^2 and its seed ----------
+// A thread sums its elements as pairs of float32 (error-free products and
+// sums, about 48 bits): a float64 operation per element would cost this GPU
+// more than the memory traffic (85 us against 42 MB of eta).
+template <bool SEED>
 __global__ void __launch_bounds__(256)
 objective_kernel(const float* __restrict__ eta, const float* __restrict__ w, long long ncell, int n,
                  double* __restrict__ J, float* __restrict__ lam) {
-  double acc = 0.0;
-  const long long total = ncell * n;
   const float inv = 1.f / (float)ncell;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % n);
-    const float v = eta[e];
-    acc += (double)w[i] * (double)v * (double)v;
-    if (lam) lam[e] = 2.f * w[i] * v * inv;
+  const long long total = ncell * n;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  int i = (int)(e % n);
+  const int di = (int)(stride % n);
+  DF acc{0.f, 0.f};
+  for (; e < total; e += stride) {
+    const float v = __ldg(eta + e), wi = __ldg(w + i);
+    acc = df_add(acc, df_mul_f(two_prod(v, v), wi));
+    if (SEED) lam[e] = 2.f * wi * v * inv;
+    i += di;
+    if (i >= n) i -= n;
   }
+  double sum = (double)acc.h + (double)acc.l;
   __shared__ double s[8];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = sum;
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += s[i];
+    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += s[k];
     atomicAdd(J, t / (double)ncell);
   }
 }
@@ -442,20 +628,55 @@ extern "C" int pfg_adjoint_step(const pfg_pf_params* p, const pfg_heat_params* h
   for (int i = 0; i < 3 * p->num_oris * 3; ++i) a.dirs[i] = p->grain_dirs[i];
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const DeviceInfo& d = device_info();
-  const int cpw = 32 / ((p->num_oris + 1) / 2);  // cells per warp of kernels A and B
+  const int cpw = 32 / ((p->num_oris + 1) / 2);  // cells per warp of the element kernels
+  const int cell_blocks = (int)std::min<int64_t>((N + 255) / 256, (int64_t)d.sm_count * 16);
+  // the isotropic kernel's in-plane offsets are 32-bit (a plane of 2^31 elements
+  // takes the other kernels)
+  if (!(a.pc.aniso > 0.f) && (int64_t)p->nx * p->ny * p->num_oris < ((int64_t)1 << 31)) {
+    a.q = sc;
+    a.g = sc + N;
+    a.om2 = sc + 2 * N;
+    a.dLg = sc + 3 * N;
+    a.alpha = sc + 4 * N;
+    a.tx = kIsoWarpsX * cpw;
+    a.ty = kIsoWarpsY;
+    a.tiles_x = (p->nx + a.tx - 1) / a.tx;
+    a.tiles_y = (p->ny + a.ty - 1) / a.ty;
+    // planes per unit: fewest plane times over the waves of blocks (two per SM),
+    // counting two for the planes beside a unit's
+    const int64_t tiles = (int64_t)a.tiles_x * a.tiles_y, slots = 2LL * d.sm_count;
+    double least = 1e300;
+    for (int zch = 1; zch <= p->nz && zch <= 4096; ++zch) {
+      const int zc = (p->nz + zch - 1) / zch;
+      const int64_t units = tiles * ((p->nz + zc - 1) / zc);
+      const double cost = (double)((units + slots - 1) / slots) * (zc + 2.0);
+      if (cost < least - 1e-9) {
+        least = cost;
+        a.zc = zc;
+      }
+    }
+    const int64_t units = tiles * ((p->nz + a.zc - 1) / a.zc);
+    if (units >= ((int64_t)1 << 31)) return PFG_ERR_SHAPE;
+    adj_cell_kernel<true><<<cell_blocks, 256, 0, s>>>(a);
+    adj_heat_kernel<true><<<cell_blocks, 256, 0, s>>>(a);
+    const bool vec = p->num_oris % 2 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(eta) | reinterpret_cast<uintptr_t>(lam_in) |
+                       reinterpret_cast<uintptr_t>(lam_out)) & 7u) == 0;
+    if (vec) adj_pf_iso_kernel<true><<<(unsigned)units, kIsoThreads, 0, s>>>(a);
+    else adj_pf_iso_kernel<false><<<(unsigned)units, kIsoThreads, 0, s>>>(a);
+    return record_cuda(cudaGetLastError());
+  }
   const int warps_blocks =
       (int)std::min<int64_t>((N + 8 * cpw - 1) / (8 * cpw), (int64_t)d.sm_count * 16);
-  const bool aniso = a.pc.aniso > 0.f;
-  if (aniso) adj_pf_local_kernel<true><<<warps_blocks, 256, 0, s>>>(a);
-  else adj_pf_local_kernel<false><<<warps_blocks, 256, 0, s>>>(a);
+  adj_pf_local_kernel<<<warps_blocks, 256, 0, s>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return record_cuda(e);
-  if (aniso) adj_pf_gather_kernel<true><<<warps_blocks, 256, 0, s>>>(a);
-  else adj_pf_gather_kernel<false><<<warps_blocks, 256, 0, s>>>(a);
+  adj_pf_gather_kernel<<<warps_blocks, 256, 0, s>>>(a);
   e = cudaGetLastError();
   if (e != cudaSuccess) return record_cuda(e);
-  const int cell_blocks = (int)std::min<int64_t>((N + 255) / 256, (int64_t)d.sm_count * 16);
-  adj_heat_kernel<<<cell_blocks, 256, 0, s>>>(a);
+  a.alpha = a.u;  // u has been gathered
+  adj_cell_kernel<false><<<cell_blocks, 256, 0, s>>>(a);
+  adj_heat_kernel<false><<<cell_blocks, 256, 0, s>>>(a);
   return record_cuda(cudaGetLastError());
 }
 
@@ -468,7 +689,8 @@ extern "C" int pfg_objective(const pfg_pf_params* p, const float* eta, const flo
   const long long ncell = (long long)p->nx * p->ny * p->nz;
   const int blocks = (int)std::min<long long>((ncell * p->num_oris + 255) / 256,
                                               (long long)device_info().sm_count * 8);
-  objective_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      eta, w, ncell, p->num_oris, J, lam_seed);
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (lam_seed) objective_kernel<true><<<blocks, 256, 0, s>>>(eta, w, ncell, p->num_oris, J, lam_seed);
+  else objective_kernel<false><<<blocks, 256, 0, s>>>(eta, w, ncell, p->num_oris, J, nullptr);
   return record_cuda(cudaGetLastError());
 }

@@ -104,3 +104,33 @@ def test_adjoint_matches_float64_autograd_and_fd(aniso, steps, ckpt):
     assert rfP <= GRAD_RTOL and rfv <= GRAD_RTOL and rfe <= GRAD_RTOL
     from jax_am_gb300 import _lib
     assert _lib.device_error() == 0
+
+
+@pytest.mark.parametrize("shape,n,ckpt,aniso", [((13, 7, 5), 10, 3, 0.0), ((25, 6, 4), 5, 4, 0.0),
+                                                ((3, 13, 9), 33, 7, 0.0), ((4, 5, 2), 64, 1, 0.0),
+                                                ((9, 7, 5), 7, 3, 0.15)])
+def test_adjoint_tile_edges(shape, n, ckpt, aniso):
+    """Partial tiles, odd orientation counts (a lane with one orientation) and
+    one cell per warp, against float64 autograd to 1e-3 relative (float32
+    fields: about 1e-6); a second gradient() of the same forward(), after the
+    caller has overwritten eta0, gives the same."""
+    from jax_am_gb300.adjoint import LaserTrackProblem
+    steps = 7
+    poly, eta, Tg, pf_args, oargs, g, w = _setup(aniso, steps, ckpt, shape, n)
+    dt, x_start, y, P0, v0 = float(np.float32(3e-8)), 1e-6, 2e-6, 2.0, 0.8
+    prob = LaserTrackProblem(pf_args, poly, g, w, dt, steps, x_start, y, checkpoint_every=ckpt,
+                             T_init=torch.tensor(Tg))
+    e0 = torch.tensor(eta, dtype=torch.float32, device="cuda")
+    J = prob.forward(P0, v0, e0)
+    e0.zero_()
+    gP, gv, ge = prob.gradient()
+    gP2, gv2, ge2 = prob.gradient()
+    assert torch.equal(ge, ge2) and abs(gP - gP2) <= 1e-12 * abs(gP)
+    leaves = [torch.tensor(x, dtype=torch.float64, requires_grad=True) for x in (P0, v0, eta)]
+    Jt = _torch_J(*leaves, torch.tensor(Tg), oargs, g, torch.tensor(w),
+                  torch.tensor(poly.unique_grain_directions), steps, dt, x_start, y, shape)
+    Jt.backward()
+    rP, rv, re = (x.grad.numpy() for x in leaves)
+    assert abs(J - Jt.item()) <= 1e-5 * abs(Jt.item())
+    assert abs(gP - rP) <= 1e-3 * abs(rP) and abs(gv - rv) <= 1e-3 * abs(rv)
+    assert np.linalg.norm(ge.double().cpu().numpy() - re) <= 1e-3 * np.linalg.norm(re)
