@@ -71,6 +71,32 @@ int set_tune(int key, int value) {
   }
 }
 
+// A unit of zc planes takes about zc + 1.6 plane times beside another CTA on its
+// SM (the prologue waits for three planes), and 0.8 zc + 1.4 alone (measured
+// on GB300: 5.6 and 4.45 us a plane for the compensated laser step).  Whole
+// rounds of 2 sm_count units, then the rest, alone if there is an SM for each.
+// Against the earlier rule (waves of zc + 1/2, at least four planes a unit, or
+// eight in the warp planner), per step: 64 x 64 x 32 x 20 moving gradient 13.8
+// -> 11.2 us (2 planes a unit instead of 4), 100 x 50 x 25 x 20 laser 31.9 ->
+// 25.6 us (3 instead of 5), 128 x 128 x 64 x 10 46.0 -> 41.9 us (16 instead of 8).
+int plan_planes(long tiles, int nz, int sm_count) {
+  const long slots = 2L * std::max(1, sm_count);
+  int best = nz;
+  double least = 1e300;
+  for (int zch = 1; zch <= nz; ++zch) {
+    const int zc = (nz + zch - 1) / zch;
+    const long units = tiles * ((nz + zc - 1) / zc), rest = units % slots;
+    const double cost = (double)(units / slots) * (zc + 1.6) +
+                        (rest == 0 ? 0.0 : rest <= slots / 2 ? 0.8 * zc + 1.4 : zc + 1.6);
+    if (cost < least - 1e-9) {
+      least = cost;
+      best = zc;
+    }
+    if (zch > 1024) break;  // the gain of ever thinner chunks has long ended
+  }
+  return best;
+}
+
 bool plan_warp_tiles(int nx, int ny, int nz, int n, int sm_count, int max_smem_per_sm,
                      TilePlan* out) {
   return plan_warp_tiles_budget(nx, ny, nz, n, sm_count,
@@ -142,6 +168,7 @@ bool plan_warp_tiles_ex(int nx, int ny, int nz, int n, int sm_count, size_t budg
   zch = std::max(1L, std::min(zch, (long)std::max(1, nz / 8)));
   if (g_tune_zchunks) zch = std::min<long>(g_tune_zchunks, nz);
   t.zc = (int)((nz + zch - 1) / zch);
+  if (ctas_per_sm == 2 && !g_tune_zchunks) t.zc = plan_planes(tiles, nz, sm_count);
   t.zchunks = (nz + t.zc - 1) / t.zc;
   t.units = tiles * t.zchunks;
   *out = t;

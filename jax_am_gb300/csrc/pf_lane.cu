@@ -521,20 +521,7 @@ bool plan_lane_tiles(int nx, int ny, int nz, int n, int sm_count, int max_smem_p
   t.tiles_x = (nx + tx - 1) / tx;
   t.tiles_y = (ny + ty - 1) / ty;
   const long tiles = (long)t.tiles_x * t.tiles_y;
-  const long slots_gpu = (long)kLaneCTAs * sm_count;
-  // z chunks: a wave of CTAs lasts about (planes per unit + 1/2) plane times
-  // (the prologue); pick the chunking with the fewest plane times in all
-  int best_zc = nz;
-  double best = 1e300;
-  for (int zch = 1; zch <= std::max(1, nz / 4); ++zch) {
-    const int zc = (nz + zch - 1) / zch;
-    const long units = tiles * ((nz + zc - 1) / zc);
-    const double cost = (double)((units + slots_gpu - 1) / slots_gpu) * (zc + 0.5);
-    if (cost < best - 1e-9) {
-      best = cost;
-      best_zc = zc;
-    }
-  }
+  int best_zc = plan_planes(tiles, nz, sm_count);
   if (zchunks_override > 0) best_zc = (nz + std::min(zchunks_override, nz) - 1) /
                                       std::min(zchunks_override, nz);
   t.zc = best_zc;

@@ -57,6 +57,9 @@ __device__ __forceinline__ void end_step(const StepArgs& a, double t) {
 
 struct TilePlan;
 int set_tune(int key, int value);
+// Planes per unit of a z-marching kernel that keeps two CTAs per SM: the split
+// of nz with the shortest schedule of its units (pf_fast.cu).
+int plan_planes(long tiles, int nz, int sm_count);
 // Warp-per-cells kernel (pf_fast.cu).
 bool plan_warp_tiles(int nx, int ny, int nz, int n, int sm_count, int max_smem_per_sm,
                      TilePlan* out);
