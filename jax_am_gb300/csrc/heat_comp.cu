@@ -91,7 +91,9 @@ heat_comp_kernel(const __grid_constant__ StepArgs a) {
     DF Tn = c;
     // warp-uniform choice, as in the fused kernel
     if (__any_sync(0xffffffffu, valid && (tmax > a.hd.hot || z == nz - 1))) {
-      if (valid)
+      if (!__any_sync(0xffffffffu, on_face && valid))
+        Tn = heat_core_df(a.hc, a.hd, c, n);
+      else if (valid)
         Tn = heat_update_df_accurate(a.hc, a.hd, c, n, gx, gy, z, xld, yld, Pw, a.T_out,
                                      a.T_lo_out, idx, 1, gsy, gsz);
     } else if (__any_sync(0xffffffffu, on_face && valid)) {

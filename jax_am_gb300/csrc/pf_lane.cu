@@ -362,7 +362,9 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
           // warp-uniform choice: DF arithmetic where the temperature is far
           // from ambient or the beam heats the top face
           if (__any_sync(0xffffffffu, valid && (tmax > a.hd.hot || z == a.nz - 1))) {
-            if (valid)
+            if (!__any_sync(0xffffffffu, on_face && valid))
+              Tn = heat_core_df(a.hc, a.hd, c, n);
+            else if (valid)
               Tn = heat_update_df_accurate(a.hc, a.hd, c, n, gx, gy, z, xld, yld, Pw, a.T_out,
                                            a.T_lo_out, idx, 1, gsy, gsz);
           } else if (__any_sync(0xffffffffu, on_face && valid)) {

@@ -372,7 +372,11 @@ HeatDF make_heat_df(const pfg_heat_params& h, float dt) {
   d.rd2[0] = df_split(1.0 / ((double)h.dx * (double)h.dx));
   d.rd2[1] = df_split(1.0 / ((double)h.dy * (double)h.dy));
   d.rd2[2] = df_split(1.0 / ((double)h.dz * (double)h.dz));
-  d.dt = DF{dt, 0.f};
+  d.k1dt = df_split(0.0163 * (double)dt);
+  d.k0dt = df_split(4.5847 * (double)dt);
+  d.c1r = df_split(0.2441 * (double)h.rho);
+  d.c0r = df_split(338.39 * (double)h.rho);
+  d.lr = df_split((double)h.latent * (double)h.rho);
   d.hot = h.T0 + 50.f;
   return d;
 }
