@@ -441,6 +441,20 @@ int64_t pfg_grain_scratch_bytes(const pfg_pf_params* p);
 int pfg_grains(const pfg_pf_params* p, const int32_t* ori, const float* T, int T_ghosted,
                int32_t* grain_of_cell, pfg_grain* grains, int64_t max_grains, int64_t* num_grains,
                void* scratch, int64_t scratch_bytes, void* stream);
+/* Cell count and PCA aspect ratio of each grain (utils.py:286-310: 2 l0 / (l1 +
+ * l2), l the square roots of the descending eigenvalues of the cell centres'
+ * covariance; 1 below 5 cells, infinite for a line of cells) from the records
+ * that pfg_grains enqueued before: entry g for grain g < min(*num_grains,
+ * max_grains).  Exact covariance numerators, float64 from there. */
+typedef struct pfg_grain_shape {
+  int64_t first_cell;
+  int32_t ori;
+  int32_t reserved;
+  int64_t cells;
+  double aspect_ratio;
+} pfg_grain_shape;
+int pfg_grain_shapes(const pfg_grain* grains, const int64_t* num_grains, int64_t max_grains,
+                     pfg_grain_shape* out, void* stream);
 /* Renumber a grain_of_cell array in place: labels[i] = rank[labels[i]], -1
  * stays.  rank: device int32 per grain number (the caller's order of the
  * records). */

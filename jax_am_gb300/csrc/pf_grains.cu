@@ -143,18 +143,26 @@ __global__ void __launch_bounds__(kGrainThreads) grain_tile_kernel(const GrainAr
   }
   __syncthreads();
   // Two rows' runs unite at the first cell of each overlap: where either run
-  // starts.
+  // starts.  First within the z planes; then, every run pointing at its plane's
+  // root again (the chains stay short), across them.
+  auto unite = [&](int zl, int back) {  // with the row `back` rows before
+    const int r = zl * kTileY + yl, c = r * 32 + lane, d = c - 32 * back;
+    if (s_L[c] >= 0 && s_L[d] >= 0 && s_ori[d] == s_ori[c] &&
+        ((s_start[r] | s_start[r - back]) >> lane & 1u))
+      merge<false>(s_L, c, d);
+  };
+  if (yl > 0)
+#pragma unroll
+    for (int zl = 0; zl < kTileZ; ++zl) unite(zl, 1);
+  __syncthreads();
 #pragma unroll
   for (int zl = 0; zl < kTileZ; ++zl) {
     const int r = zl * kTileY + yl, c = r * 32 + lane;
-    if (s_L[c] < 0) continue;
-    if (yl > 0 && s_L[c - 32] >= 0 && s_ori[c - 32] == s_ori[c] &&
-        ((s_start[r] | s_start[r - 1]) >> lane & 1u))
-      merge<false>(s_L, c, c - 32);
-    if (zl > 0 && s_L[c - 32 * kTileY] >= 0 && s_ori[c - 32 * kTileY] == s_ori[c] &&
-        ((s_start[r] | s_start[r - kTileY]) >> lane & 1u))
-      merge<false>(s_L, c, c - 32 * kTileY);
+    if ((s_start[r] >> lane & 1u) && s_L[c] >= 0) s_L[c] = find_root<false>(s_L, c);
   }
+  __syncthreads();
+#pragma unroll
+  for (int zl = 1; zl < kTileZ; ++zl) unite(zl, kTileY);
   __syncthreads();
 #pragma unroll
   for (int zl = 0; zl < kTileZ; ++zl) {
@@ -398,6 +406,68 @@ __global__ void __launch_bounds__(kGrainThreads) grain_moments_kernel(const Grai
 }
 static_assert(kTable == 128, "the table's hash takes 7 bits");
 
+// Eigenvalues of a symmetric 3 x 3 matrix (a00, a11, a22, a01, a02, a12) by cyclic
+// Jacobi rotations (Golub and Van Loan's symmetric Schur decomposition).
+__device__ void eigenvalues3(double* a) {
+  for (int sweep = 0; sweep < 12; ++sweep) {
+    if (a[3] == 0.0 && a[4] == 0.0 && a[5] == 0.0) return;
+    for (int k = 0; k < 3; ++k) {
+      // rotate the plane (p, q); r is the third axis
+      const int p = k == 2 ? 1 : 0, q = k == 0 ? 1 : 2, r = 3 - p - q;
+      const int pq = p + q + 2, pr = p + r + 2, qr = q + r + 2;
+      const double apq = a[pq];
+      if (apq == 0.0) continue;
+      const double tau = (a[q] - a[p]) / (2.0 * apq);
+      const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+      const double c = 1.0 / sqrt(1.0 + t * t), s = t * c;
+      a[p] -= t * apq;
+      a[q] += t * apq;
+      a[pq] = 0.0;
+      const double arp = a[pr], arq = a[qr];
+      a[pr] = c * arp - s * arq;
+      a[qr] = s * arp + c * arq;
+    }
+  }
+}
+
+// A grain's aspect ratio from its exact moments (utils.py:286-310): covariance
+// of the cell centres (ddof = 1, numerators exact in 128-bit integers), square
+// roots of its eigenvalues in descending order l0, l1, l2: 2 l0 / (l1 + l2); 1
+// below 5 cells.
+static_assert(sizeof(pfg_grain_shape) == 32, "four words per grain");
+__global__ void __launch_bounds__(128) grain_shapes_kernel(const pfg_grain* grains,
+                                                           const int64_t* num_grains,
+                                                           int64_t max_grains,
+                                                           pfg_grain_shape* out) {
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t K = *num_grains < max_grains ? *num_grains : max_grains;
+  if (g >= K) return;
+  const pfg_grain& G = grains[g];
+  const long long c = G.cells;
+  double ratio = 1.0;
+  if (c >= 5) {
+    const double den = (double)c * (double)(c - 1);  // exact below 2^53
+    double a[6];
+    const int pi[6] = {0, 1, 2, 0, 0, 1}, qi[6] = {0, 1, 2, 1, 2, 2};
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      const __int128 v = (__int128)c * G.sum2[m] - (__int128)G.sum[pi[m]] * G.sum[qi[m]];
+      // the magnitude's two halves, one rounding (exact below 2^53)
+      const unsigned __int128 u = v < 0 ? -(unsigned __int128)v : (unsigned __int128)v;
+      const double d = fma((double)(unsigned long long)(u >> 64), 18446744073709551616.0,
+                           (double)(unsigned long long)u);
+      a[m] = (v < 0 ? -d : d) / den;
+    }
+    eigenvalues3(a);
+    double l[3];
+    for (int m = 0; m < 3; ++m) l[m] = sqrt(a[m] > 0.0 ? a[m] : 0.0);
+    const double l0 = fmax(fmax(l[0], l[1]), l[2]), l2 = fmin(fmin(l[0], l[1]), l[2]);
+    const double l1 = fmax(fmin(l[0], l[1]), fmin(fmax(l[0], l[1]), l[2]));
+    ratio = 2.0 * l0 / (l1 + l2);  // collinear: infinite
+  }
+  out[g] = pfg_grain_shape{G.first_cell, G.ori, 0, c, ratio};
+}
+
 // labels[i] = rank[labels[i]] in place (-1 stays)
 __global__ void __launch_bounds__(kGrainThreads) grain_relabel_kernel(int64_t N,
                                                                       const int32_t* rank,
@@ -471,6 +541,21 @@ extern "C" int pfg_grains(const pfg_pf_params* p, const int32_t* ori, const floa
   grain_offsets_kernel<<<1, kGrainThreads, 0, s>>>(a, nchunks);
   grain_number_kernel<<<nchunks, kGrainThreads, 0, s>>>(a, nchunks);
   grain_moments_kernel<<<tiles, kGrainThreads, 0, s>>>(a);
+  return record_cuda(cudaGetLastError());
+}
+
+extern "C" int pfg_grain_shapes(const pfg_grain* grains, const int64_t* num_grains,
+                                int64_t max_grains, pfg_grain_shape* out, void* stream) {
+  if (max_grains < 0) return PFG_ERR_PARAM;
+  if (!num_grains || (max_grains > 0 && (!grains || !out))) return PFG_ERR_NULL;
+  if ((reinterpret_cast<uintptr_t>(grains) | reinterpret_cast<uintptr_t>(out)) % 8 != 0)
+    return PFG_ERR_ALIGN;
+  if (!device_info().ok) return PFG_ERR_NO_DEVICE;
+  const int64_t blocks = (max_grains + 127) / 128;
+  if (blocks > 0x7fffffff) return PFG_ERR_SHAPE;
+  if (blocks)
+    grain_shapes_kernel<<<(unsigned)blocks, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+        grains, num_grains, max_grains, out);
   return record_cuda(cudaGetLastError());
 }
 

@@ -8,10 +8,10 @@ aspect ratio ``2 l0 / (l1 + l2)`` (``l`` = square roots of the explained
 variances of its volume-weighted cell centres, descending), or 1 when it has
 fewer than 5 cells.
 
-``segment_grains`` runs the connected-component labelling and the per-grain
-moment sums on the GPU (``pfg_grains``); the volumes and aspect ratios follow
-on the host from each grain's exact integer moments (one 3 x 3 eigenproblem
-per grain).  ``process_eta`` is the drop-in for the reference function,
+``segment_grains`` runs the connected-component labelling, the per-grain
+moment sums (``pfg_grains``) and the aspect ratios (one 3 x 3 eigenproblem per
+grain from its exact integer moments, ``pfg_grain_shapes``) on the GPU; the host
+sorts the grains.  ``process_eta`` is the drop-in for the reference function,
 reading the solution that ``PFSolver.write_sols`` wrote.
 
 A collinear grain (all cells on one line) has two zero variances: its
@@ -55,44 +55,33 @@ def _cell_volume(pf_args):
 
 def aspect_ratios(records):
     """Aspect ratios of grains given as (cells, sums, sums2) records of their
-    integer moments (see ``_aspect_ratios``)."""
-    if not len(records):
-        return np.ones(0)
-    c, s, s2 = (np.array([r[k] for r in records], dtype=np.int64) for k in range(3))
-    return _aspect_ratios(c, s, s2)
-
-
-def _aspect_ratios(cells, sums, sums2):
-    """Aspect ratios from the grains' integer moments ((K,), (K, 3) and (K, 6)
-    int64): the covariance of the cell centres (ddof = 1, exact integer
-    numerators), its eigenvalues in descending order, 2 sqrt(ev0) / (sqrt(ev1)
-    + sqrt(ev2)); 1 below 5 cells (utils.py:286-310).  Cell-centre scaling (h,
-    the volume weights) cancels."""
-    ar = np.ones(len(cells))
-    big = np.flatnonzero(cells >= 5)
-    if not len(big):
+    integer moments: the covariance of the cell centres (ddof = 1, exact
+    integer numerators), its eigenvalues in descending order, 2 sqrt(ev0) /
+    (sqrt(ev1) + sqrt(ev2)); 1 below 5 cells (utils.py:286-310).  Cell-centre
+    scaling (h, the volume weights) cancels.  ``segment_grains`` takes them from
+    the GPU (``pfg_grain_shapes``)."""
+    ar = np.ones(len(records))
+    big = [k for k in range(len(records)) if records[k][0] >= 5]
+    if not big:
         return ar
-    c, s, s2 = cells[big], sums[big], sums2[big]
-    # c * sum(ab) - sum(a) sum(b) over c (c - 1), correctly rounded: integers
-    # below 2^53 are exact in int64 and float64, the few others take Python's
-    limit = 2.0 ** 53
-    exact = (c.astype(np.float64) * np.maximum(s2.max(axis=1), c) < limit) & (
-        s.max(axis=1).astype(np.float64) ** 2 < limit)
-    a, b = (0, 1, 2, 0, 0, 1), (0, 1, 2, 1, 2, 2)
-    with np.errstate(over="ignore"):
-        v = (c[:, None] * s2 - s[:, a] * s[:, b]) / (c * (c - 1)).astype(np.float64)[:, None]
-    for j in np.flatnonzero(~exact):
-        cj = int(c[j])
-        for m in range(6):
-            v[j, m] = (cj * int(s2[j, m]) - int(s[j, a[m]]) * int(s[j, b[m]])) / (cj * (cj - 1))
-    cov = np.empty((len(big), 3, 3))
-    cov[:, a, b] = v
-    cov[:, b, a] = v
+    cov = np.zeros((len(big), 3, 3))
+    pairs = ((0, 0, 0), (1, 1, 1), (2, 2, 2), (0, 1, 3), (0, 2, 4), (1, 2, 5))
+    for j, k in enumerate(big):
+        c, s, s2 = records[k]
+        c = int(c)
+        den = c * (c - 1)
+        for a, b, m in pairs:
+            # exact: (c * sum(ab) - sum(a) sum(b)) / (c (c - 1)), big Python ints
+            v = (c * int(s2[m]) - int(s[a]) * int(s[b])) / den
+            cov[j, a, b] = cov[j, b, a] = v
     ev = np.linalg.eigvalsh(cov)[:, ::-1]
     ln = np.sqrt(np.maximum(ev, 0.0))
     with np.errstate(divide="ignore", invalid="ignore"):
         ar[big] = 2.0 * ln[:, 0] / (ln[:, 1] + ln[:, 2])
     return ar
+
+
+_FIRST_ROWS = 4096  # grains that the first copy to the host has room for
 
 
 def segment_grains(pf_args, ori_inds, T, T_ghosted=False, max_grains=None):
@@ -126,39 +115,47 @@ def segment_grains(pf_args, ori_inds, T, T_ghosted=False, max_grains=None):
     stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
     nbytes = int(lib.pfg_grain_scratch_bytes(ctypes.byref(params)))
     scratch = torch.empty(max(nbytes, 16), dtype=torch.uint8, device="cuda")
-    count = torch.zeros(1, dtype=torch.int64, device="cuda")
     labels = torch.empty(N, dtype=torch.int32, device="cuda")
-    rec = ctypes.sizeof(_lib.Grain)
+    rec = ctypes.sizeof(_lib.Grain) // 8
     cap = int(max_grains) if max_grains else max(1024, N // 64)
     while True:
-        buf = torch.empty(max(cap, 1) * rec // 8, dtype=torch.int64, device="cuda")
+        buf = torch.empty(max(cap, 1) * rec, dtype=torch.int64, device="cuda")
+        # the count, then a row of four words per grain: one copy brings both
+        shapes = torch.empty((cap + 1, 4), dtype=torch.int64, device="cuda")
         st = lib.pfg_grains(ctypes.byref(params), _lib.ptr(ori), _lib.ptr(T), int(T_ghosted),
-                            _lib.ptr(labels), _lib.ptr(buf), cap, _lib.ptr(count),
+                            _lib.ptr(labels), _lib.ptr(buf), cap, _lib.ptr(shapes),
                             _lib.ptr(scratch), scratch.numel(), stream)
         _lib.check(st, "pfg_grains")
-        K = int(count.item())
+        st = lib.pfg_grain_shapes(_lib.ptr(buf), _lib.ptr(shapes), cap,
+                                  ctypes.c_void_p(shapes.data_ptr() + 32), stream)
+        _lib.check(st, "pfg_grain_shapes")
+        host = shapes[: min(cap, _FIRST_ROWS) + 1].cpu()
+        K = int(host[0, 0])
         if K <= cap:
             break
         cap = K
-    raw = buf[: K * rec // 8].cpu().numpy().view(np.int64).reshape(K, rec // 8)
+    if K >= len(host):
+        host = shapes[: K + 1].cpu()
+    raw = host[1: K + 1].numpy()
     # column 1 holds (ori, reserved) as two little-endian int32
-    first, ori_g = raw[:, 0], (raw[:, 1] & 0xFFFFFFFF).astype(np.int64)
-    cells, sums, sums2 = raw[:, 2], raw[:, 3:6], raw[:, 6:12]
-    order = np.lexsort((first, ori_g))  # by orientation, then smallest cell index
-    rank = np.empty(K, dtype=np.int32)
-    rank[order] = np.arange(K, dtype=np.int32)
+    ori_g = raw[:, 1] & 0xFFFFFFFF
+    # by orientation, then smallest cell index (the order of the rows)
+    order = np.argsort(ori_g, kind="stable")
     if K:
+        rank = np.empty(K, dtype=np.int32)
+        rank[order] = np.arange(K, dtype=np.int32)
         rank_t = torch.from_numpy(rank).to("cuda")
         st = lib.pfg_grain_relabel(N, _lib.ptr(rank_t), _lib.ptr(labels), stream)
         _lib.check(st, "pfg_grain_relabel")
-    cells, sums, sums2 = cells[order], sums[order], sums2[order]
+    raw = raw[order]
+    cells = np.ascontiguousarray(raw[:, 2])
     return {
         "labels": labels,
-        "ori": ori_g[order].astype(np.int64),
-        "first_cell": first[order],
+        "ori": ori_g[order],
+        "first_cell": np.ascontiguousarray(raw[:, 0]),
         "cells": cells,
         "volumes": cells * _cell_volume(pf_args),
-        "aspect_ratios": _aspect_ratios(cells, sums, sums2),
+        "aspect_ratios": np.ascontiguousarray(raw[:, 3]).view(np.float64),
     }
 
 
