@@ -517,69 +517,127 @@ pf_inspect_kernel(const __grid_constant__ DiagArgs a) {
 // ---------------------------------------------------------------------------
 // The full record (free energy, per-orientation mass and the inspect metrics)
 // with one lane per cell, for num_oris a multiple of 4 up to 20.  A warp takes
-// 32 consecutive cells at a time: their n floats are contiguous, so it stages
-// them in its shared-memory slice with 16-byte cp.async copies (the next
-// chunk's copies in flight while this one is reduced), then each lane reduces
-// its cell's orientations in order: sum eta^2, sum eta^4, the gradient energy
-// against the forward neighbours (x + 1 from the staged chunk where it is in
-// it, y + 1 and z + 1 from L2), the argmax, and the per-orientation mass in
-// the lane's own compensated sums.  No per-cell shuffles.  Per-block partial
-// records as for pf_diag_kernel.
+// 32 consecutive cells at a time.  Their n floats are contiguous, and so are
+// those of the cells' y + 1 and z + 1 neighbours (the 32 cells nx and nx * ny
+// further on): it stages all three, with the one cell that x + 1 adds, in its
+// shared-memory slice with 16-byte cp.async copies (the next chunk's in flight
+// while this one is reduced).  Each lane then reduces its cell's orientations
+// in order: sum eta^2, sum eta^4, the gradient energy against the forward
+// neighbours, the argmax, and the per-orientation mass in the lane's own
+// compensated sums.  No per-cell shuffles.  Per-block partial records as for
+// pf_diag_kernel.
+//
+// Bound: instruction issue at 14 warps an SM (the mass sums take 40 registers
+// a lane).  Lanes that load their y + 1 and z + 1 cells themselves touch 20
+// lines an instruction (262 us at 8M cells, n = 20); staged 242; with packed
+// pairs of floats for everything but the argmax 219 (4.3 TB/s of DRAM reads,
+// 546 instructions a chunk, 52 % of the issue slots).  A vote to skip vectors
+// that are zero in the warp's cells and neighbours (most are) costs more than
+// it saves, as no vector's arithmetic then overlaps another's loads: 270.
 // ---------------------------------------------------------------------------
-constexpr int kCellWarps = 8;
 constexpr int kCellMaxVec = 5;  // n <= 20 (the per-lane mass sums fit in registers)
+constexpr int kCellSlots = 33 + 32 + 32;  // cells of a staged chunk: own and x + 1, y + 1, z + 1
+// as many warps as their two staged chunks leave room for, two blocks an SM
+__host__ __device__ constexpr int cell_warps(int nv) { return nv >= 5 ? 7 : 8; }
+
+// Two floats in a 64-bit register pair, and the packed operations on them.
+struct F2 {
+  unsigned long long b = 0;
+};
+struct F2x2 {
+  F2 h[2];
+};
+__device__ __forceinline__ float f2_lo(F2 a) { return __uint_as_float((unsigned)a.b); }
+__device__ __forceinline__ float f2_hi(F2 a) { return __uint_as_float((unsigned)(a.b >> 32)); }
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.b) : "l"(a.b), "l"(b.b));
+  return d;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.b) : "l"(a.b), "l"(b.b));
+  return d;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.b) : "l"(a.b), "l"(b.b), "l"(c.b));
+  return d;
+}
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {  // one rounding: -1 * b is exact
+  return f2_fma(b, F2{0xbf800000bf800000ull}, a);
+}
+__device__ __forceinline__ F2x2 load_f2(const float4* p) {
+  const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(p);
+  return F2x2{{F2{u.x}, F2{u.y}}};
+}
 
 template <int NV>  // num_oris = 4 NV
-__global__ void __launch_bounds__(32 * kCellWarps, 2)
+__global__ void __launch_bounds__(32 * cell_warps(NV), 2)
 pf_diag_cells_kernel(const __grid_constant__ DiagArgs a) {
   extern __shared__ float4 s_chunks[];  // per warp: two chunks of 32 cells
-  __shared__ double s_mass[kCellWarps][4 * kCellMaxVec];
-  __shared__ double s_energy[kCellWarps], s_maxT[kCellWarps];
-  __shared__ long long s_cnt[kCellWarps][3];
+  constexpr int kWarps = cell_warps(NV);
+  __shared__ double s_mass[kWarps][4 * kCellMaxVec];
+  __shared__ double s_energy[kWarps], s_maxT[kWarps];
+  __shared__ long long s_cnt[kWarps][3];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int n = 4 * NV, nv = NV;
   const int ncell = a.nx * a.ny * a.nz;  // < 2^31 (host checks)
   const int xy = a.nx * a.ny;
   const int64_t gsy = a.nx + 2, gsz = (int64_t)(a.ny + 2) * (a.nx + 2);
-  float4* buf0 = s_chunks + (size_t)warp * 2 * 32 * nv;
-  float4* buf1 = buf0 + 32 * nv;
+  float4* const slice = s_chunks + (size_t)warp * 2 * kCellSlots * nv;
   const float4* eta4 = reinterpret_cast<const float4*>(a.eta);
   const int nchunks = (int)(((int64_t)ncell + 31) / 32);
-  const int cstride = gridDim.x * kCellWarps;
+  const int cstride = gridDim.x * kWarps;
 
-  float mh[n], ml[n];  // compensated mass per orientation
+  F2 mh[n / 2], ml[n / 2];  // compensated mass per orientation
 #pragma unroll
-  for (int i = 0; i < n; ++i) mh[i] = ml[i] = 0.f;
+  for (int i = 0; i < n / 2; ++i) mh[i] = ml[i] = F2{};
   CSum energy;
   float maxT = -INFINITY;
   int changed = 0, liquid = 0, nonfinite = 0;
 
-  // the chunk's y + 1 and z + 1 neighbours are the 32 cells nx and nx * ny
-  // further on: their 128-byte lines (at most 21 for n <= 20) are prefetched
-  // into L1 one chunk ahead, so the lanes' 16-byte loads of them hit L1
-  const int64_t nbytes = (int64_t)ncell * n * 4;
-  const char* eta_b = reinterpret_cast<const char*>(a.eta);
-  auto prefetch_span = [&](int64_t cell0) {
-    const int64_t b0 = (cell0 * n * 4) & ~(int64_t)127;
-    const int64_t b = b0 + (int64_t)lane * 128;
-    if (lane * 128 < 32 * n * 4 + 128 && b < nbytes)
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(eta_b + b));
+  // cells [c, c + 32) of the field, as far as there are any
+  auto copy = [&](int64_t c, float4* dst) {
+    const float4* src = eta4 + c * nv + lane;
+    dst += lane;
+    if (c + 32 <= ncell) {
+#pragma unroll
+      for (int k = 0; k < nv; ++k) cp_async<16>(dst + 32 * k, src + 32 * k);
+    } else {
+      const int64_t tot = (ncell - c) * nv;
+      for (int k = 0; lane + k < tot; k += 32) cp_async<16>(dst + k, src + k);
+    }
   };
-  auto stage = [&](int chunk, float4* dst) {
-    const int c0 = chunk * 32;
-    const int tot = min(32, ncell - c0) * nv;
-    const float4* src = eta4 + (int64_t)c0 * nv;
-    for (int j = lane; j < tot; j += 32) cp_async<16>(dst + j, src + j);
-    prefetch_span((int64_t)c0 + a.nx);
-    prefetch_span((int64_t)c0 + xy);
+  int sx = 0, sy = 0, sz = 0, sprev = 0;  // of the staged chunk
+  float sT = 0.f;
+  auto stage = [&](int chunk, float4* dst, int& x, int& y, int& z, float& T, int& prev) {
+    const int64_t c0 = (int64_t)chunk * 32;
+    copy(c0, dst);
+    if (lane < nv && c0 + 32 < ncell)
+      cp_async<16>(dst + 32 * nv + lane, eta4 + (c0 + 32) * nv + lane);
+    copy(c0 + a.nx, dst + 33 * nv);
+    copy(c0 + xy, dst + 65 * nv);
+    const int c = (int)c0 + lane;
+    if (c < ncell) {
+      z = fast_div(c, a.div_xy);
+      const int r = c - z * xy;
+      y = fast_div(r, a.div_x);
+      x = r - y * a.nx;
+      T = __ldg(a.T + (a.T_ghosted ? (int64_t)(z + 1) * gsz + (int64_t)(y + 1) * gsy + x + 1
+                                   : (int64_t)c));
+      if (a.argmax0) prev = __ldg(a.argmax0 + c);
+    }
   };
-  int ch = blockIdx.x * kCellWarps + warp;
-  if (ch < nchunks) stage(ch, buf0);
+  int ch = blockIdx.x * kWarps + warp;
+  if (ch < nchunks) stage(ch, slice, sx, sy, sz, sT, sprev);
   cp_async_commit();
   for (int it = 0; ch < nchunks; ch += cstride, ++it) {
-    float4* cur = (it & 1) ? buf1 : buf0;
-    float4* nxt = (it & 1) ? buf0 : buf1;
-    if (ch + cstride < nchunks) stage(ch + cstride, nxt);
+    float4* cur = slice + ((it & 1) ? kCellSlots * nv : 0);
+    const int x = sx, y = sy, z = sz, prev = sprev;
+    const float T = sT;
+    if (ch + cstride < nchunks)
+      stage(ch + cstride, slice + ((it & 1) ? 0 : kCellSlots * nv), sx, sy, sz, sT, sprev);
     cp_async_commit();
     cp_async_wait(1);  // this chunk has landed; the next may stay in flight
     __syncwarp();
@@ -587,53 +645,53 @@ pf_diag_cells_kernel(const __grid_constant__ DiagArgs a) {
     const int cells = min(32, ncell - c0);
     if (lane < cells) {
       const int c = c0 + lane;
-      const int z = fast_div(c, a.div_xy), r = c - z * xy, y = fast_div(r, a.div_x);
-      const int x = r - y * a.nx;
-      const int64_t ti = a.T_ghosted ? (int64_t)(z + 1) * gsz + (int64_t)(y + 1) * gsy + x + 1
-                                     : (int64_t)c;
-      const float T = __ldg(a.T + ti);
       // forward neighbours under the boundary conditions (-1: the cell itself)
       const int cx = (x + 1 < a.nx) ? c + 1 : (a.bcx ? c - (a.nx - 1) : -1);
       const int cy = (y + 1 < a.ny) ? c + a.nx : (a.bcy ? c - (a.ny - 1) * a.nx : -1);
       const int cz = (z + 1 < a.nz) ? c + xy : (a.bcz ? c - (a.nz - 1) * xy : -1);
       const float4* e = cur + lane * nv;
-      const float4* ex = (cx == c + 1 && lane + 1 < cells) ? cur + (lane + 1) * nv
-                                                            : eta4 + (int64_t)(cx < 0 ? c : cx) * nv;
-      const float4* ey = eta4 + (int64_t)(cy < 0 ? c : cy) * nv;
-      const float4* ez = eta4 + (int64_t)(cz < 0 ? c : cz) * nv;
-      float s2 = 0.f, s4 = 0.f, gxx = 0.f, gyy = 0.f, gzz = 0.f, best = -INFINITY;
-      int bi = 0;
+      float4 *ey = cur + (33 + lane) * nv, *ez = cur + (65 + lane) * nv;
+      if (cy != c + a.nx) {  // at the last row or plane: the lane's own slot takes the neighbour
+        for (int v = 0; v < nv; ++v) ey[v] = (cy < 0) ? e[v] : __ldg(eta4 + (int64_t)cy * nv + v);
+      }
+      if (cz != c + xy) {
+        for (int v = 0; v < nv; ++v) ez[v] = (cz < 0) ? e[v] : __ldg(eta4 + (int64_t)cz * nv + v);
+      }
+      const float4* ex = (cx == c + 1) ? e + nv : (cx < 0 ? e : eta4 + (int64_t)cx * nv);
+      // two orientations at a time: each half of a pair rounds as the single
+      // operation does
+      F2 p2{}, p4{}, pxx{}, pyy{}, pzz{};
+      float best = -INFINITY;
+      int bv = 0;  // the first vector that holds the maximum
 #pragma unroll
       for (int v = 0; v < nv; ++v) {
-        {
-          const float4 u = e[v];
-          const float4 X = (cx < 0) ? u : ex[v];
-          const float4 Y = (cy < 0) ? u : __ldg(ey + v);
-          const float4 Z = (cz < 0) ? u : __ldg(ez + v);
-          const float uu[4] = {u.x, u.y, u.z, u.w}, xx[4] = {X.x, X.y, X.z, X.w};
-          const float yy[4] = {Y.x, Y.y, Y.z, Y.w}, zz[4] = {Z.x, Z.y, Z.z, Z.w};
+        const F2x2 u = load_f2(e + v), X = load_f2(ex + v);
+        const F2x2 Y = load_f2(ey + v), Z = load_f2(ez + v);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float q = uu[k];
-            const int i = 4 * v + k;
-            if (q > best) { best = q; bi = i; }
-            {  // mass: compensated sum (TwoSum)
-              const float sum = __fadd_rn(mh[i], q);
-              const float bp = __fsub_rn(sum, mh[i]);
-              const float ap = __fsub_rn(sum, bp);
-              ml[i] = __fadd_rn(ml[i], __fadd_rn(__fsub_rn(mh[i], ap), __fsub_rn(q, bp)));
-              mh[i] = sum;
-            }
-            const float qq = q * q;
-            s2 += qq;
-            s4 = fmaf(qq, qq, s4);
-            const float gx = xx[k] - q, gy = yy[k] - q, gz = zz[k] - q;
-            gxx = fmaf(gx, gx, gxx);
-            gyy = fmaf(gy, gy, gyy);
-            gzz = fmaf(gz, gz, gzz);
-          }
+        for (int k = 0; k < 2; ++k) {
+          const F2 q = u.h[k];
+          F2& hi = mh[2 * v + k];
+          const F2 sum = f2_add(hi, q);  // mass: compensated sum (TwoSum)
+          const F2 bp = f2_sub(sum, hi), ap = f2_sub(sum, bp);
+          ml[2 * v + k] = f2_add(ml[2 * v + k], f2_add(f2_sub(hi, ap), f2_sub(q, bp)));
+          hi = sum;
+          const F2 qq = f2_mul(q, q);
+          p2 = f2_add(p2, qq);
+          p4 = f2_fma(qq, qq, p4);
+          const F2 gx = f2_sub(X.h[k], q), gy = f2_sub(Y.h[k], q), gz = f2_sub(Z.h[k], q);
+          pxx = f2_fma(gx, gx, pxx);
+          pyy = f2_fma(gy, gy, pyy);
+          pzz = f2_fma(gz, gz, pzz);
         }
+        const float m = fmaxf(fmaxf(f2_lo(u.h[0]), f2_hi(u.h[0])),
+                              fmaxf(f2_lo(u.h[1]), f2_hi(u.h[1])));
+        if (m > best) { best = m; bv = v; }
       }
+      const float s2 = f2_lo(p2) + f2_hi(p2), s4 = f2_lo(p4) + f2_hi(p4);
+      const float gxx = f2_lo(pxx) + f2_hi(pxx), gyy = f2_lo(pyy) + f2_hi(pyy);
+      const float gzz = f2_lo(pzz) + f2_hi(pzz);
+      const float4 w = e[bv];  // the first orientation that attains it
+      int bi = 4 * bv + (w.x == best ? 0 : w.y == best ? 1 : w.z == best ? 2 : 3);
       const float g2 = fmaf(a.gwx, gxx, fmaf(a.gwy, gyy, a.gwz * gzz));
       // A non-finite value makes the sum of squares non-finite (so can a
       // finite value above 2^64; the exact pass below then finds no
@@ -658,7 +716,7 @@ pf_diag_cells_kernel(const __grid_constant__ DiagArgs a) {
       if (T >= a.tl_ge) ++liquid;
       if (T > maxT || isnan(T)) maxT = isnan(maxT) ? maxT : T;
       if (a.argmax_out) a.argmax_out[c] = bi;
-      if (a.argmax0 && __ldg(a.argmax0 + c) != bi) ++changed;
+      if (a.argmax0 && prev != bi) ++changed;
     }
     __syncwarp();  // this buffer is restaged in the next iteration but one
   }
@@ -679,7 +737,9 @@ pf_diag_cells_kernel(const __grid_constant__ DiagArgs a) {
 #pragma unroll
   for (int i = 0; i < n; ++i) {
     {
-      double m = (double)mh[i] + (double)ml[i];
+      const F2 H = mh[i / 2], L = ml[i / 2];
+      double m = (i & 1) ? (double)f2_hi(H) + (double)f2_hi(L)
+                         : (double)f2_lo(H) + (double)f2_lo(L);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
       if (lane == 0) s_mass[warp][i] = m;
@@ -696,13 +756,13 @@ pf_diag_cells_kernel(const __grid_constant__ DiagArgs a) {
   DiagPartial* out = a.partials + blockIdx.x;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     double sm = 0.0;
-    for (int w = 0; w < kCellWarps; ++w) sm += s_mass[w][i];
+    for (int w = 0; w < kWarps; ++w) sm += s_mass[w][i];
     out->mass[i] = sm;
   }
   if (threadIdx.x == 0) {
     double e2 = 0.0, t2 = -INFINITY;
     long long d0 = 0, d1 = 0, d2 = 0;
-    for (int w = 0; w < kCellWarps; ++w) {
+    for (int w = 0; w < kWarps; ++w) {
       e2 += s_energy[w];
       if (s_maxT[w] > t2 || isnan(s_maxT[w])) t2 = isnan(t2) ? t2 : s_maxT[w];
       d0 += s_cnt[w][0];
@@ -724,7 +784,7 @@ static cudaError_t launch_diag_cells_t(const DiagArgs& a, int nb, size_t smem, c
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  pf_diag_cells_kernel<NV><<<nb, 32 * kCellWarps, smem, s>>>(a);
+  pf_diag_cells_kernel<NV><<<nb, 32 * cell_warps(NV), smem, s>>>(a);
   return cudaSuccess;
 }
 
@@ -785,9 +845,10 @@ int launch_diag(const pfg_pf_params* p, const float* eta, const float* T, int T_
     // the lane-per-cell record: no more blocks than partial records or than
     // chunks of 32 cells per warp
     const long long nchunks = ((long long)a.nx * a.ny * a.nz + 31) / 32;
-    const long long need = (nchunks + kCellWarps - 1) / kCellWarps;
+    const int w = cell_warps(a.n / 4);
+    const long long need = (nchunks + w - 1) / w;
     nb = (int)(need < nb ? (need < 1 ? 1 : need) : nb);
-    const size_t smem = (size_t)kCellWarps * 2 * 32 * a.n * sizeof(float);
+    const size_t smem = (size_t)w * 2 * kCellSlots * a.n * sizeof(float);
     cudaError_t e = launch_diag_cells(a, nb, smem, s);
     if (e != cudaSuccess) return record_cuda(e);
   } else switch (diag_group(a.n)) {

@@ -48,6 +48,29 @@ def test_diag_vs_oracle(shape, n, bc):
     np.testing.assert_array_equal(am, np.argmax(eta.astype(np.float32), axis=1))
 
 
+@pytest.mark.parametrize("shape,n,bc", [((32, 1, 3), 20, ("periodic", "neumann", "neumann")),
+                                        ((33, 2, 2), 12, ("neumann", "periodic", "periodic")),
+                                        ((7, 9, 11), 16, ("periodic", "periodic", "neumann")),
+                                        ((65, 3, 1), 20, ("neumann", "neumann", "periodic"))])
+def test_diag_chunk_edges(shape, n, bc):
+    """Chunks of 32 cells that end at, before and after a row's end, mixed
+    boundary conditions, and values that are all negative (the maximum is
+    below the zeros of an absent cell)."""
+    from jax_am_gb300.phase_field.allen_cahn import PFSolver
+    poly, eta, T, pf_args, oargs, obc = pf_case(shape, n, 0.0, seed=21, bc=bc)
+    s = PFSolver(pf_args, poly)
+    eta = (eta - 2.0).astype(np.float32)
+    eta[:, n // 2] = eta[:, n - 1]  # ties
+    am0 = np.roll(eta, 1, axis=0)
+    d = s.diagnostics(eta, T, am0)
+    m = O.inspect(eta, am0, T, oargs["T_liquidus"])
+    assert d["n_ori_changed"] == round(m["pct_ori_changed"] * len(eta) / 100)
+    assert d["max_T"] == m["max_T"] and d["n_nonfinite"] == 0
+    np.testing.assert_allclose(d["mass"], eta.astype(np.float64).sum(axis=0), rtol=1e-12)
+    e_ref = O.free_energy(eta.astype(np.float64), T, oargs, None, obc)
+    assert d["energy"] == pytest.approx(e_ref, rel=ENERGY_RTOL)
+
+
 def test_inspect_sol_raises_on_nan(capsys):
     from jax_am_gb300.phase_field.allen_cahn import PFSolver
     poly, eta, T, pf_args, oargs, obc = pf_case((5, 5, 5), 4, 0.0, seed=13)
