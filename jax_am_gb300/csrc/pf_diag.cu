@@ -540,33 +540,9 @@ constexpr int kCellSlots = 33 + 32 + 32;  // cells of a staged chunk: own and x 
 // as many warps as their two staged chunks leave room for, two blocks an SM
 __host__ __device__ constexpr int cell_warps(int nv) { return nv >= 5 ? 7 : 8; }
 
-// Two floats in a 64-bit register pair, and the packed operations on them.
-struct F2 {
-  unsigned long long b = 0;
-};
 struct F2x2 {
   F2 h[2];
 };
-__device__ __forceinline__ float f2_lo(F2 a) { return __uint_as_float((unsigned)a.b); }
-__device__ __forceinline__ float f2_hi(F2 a) { return __uint_as_float((unsigned)(a.b >> 32)); }
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  F2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.b) : "l"(a.b), "l"(b.b));
-  return d;
-}
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-  F2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.b) : "l"(a.b), "l"(b.b));
-  return d;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.b) : "l"(a.b), "l"(b.b), "l"(c.b));
-  return d;
-}
-__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {  // one rounding: -1 * b is exact
-  return f2_fma(b, F2{0xbf800000bf800000ull}, a);
-}
 __device__ __forceinline__ F2x2 load_f2(const float4* p) {
   const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(p);
   return F2x2{{F2{u.x}, F2{u.y}}};

@@ -41,6 +41,38 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return r;
 }
 
+// Two floats in a 64-bit register pair, and the packed operations on them.
+struct F2 {
+  unsigned long long b = 0;
+};
+__device__ __forceinline__ float f2_lo(F2 a) { return __uint_as_float((unsigned)a.b); }
+__device__ __forceinline__ float f2_hi(F2 a) { return __uint_as_float((unsigned)(a.b >> 32)); }
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.b) : "l"(a.b), "l"(b.b));
+  return d;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.b) : "l"(a.b), "l"(b.b));
+  return d;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.b) : "l"(a.b), "l"(b.b), "l"(c.b));
+  return d;
+}
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {
+  F2 d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d.b) : "l"(a.b), "l"(b.b));
+  return d;
+}
+__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
+  F2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d.b) : "f"(lo), "f"(hi));
+  return d;
+}
+
 // Vector of V floats moved as one 4/8/16-byte access.
 template <int V>
 struct VecF {
