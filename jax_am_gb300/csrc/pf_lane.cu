@@ -50,55 +50,6 @@ __device__ __forceinline__ float quench_T(const StepArgs& a, int z, double t) {
   return (float)(a.q.T_base + a.q.grad * (zc - a.q.z0) - a.q.grad * a.q.vel * t);
 }
 
-// Folded update of one element (allen_cahn.py:42-51,58,60-85 with the
-// Euler step, :106-114).  Per cell, k = (A1, B1, C1, W):
-//   eta' = e (A1 + B1 e^2) + (C1 + W (cn + cn^2)) lap'
-// with A1 = 1 + cg K, B1 = -3 cg, C1 = cl wx (1 + A), W = 2 A cl wx,
-// lap' = (xp + xm) + ry (yp + ym) + rz (zp + zm) - 2 (1 + ry + rz) e, and
-// cn = -cos^2 of the smallest angle between the central difference and the
-// orientation's cube axes: cos^4 + sin^4 = 1 - 2 c2 (1 - c2) with
-// c2 = max_k (d_k . g)^2 / |g|^2 (allen_cahn.py:28-39); the third axis is
-// orthogonal to the first two, so (d_2 . g)^2 = |g|^2 - q0 - q1.  |g|^2
-// starts from 1e-30, so a zero gradient gives cn = 0: the reference's
-// NaN-to-zero rule (c2 = 1 gives the same factor), with no clamp.
-// Two orientations at a time, as packed pairs of floats (each half rounds as
-// the single operation does); the projections on the axes stay single, their
-// constant operands come from the parameters.  The kernel is bound by issue
-// slots and dependent instructions at 16 warps an SM, and a packed instruction
-// takes one slot: 408 us -> 391 us a fused step at 8M cells, n = 20; the
-// point-source step at 1M cells 55 -> 51 us.
-struct LaneLap {
-  F2 ry, rz, nm;
-};
-struct LaneCoef {
-  F2 x, y, z, w;
-};
-template <bool ANISO>
-__device__ __forceinline__ F2 lane_pair(const LaneLap& L, F2 e, F2 xm, F2 xp, F2 ym, F2 yp, F2 zm,
-                                        F2 zp, const float* d0, const float* d1,
-                                        const LaneCoef& k) {
-  const F2 lap = f2_fma(L.rz, f2_add(zp, zm),
-                        f2_fma(L.ry, f2_add(yp, ym), f2_fma(L.nm, e, f2_add(xp, xm))));
-  F2 u = k.z;
-  if constexpr (ANISO) {
-    const F2 gx = f2_sub(xp, xm), gy = f2_sub(yp, ym), gz = f2_sub(zp, zm);
-    const F2 ee = f2_fma(gx, gx, f2_fma(gy, gy, f2_fma(gz, gz, f2_pack(1e-30f, 1e-30f))));
-    auto dot = [&](const float* d) {
-      return f2_pack(fmaf(d[0], f2_lo(gx), fmaf(d[1], f2_lo(gy), d[2] * f2_lo(gz))),
-                     fmaf(d[3], f2_hi(gx), fmaf(d[4], f2_hi(gy), d[5] * f2_hi(gz))));
-    };
-    const F2 p0 = dot(d0), p1 = dot(d1);
-    const F2 q0 = f2_mul(p0, p0), q1 = f2_mul(p1, p1);
-    const F2 q2 = f2_sub(f2_sub(ee, q0), q1);
-    float ml, mh;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(ml) : "f"(f2_lo(q0)), "f"(f2_lo(q1)), "f"(f2_lo(q2)));
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(mh) : "f"(f2_hi(q0)), "f"(f2_hi(q1)), "f"(f2_hi(q2)));
-    const F2 cn = f2_pack(ml * rcp_approx(-f2_lo(ee)), mh * rcp_approx(-f2_hi(ee)));
-    u = f2_fma(k.w, f2_fma(cn, cn, cn), k.z);
-  }
-  return f2_fma(u, lap, f2_mul(e, f2_fma(k.y, f2_mul(e, e), k.x)));
-}
-
 // Per-cell folded coefficients from the temperature part and S.
 __device__ __forceinline__ float4 lane_fold(const PFConsts& c, const TempCoef& tc, float S) {
   if (tc.liquid != 0.f) return make_float4(0.f, 0.f, 0.f, 0.f);
@@ -274,13 +225,7 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
   const int64_t cell0 = (int64_t)gy * a.nx + gx;  // cell index within a plane
   const int64_t plane_cells = (int64_t)a.ny * a.nx;
 
-  LaneLap L;
-  {
-    const float ry = a.pc.wy / a.pc.wx, rz = a.pc.wz / a.pc.wx, nm = -2.f * (1.f + ry + rz);
-    L.ry = f2_pack(ry, ry);
-    L.rz = f2_pack(rz, rz);
-    L.nm = f2_pack(nm, nm);
-  }
+  const LapPair L = lap_pair(a.pc);
   float xl = 0.f, yl = 0.f, Pw = 0.f;
   DF xld{0.f, 0.f}, yld{0.f, 0.f};
   if constexpr (HEAT) {
@@ -431,8 +376,7 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
       // the skip below needs finite coefficients in every cell of the warp
       const bool kfinite = __all_sync(0xffffffffu, !valid || (isfinite(k.x) && isfinite(k.y) &&
                                                                isfinite(k.z) && isfinite(k.w)));
-      const LaneCoef kk{f2_pack(k.x, k.x), f2_pack(k.y, k.y), f2_pack(k.z, k.z),
-                        f2_pack(k.w, k.w)};
+      const CoefPair kk = coef_pair(k);
       // ---- element updates, one 16-byte vector of orientations at a time
       const float* p1 = e1 + own;
       const float* p2 = e2 + own;
@@ -464,10 +408,16 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
             auto pair = [&](const float4& u) {
               return h == 0 ? f2_pack(u.x, u.y) : f2_pack(u.z, u.w);
             };
-            const int o = 4 * v + 2 * h;  // orientation
-            const F2 t = lane_pair<ANISO>(L, pair(cc[v]), pair(xm), pair(xp), pair(ym), pair(yp),
-                                          pair(zm[v]), pair(zp), a.dirs + o * 3,
-                                          a.dirs + (N + o) * 3, kk);
+            // the axes of orientations 4v + 2h, 4v + 2h + 1: the projections stay
+            // single, with their constant operands from the parameters
+            const float* d = a.dirs + (4 * v + 2 * h) * 3;
+            const F2 t = elem_pair<ANISO>(
+                L, pair(cc[v]), pair(xm), pair(xp), pair(ym), pair(yp), pair(zm[v]), pair(zp), kk,
+                [&](int j, F2 gx, F2 gy, F2 gz) {
+                  const float* q = d + j * N * 3;
+                  return f2_pack(fmaf(q[0], f2_lo(gx), fmaf(q[1], f2_lo(gy), q[2] * f2_lo(gz))),
+                                 fmaf(q[3], f2_hi(gx), fmaf(q[4], f2_hi(gy), q[5] * f2_hi(gz))));
+                });
             r[2 * h] = f2_lo(t);
             r[2 * h + 1] = f2_hi(t);
           }

@@ -217,6 +217,61 @@ __device__ __forceinline__ CellCoef cell_coefficients(const TempCoef& t, float S
   return r;
 }
 
+// Folded update (allen_cahn.py:42-51,58,60-85 with the Euler step, :106-114)
+// of two orientations of a cell, as packed pairs of floats (each half rounds
+// as the single operation does).  Per cell, k = (A1, B1, C1, W):
+//   eta' = e (A1 + B1 e^2) + (C1 + W (cn + cn^2)) lap'
+// with A1 = 1 + cg K, B1 = -3 cg, C1 = cl wx (1 + A), W = 2 A cl wx,
+// lap' = (xp + xm) + ry (yp + ym) + rz (zp + zm) - 2 (1 + ry + rz) e, and
+// cn = -cos^2 of the smallest angle between the central difference and the
+// orientation's cube axes: cos^4 + sin^4 = 1 - 2 c2 (1 - c2) with
+// c2 = max_k (d_k . g)^2 / |g|^2 (allen_cahn.py:28-39); the third axis is
+// orthogonal to the first two, so (d_2 . g)^2 = |g|^2 - q0 - q1.  |g|^2
+// starts from 1e-30, so a zero gradient gives cn = 0: the reference's
+// NaN-to-zero rule (c2 = 1 gives the same factor), with no clamp.  For any
+// gradient that matters, |g|^2 >= ~1e-14 and the 1e-30 is far below an ulp;
+// rounding can leave c2 a few ulps above 1, which changes the anisotropy term
+// by a relative ~1e-7 instead of clamping it to 0.
+// dot(j, gx, gy, gz) is the pair's projection on axis j.  The step kernels are
+// bound by issue slots and chains of dependent instructions, and a packed
+// instruction takes one slot: cell-per-lane kernel 408 -> 391 us a fused step
+// at 8M cells, n = 20 (its projections stay single: their constants are
+// parameter operands); TMA-fed kernel 338 -> 311 us at 4M, n = 30, and
+// 55 -> 53.5 us without anisotropy at 1M, n = 10.
+struct LapPair {
+  F2 ry, rz, nm;  // w_y / w_x, w_z / w_x, -2 (1 + ry + rz)
+};
+__device__ __forceinline__ LapPair lap_pair(const PFConsts& c) {
+  const float ry = c.wy / c.wx, rz = c.wz / c.wx, nm = -2.f * (1.f + ry + rz);
+  return LapPair{f2_pack(ry, ry), f2_pack(rz, rz), f2_pack(nm, nm)};
+}
+struct CoefPair {
+  F2 x, y, z, w;
+};
+__device__ __forceinline__ CoefPair coef_pair(const float4& k) {
+  return CoefPair{f2_pack(k.x, k.x), f2_pack(k.y, k.y), f2_pack(k.z, k.z), f2_pack(k.w, k.w)};
+}
+template <bool ANISO, class Dot>
+__device__ __forceinline__ F2 elem_pair(const LapPair& L, F2 e, F2 xm, F2 xp, F2 ym, F2 yp, F2 zm,
+                                        F2 zp, const CoefPair& k, Dot&& dot) {
+  const F2 lap = f2_fma(L.rz, f2_add(zp, zm),
+                        f2_fma(L.ry, f2_add(yp, ym), f2_fma(L.nm, e, f2_add(xp, xm))));
+  F2 u = k.z;
+  if constexpr (ANISO) {
+    const F2 gx = f2_sub(xp, xm), gy = f2_sub(yp, ym), gz = f2_sub(zp, zm);
+    const F2 ee = f2_fma(gx, gx, f2_fma(gy, gy, f2_fma(gz, gz, f2_pack(1e-30f, 1e-30f))));
+    const F2 p0 = dot(0, gx, gy, gz), p1 = dot(1, gx, gy, gz);
+    const F2 q0 = f2_mul(p0, p0), q1 = f2_mul(p1, p1);
+    const F2 q2 = f2_sub(f2_sub(ee, q0), q1);
+    float ml, mh;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(ml) : "f"(f2_lo(q0)), "f"(f2_lo(q1)), "f"(f2_lo(q2)));
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(mh) : "f"(f2_hi(q0)), "f"(f2_hi(q1)), "f"(f2_hi(q2)));
+    const F2 cn = f2_pack(ml * rcp_approx(-f2_lo(ee)), mh * rcp_approx(-f2_hi(ee)));
+    u = f2_fma(k.w, f2_fma(cn, cn, cn), k.z);
+  }
+  return f2_fma(u, lap, f2_mul(e, f2_fma(k.y, f2_mul(e, e), k.x)));
+}
+
 // Cubic anisotropy factor 1 + A (cos^4 t + sin^4 t) where t is the smallest
 // folded angle between the central-difference vector e and the orientation's
 // three rotated cube axes (allen_cahn.py:28-39).  cos t = max_k |d_k.e|/|e|,

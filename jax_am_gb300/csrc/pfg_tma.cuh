@@ -25,39 +25,7 @@ __device__ __forceinline__ bool tma_wait(uint64_t* bar, unsigned parity, int* er
   return false;
 }
 
-// Folded update of one element (see pfg_warp.cuh for the derivation).  The
-// per-cell coefficients are k = (A1, B1, C1, W) with W = -C2 = 2 A cl w_x, and
-// the anisotropy enters through cn = -cos^2 = m * rcp(-ee):
-// C1 + C2 c2 (1 - c2) = C1 + W (cn + cn^2).  ee starts from 1e-30 instead of
-// 0, so |e| = 0 gives m = 0, cn = 0 and cn + cn^2 = 0: the value of the
-// reference's NaN-to-zero rule (cos^2 = 1), with no clamp.  For any gradient
-// that matters, ee >= ~1e-14 and the 1e-30 is far below an ulp; rounding can
-// leave m / ee a few ulps above 1, which changes the anisotropy term by a
-// relative ~1e-7 instead of clamping it to 0.
-struct LapConstsT {
-  float ry, rz, nm;
-};
-template <bool ANISO>
-__device__ __forceinline__ float tma_update_elem(const LapConstsT& L, float e, float xm, float xp,
-                                                 float ym, float yp, float zm, float zp,
-                                                 const float* d, const float4 k) {
-  const float lap = fmaf(L.rz, zp + zm, fmaf(L.ry, yp + ym, fmaf(L.nm, e, xp + xm)));
-  float u = k.z;
-  if constexpr (ANISO) {
-    const float ex = xp - xm, ey = yp - ym, ez = zp - zm;
-    const float ee = fmaf(ex, ex, fmaf(ey, ey, fmaf(ez, ez, 1e-30f)));
-    const float p0 = fmaf(d[0], ex, fmaf(d[1], ey, d[2] * ez));
-    const float p1 = fmaf(d[3], ex, fmaf(d[4], ey, d[5] * ez));
-    const float q0 = p0 * p0, q1 = p1 * p1;
-    const float q2 = ee - q0 - q1;
-    float m;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(q0), "f"(q1), "f"(q2));
-    const float cn = m * rcp_approx(-ee);
-    u = fmaf(k.w, fmaf(cn, cn, cn), k.z);
-  }
-  return fmaf(u, lap, e * fmaf(k.y, e * e, k.x));
-}
-
+// Per-cell folded coefficients (see elem_pair).
 __device__ __forceinline__ float4 tma_fold(const PFConsts& c, const TempCoef& tc, float S) {
   if (tc.liquid != 0.f) return make_float4(0.f, 0.f, 0.f, 0.f);
   const float K = 4.f * S + tc.om2 - 1.f;
@@ -276,18 +244,18 @@ __device__ __forceinline__ void tma_unit(const StepArgs& a, int unit, const floa
   const int off_xm = (gx == 0 && a.bcx == PFG_BC_NEUMANN) ? 0 : -n;
   const int off_xp = (gx == a.nx - 1 && a.bcx == PFG_BC_NEUMANN) ? 0 : n;
 
-  float dl[ANISO ? 6 * VEC : 1];
+  F2 dl[ANISO ? 3 * VEC : 1];  // the axes of each pair of the lane's orientations
   if constexpr (ANISO) {
     const int ib = min(i0, n - VEC);
 #pragma unroll
-    for (int v = 0; v < VEC; ++v)
+    for (int v = 0; v < VEC; v += 2)
 #pragma unroll
-      for (int j = 0; j < 6; ++j) dl[v * 6 + j] = a.dirs[((j / 3) * n + ib + v) * 3 + (j % 3)];
+      for (int j = 0; j < 6; ++j) {
+        const float* d = a.dirs + ((j / 3) * n + ib + v) * 3 + (j % 3);
+        dl[v * 3 + j] = f2_pack(d[0], d[3]);
+      }
   }
-  LapConstsT L;
-  L.ry = a.pc.wy / a.pc.wx;
-  L.rz = a.pc.wz / a.pc.wx;
-  L.nm = -2.f * (1.f + L.ry + L.rz);
+  const LapPair L = lap_pair(a.pc);
 
   float xl = 0.f, yl = 0.f, Pw = 0.f;
   if constexpr (TSRC == kTHeat) {
@@ -313,6 +281,18 @@ __device__ __forceinline__ void tma_unit(const StepArgs& a, int unit, const floa
     c_g[q] = (c_hy[q] + 1) * gsy + c_hx[q] + 1;
   }
 
+  // low parts of a compensated temperature at this thread's cells, of the next
+  // plane that needs coefficients: loaded a plane ahead (311 -> 296 us a
+  // compensated step at 4M cells, n = 30)
+  float lo[2] = {0.f, 0.f};
+  auto load_lo = [&](int pz) {
+    if constexpr (TSRC == kTHeat) {
+      if (!a.T_lo) return;
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (c_ok[q]) lo[q] = __ldg(a.T_lo + (int64_t)(pz + 1) * gsz + c_g[q]);
+    }
+  };
   // per-cell coefficients of plane pz (in slot s) -> cc[buf]
   auto cell_coefs = [&](int s, int buf, int pz) {
     const float* es = eta_s + (size_t)s * slot_floats;
@@ -370,15 +350,16 @@ __device__ __forceinline__ void tma_unit(const StepArgs& a, int unit, const floa
       else if constexpr (TSRC == kTHeat) {
         // compensated state (a.T_lo set): zeta from the exact pair
         tc = a.T_lo ? temp_coefficients_pair(
-                          a.pc, ts[c_toff[q]],
-                          __ldg(a.T_lo + (int64_t)(pz + 1) * gsz + c_g[q]), a.dt)
+                          a.pc, ts[c_toff[q]], lo[q], a.dt)
                     : temp_coefficients_fast(a.pc, ts[c_toff[q]], a.dt);
       }
       else tc = temp_coefficients_fast(a.pc, ts[c_toff[q]], a.dt);
       cb[c_cc[q]] = tma_fold(a.pc, tc, s0 + s1);
     }
+    if (pz + 1 < ze) load_lo(pz + 1);
   };
 
+  load_lo(zb);
   // ---- prologue: planes 0 .. S-2 in flight (slot j), wait for planes 0, 1, 2
   int issued = 0;
   for (int j = 0; j < S - 1 && j < nplanes; ++j) { stage(j, j); issued = j + 1; }
@@ -446,12 +427,20 @@ __device__ __forceinline__ void tma_unit(const StepArgs& a, int unit, const floa
     auto row_out = [&](int r, float* dst, const VecF<VEC>& c, const VecF<VEC>& xm,
                        const VecF<VEC>& xp, const VecF<VEC>& ym, const VecF<VEC>& yp,
                        const VecF<VEC>& zm, const VecF<VEC>& zp) {
-      const float4 kc = ccb[r * P_tx + xs];
+      const CoefPair kc = coef_pair(ccb[r * P_tx + xs]);
       VecF<VEC> out;
 #pragma unroll
-      for (int v = 0; v < VEC; ++v)
-        out.v[v] = tma_update_elem<ANISO>(L, c.v[v], xm.v[v], xp.v[v], ym.v[v], yp.v[v], zm.v[v],
-                                          zp.v[v], &dl[ANISO ? v * 6 : 0], kc);
+      for (int v = 0; v < VEC; v += 2) {
+        auto pair = [&](const VecF<VEC>& u) { return f2_pack(u.v[v], u.v[v + 1]); };
+        const F2 t = elem_pair<ANISO>(
+            L, pair(c), pair(xm), pair(xp), pair(ym), pair(yp), pair(zm), pair(zp), kc,
+            [&](int j, F2 gx, F2 gy, F2 gz) {
+              const F2* d = &dl[ANISO ? v * 3 + 3 * j : 0];
+              return f2_fma(d[0], gx, f2_fma(d[1], gy, f2_mul(d[2], gz)));
+            });
+        out.v[v] = f2_lo(t);
+        out.v[v + 1] = f2_hi(t);
+      }
       if (col_valid) out.store(dst);
     };
     int r = r_begin;
