@@ -182,7 +182,7 @@ __device__ __forceinline__ void tma_unit(const StepArgs& a, int unit, const floa
   {
     const int tcols = (TSRC == kTHeat) ? txv + 2 : txv;
     const int tcount = (TSRC == kTHeat) ? rows * tcols : tyv * txv;
-    const uint64_t mg = div_magic(tcols);
+    const uint32_t mg = div_magic(tcols);
 #pragma unroll
     for (int q = 0; q < kTQ; ++q) {
       const int i = threadIdx.x + q * NC;
