@@ -78,7 +78,16 @@ __device__ __forceinline__ void stage_plane_w(const StepArgs& a, float* eta_s, f
   float* es = eta_s + (size_t)slot * (a.ty + 2) * a.pitch;
   float* ts = T_s + (size_t)slot * a.tslot;
   const int tp = a.tx + 2;
-  for (int r = warp; r < tyv + 2; r += kThreads / 32) {
+  // with the heat update the per-cell pass is long: the warps that own no cells
+  // in it stage, at least four of them (60.2 -> 57.1 us a step at 141 x 70 x 40,
+  // n = 30; without heat all eight: four take 3 to 12 % longer)
+  int w0 = 0;
+  if constexpr (TSRC == kTHeat) {
+    const int cell_warps = (txv * tyv + 31) >> 5;
+    if (cell_warps < kThreads / 32) w0 = min(cell_warps, kThreads / 64);
+  }
+  for (int r = warp - w0; r < tyv + 2; r += kThreads / 32 - w0) {
+    if (r < 0) break;
     const int gy = bc_index(y0 - 1 + r, ny, a.bcy);
     const float* row = a.eta_in + ((int64_t)gz * ny + gy) * nx * n;
     float* dst = es + r * a.pitch;
