@@ -1,5 +1,7 @@
-// Cell-per-lane TMA stencil step: the fast path for num_oris = 20 (every
-// configuration of the reference), with 16-byte orientation vectors.
+// Cell-per-lane TMA stencil step: the fast path for even num_oris from 10 to
+// 24, with 16-byte orientation vectors where num_oris % 4 == 0 and 8-byte ones
+// otherwise (then nx is even and x Neumann, as in the TMA-fed kernel).  26 and
+// up do not leave shared memory for two CTAs an SM.
 //
 // Each thread owns one cell of a TX x TY tile (TX * TY = the CTA's threads:
 // one cell per thread) and marches it through a chunk of z planes.  All per-cell work is
@@ -23,6 +25,13 @@
 // Every wait is bounded; a wait that runs out sets the device error flag,
 // the CTA waits for its copies in flight (each with the full bound) and
 // returns.
+//
+// Bound: issue slots and chains of dependent instructions at 16 warps an SM.
+// Against the TMA-fed kernel, whose lanes share a cell (its per-cell work goes
+// through shared memory, and no vector of zeros is skipped), a moving-gradient
+// step at 128 x 128 x 64 cells, isotropic: n = 10 49 -> 33 us, 12 62 -> 30,
+// 16 49 -> 39, 20 64 -> 43, 24 79 -> 49; anisotropic 51 -> 37, 69 -> 36,
+// 51 -> 43, 65 -> 46, 86 -> 52.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -50,6 +59,11 @@ __device__ __forceinline__ float quench_T(const StepArgs& a, int z, double t) {
   return (float)(a.q.T_base + a.q.grad * (zc - a.q.z0) - a.q.grad * a.q.vel * t);
 }
 
+// s + lo^2 + hi^2 of a pair.
+__device__ __forceinline__ float add_squares(F2 u, float s) {
+  return fmaf(f2_lo(u), f2_lo(u), fmaf(f2_hi(u), f2_hi(u), s));
+}
+
 // Per-cell folded coefficients from the temperature part and S.
 __device__ __forceinline__ float4 lane_fold(const PFConsts& c, const TempCoef& tc, float S) {
   if (tc.liquid != 0.f) return make_float4(0.f, 0.f, 0.f, 0.f);
@@ -58,43 +72,74 @@ __device__ __forceinline__ float4 lane_fold(const PFConsts& c, const TempCoef& t
   return make_float4(1.f + tc.cg * K, -3.f * tc.cg, clw * (1.f + c.aniso), 2.f * c.aniso * clw);
 }
 
-__device__ __forceinline__ float4 lds4(const float* p) {
-  return *reinterpret_cast<const float4*>(p);
+// A vector of VP pairs (16 or 8 bytes).
+template <int VP>
+__device__ __forceinline__ void load_pairs(F2* v, const float* p) {
+  if constexpr (VP == 2) {
+    const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(p);
+    v[0].b = u.x;
+    v[1].b = u.y;
+  } else {
+    v[0].b = *reinterpret_cast<const unsigned long long*>(p);
+  }
+}
+template <int VP>
+__device__ __forceinline__ void store_pairs(float* p, const F2* v) {
+  if constexpr (VP == 2)
+    *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v[0].b, v[1].b);
+  else
+    *reinterpret_cast<unsigned long long*>(p) = v[0].b;
 }
 
-template <int NV>
-__device__ __forceinline__ void load_cell(float4 (&v)[NV], const float* p) {
-#pragma unroll
-  for (int i = 0; i < NV; ++i) v[i] = lds4(p + 4 * i);
-}
-
-// NV: 16-byte vectors per cell (num_oris = 4 NV); NC threads, MINB CTAs per
-// SM; TX: tile width (16 or 32; the tile is TX x NC/TX cells); S: ring slots
-// (3 or 4); COMP: the fused heat state is compensated (T = T + T_lo,
-// double-float update).
+// The launch shape of an orientation count.
+template <int N>
+struct LanePlan {
+  static constexpr int VP = N % 4 == 0 ? 2 : 1;  // pairs per vector
+  static constexpr int TX = 16, NC = 256;        // 16 x 16 tiles, one cell per thread
+  // cells of a staged row: with 8-byte vectors a row is copied from and to an
+  // even cell (whole 16 bytes)
+  static constexpr int ROWC = VP == 2 ? TX + 2 : TX + 4;
+  // The lanes of one shared-memory phase (8 lanes of a 16-byte load, 16 of an
+  // 8-byte one) fall on distinct banks: cells along x do by their stride unless
+  // N % 8 == 0, where a phase then takes XB cells of each of 8 / XB rows; and
+  // the row pitch places the phase's rows beside one another.  (Without, at
+  // 1M cells, n = 16: 67 us a step against the TMA-fed kernel's 49.)
+  static constexpr int XB = N % 16 == 0 ? 2 : N % 8 == 0 ? 4 : 8;
+  static constexpr int row = ROWC * N;
+  static constexpr int want = VP == 1 ? 16 : 4;  // the pitch's bank, where it matters
+  static constexpr int pitch =
+      (VP == 1 || XB < 8) ? row + ((want - row) % 32 + 32) % 32 : row;  // floats
+  static constexpr size_t slot = (size_t)(NC / TX + 2) * pitch * 4;
+  static constexpr int tslot = ((TX + 2) * (NC / TX + 2) + 3) / 4 * 4;
+  // ring slots: four where two CTAs then fit an SM
+  static constexpr int S = 4 * (slot + 2 * tslot * 4) <= 114304 ? 4 : 3;
+};
+// COMP: the fused heat state is compensated (T = T + T_lo, double-float
+// update).
 //
 // Ring: plane j (grid plane zb - 1 + j) sits in slot j % S and its copies
 // complete phase (j / S) & 1 of that slot's barrier.  Iteration m (z =
 // zb + m) reads plane m + 1 (the x/y neighbours) and plane m + 2 (the cell
 // above); plane m was last read in iteration m - 1, so right after the
 // barrier that opens iteration m its slot takes plane m + S.
-template <int NV, bool ANISO, int TSRC, int NC, int MINB, int TX, int S, bool COMP>
-__global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant__ StepArgs a) {
-  static_assert(NC % TX == 0 && NC % 32 == 0, "whole rows, whole warps");
-  constexpr int TY = NC / TX;
-  constexpr int N = 4 * NV;
+template <int N, bool ANISO, int TSRC, bool COMP>
+__global__ void __launch_bounds__(LanePlan<N>::NC, 2)
+pf_lane_kernel(const __grid_constant__ StepArgs a) {
+  using LP = LanePlan<N>;
+  constexpr int NC = LP::NC, TX = LP::TX, TY = NC / TX, S = LP::S;
+  constexpr int VP = LP::VP, V = 2 * VP, NP = N / 2, NV = N / V;
+  constexpr bool HALF = VP == 1;  // 8-byte vectors: rows start and end at even cells
   constexpr int TPX = TX + 2, TPY = TY + 2;  // staged tile with its halo
-  constexpr int ROWF = TPX * N;               // floats per staged row
+  constexpr int ROWF = LP::pitch;             // floats per staged row
   constexpr int SLOTF = TPY * ROWF;           // floats per eta slot
-  constexpr int TSLOT = (TPX * TPY + 3) / 4 * 4;
+  constexpr int TSLOT = LP::tslot;
   constexpr bool HEAT = TSRC == kTHeat;
-  static_assert(S == 3 || S == 4, "3 or 4 plane slots");
+  static_assert(N % 2 == 0 && (S == 3 || S == 4), "pairs; 3 or 4 plane slots");
   static_assert(!COMP || HEAT, "the compensated state is the fused heat state");
   extern __shared__ __align__(128) float smem[];
   float* eta_s = smem;
   float* T_s = eta_s + S * SLOTF;
   float* TL_s = T_s + S * TSLOT;  // low parts of the compensated temperature
-  uint64_t* full = reinterpret_cast<uint64_t*>(TL_s + (COMP ? S * TSLOT : 0));
 
   // ---- work unit: (tile, z chunk), z chunk slowest
   const int per_plane = a.tiles_x * a.tiles_y;
@@ -110,6 +155,7 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
   const int nplanes = ze - zb + 2;  // planes zb-1 .. ze
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  __shared__ uint64_t full[S];  // the ring's barriers
   __shared__ int s_abort;
   __shared__ double s_t0;
   __shared__ long long s_step;
@@ -151,8 +197,11 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
 
   // ---- staging of plane j into slot j % S: eta rows by warp 0 (TMA), the
   // ghosted temperature tile by every thread (cp.async)
-  const int cx0 = max(x0 - 1, 0), cx1 = min(xe + 1, a.nx);
-  const int dst_cell0 = cx0 - (x0 - 1);
+  // (8-byte vectors: x0, xe and nx are even and x is Neumann (the planner))
+  const int cx0 = HALF ? max(x0 - 2, 0) : max(x0 - 1, 0);
+  const int cx1 = HALF ? (xe < a.nx ? xe + 2 : a.nx) : min(xe + 1, a.nx);
+  const int dst_cell0 = HALF ? 0 : cx0 - (x0 - 1);
+  const int pos0 = HALF ? x0 - cx0 : 1;  // staged position of cell x0
   const bool wrap_left = (x0 == 0) && a.bcx == PFG_BC_PERIODIC;
   const bool wrap_right = (xe == a.nx) && a.bcx == PFG_BC_PERIODIC;
   const int rows = tyv + 2;
@@ -211,12 +260,15 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
   // their neighbours span fewer grains than a 16 x 2 strip, so more of its
   // orientation vectors are exact zeros (1.4 % faster than 16 x 2); a row of
   // 8 lanes at an 80-byte stride reads shared memory without bank conflicts
-  const int tr = ((threadIdx.x >> 5) / (TX / 8)) * 4 + ((threadIdx.x & 31) >> 3);
-  const int tc = ((threadIdx.x >> 5) % (TX / 8)) * 8 + (threadIdx.x & 7);
+  constexpr int XB = LP::XB;
+  const int lx = lane % XB + XB * ((lane >> 3) % (8 / XB));
+  const int ly = (lane % 8) / XB + (8 / XB) * (lane / (64 / XB));
+  const int tr = (warp / (TX / 8)) * 4 + ly;
+  const int tc = (warp % (TX / 8)) * 8 + lx;
   const bool valid = tr < tyv && tc < txv;
   const bool warp_on = ((threadIdx.x >> 5) / (TX / 8)) * 4 < tyv;  // some row of this warp is in the tile
   const int gx = x0 + tc, gy = y0 + tr;
-  const int own = (tr + 1) * ROWF + (tc + 1) * N;  // staged offset of the cell
+  const int own = (tr + 1) * ROWF + (tc + pos0) * N;  // staged offset of the cell
   // Neumann along x: the edge cell is its own neighbour (its halo is not staged)
   const int oxm = (gx == 0 && a.bcx == PFG_BC_NEUMANN) ? 0 : -N;
   const int oxp = (gx == a.nx - 1 && a.bcx == PFG_BC_NEUMANN) ? 0 : N;
@@ -255,11 +307,12 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
   // (that plane's slot is refilled while plane z is computed); plane z's come
   // from its slot.  (Unrolling the z loop to rotate register sets instead of
   // copying them makes the loop body overflow the instruction cache.)
-  float4 zm[NV], cc[NV];
+  F2 zm[NP], cc[NP];
   float Tzm = 0.f, Tc = 0.f;
   float Lzm = 0.f, Lc = 0.f;  // their low parts (COMP)
   if (ok) {
-    load_cell<NV>(zm, eta_s + 0 * SLOTF + own);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) load_pairs<VP>(zm + v * VP, eta_s + 0 * SLOTF + own + v * V);
     if constexpr (HEAT) Tzm = T_s[0 * TSLOT + town];
     if constexpr (COMP) Lzm = TL_s[0 * TSLOT + town];
   }
@@ -287,7 +340,8 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
       if (threadIdx.x == 0 && z + 1 < ze) s_Tq[(m + 1) & 1] = quench_T(a, z + 1, t0);
     const float* e1 = eta_s + s1 * SLOTF;
     const float* e2 = eta_s + s2 * SLOTF;
-    load_cell<NV>(cc, e1 + own);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) load_pairs<VP>(cc + v * VP, e1 + own + v * V);
     float Tzp = 0.f, Lzp = 0.f;
     if constexpr (HEAT) {
       Tc = T_s[s1 * TSLOT + town];
@@ -363,11 +417,18 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
       }
       // ---- per-cell coefficients
       float s_a = 0.f, s_b = 0.f;
+      if constexpr (N % 4 == 0 && N != 20) {  // the TMA-fed kernel's order
 #pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        const float4 u = cc[v];
-        s_a = fmaf(u.x, u.x, fmaf(u.y, u.y, s_a));
-        s_b = fmaf(u.z, u.z, fmaf(u.w, u.w, s_b));
+        for (int v = 0; v < NV; ++v) {
+          float& s = (v & 1) ? s_b : s_a;
+          s = add_squares(cc[2 * v], add_squares(cc[2 * v + 1], s));
+        }
+      } else {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          float& s = (p & 1) ? s_b : s_a;
+          s = add_squares(cc[p], s);
+        }
       }
       TempCoef tcf;
       if constexpr (COMP) tcf = temp_coefficients_pair(a.pc, Tcell, Lc, a.dt);
@@ -377,14 +438,17 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
       const bool kfinite = __all_sync(0xffffffffu, !valid || (isfinite(k.x) && isfinite(k.y) &&
                                                                isfinite(k.z) && isfinite(k.w)));
       const CoefPair kk = coef_pair(k);
-      // ---- element updates, one 16-byte vector of orientations at a time
+      // ---- element updates, one vector of orientations at a time
       const float* p1 = e1 + own;
       const float* p2 = e2 + own;
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        const float4 xm = lds4(p1 + oxm + 4 * v), xp = lds4(p1 + oxp + 4 * v);
-        const float4 ym = lds4(p1 - ROWF + 4 * v), yp = lds4(p1 + ROWF + 4 * v);
-        const float4 zp = lds4(p2 + 4 * v);
+        F2 xm[VP], xp[VP], ym[VP], yp[VP], zp[VP], r[VP];
+        load_pairs<VP>(xm, p1 + oxm + V * v);
+        load_pairs<VP>(xp, p1 + oxp + V * v);
+        load_pairs<VP>(ym, p1 - ROWF + V * v);
+        load_pairs<VP>(yp, p1 + ROWF + V * v);
+        load_pairs<VP>(zp, p2 + V * v);
         // Exact zeros: an orientation that is zero (+0.0) at every cell of
         // the warp and at all their six neighbours stays exactly zero
         // (gradient, Laplacian and local term vanish, and the update of +0.0
@@ -393,42 +457,34 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
         // such zeros.  The test is per pair of orientations (0.8 % faster
         // than per vector of four): the cells' own values (in registers)
         // first, the neighbours only when those are zero across the warp.
-        float r[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {  // orientations 4v + 2h, 4v + 2h + 1
-          auto pr = [&](const float4& u) {
-            return h == 0 ? (__float_as_uint(u.x) | __float_as_uint(u.y))
-                          : (__float_as_uint(u.z) | __float_as_uint(u.w));
-          };
-          bool work = !kfinite || __any_sync(0xffffffffu, (pr(cc[v]) | pr(zm[v])) != 0u);
+        for (int h = 0; h < VP; ++h) {
+          const int p = v * VP + h;  // orientations 2p, 2p + 1
+          bool work = !kfinite || __any_sync(0xffffffffu, (cc[p].b | zm[p].b) != 0ull);
           if (!work)
             work = __any_sync(0xffffffffu,
-                              (pr(xm) | pr(xp) | pr(ym) | pr(yp) | pr(zp)) != 0u);
+                              (xm[h].b | xp[h].b | ym[h].b | yp[h].b | zp[h].b) != 0ull);
+          r[h] = F2{};
           if (work) {
-            auto pair = [&](const float4& u) {
-              return h == 0 ? f2_pack(u.x, u.y) : f2_pack(u.z, u.w);
-            };
-            // the axes of orientations 4v + 2h, 4v + 2h + 1: the projections stay
-            // single, with their constant operands from the parameters
-            const float* d = a.dirs + (4 * v + 2 * h) * 3;
-            const F2 t = elem_pair<ANISO>(
-                L, pair(cc[v]), pair(xm), pair(xp), pair(ym), pair(yp), pair(zm[v]), pair(zp), kk,
+            // the axes of the pair: the projections stay single, with their
+            // constant operands from the parameters
+            const float* d = a.dirs + 2 * p * 3;
+            r[h] = elem_pair<ANISO>(
+                L, cc[p], xm[h], xp[h], ym[h], yp[h], zm[p], zp[h], kk,
                 [&](int j, F2 gx, F2 gy, F2 gz) {
                   const float* q = d + j * N * 3;
                   return f2_pack(fmaf(q[0], f2_lo(gx), fmaf(q[1], f2_lo(gy), q[2] * f2_lo(gz))),
                                  fmaf(q[3], f2_hi(gx), fmaf(q[4], f2_hi(gy), q[5] * f2_hi(gz))));
                 });
-            r[2 * h] = f2_lo(t);
-            r[2 * h + 1] = f2_hi(t);
           }
         }
-        if (valid) *reinterpret_cast<float4*>(out + 4 * v) = make_float4(r[0], r[1], r[2], r[3]);
+        if (valid) store_pairs<VP>(out + V * v, r);
       }
     }
     out += plane_cells * N;
     // plane z is the next plane's z - 1
 #pragma unroll
-    for (int v = 0; v < NV; ++v) zm[v] = cc[v];
+    for (int p = 0; p < NP; ++p) zm[p] = cc[p];
     Tzm = Tc;
     Lzm = Lc;
   }
@@ -446,47 +502,63 @@ __global__ void __launch_bounds__(NC, MINB) pf_lane_kernel(const __grid_constant
 // host side
 // ---------------------------------------------------------------------------
 
-constexpr int kLaneNV = 5;   // num_oris = 20
-constexpr int kLaneNC = 256;  // threads per CTA: one cell each
-constexpr int kLaneCTAs = 2;  // CTAs per SM
-constexpr int kLaneTX = 16;   // 16 x 16 tiles
-constexpr int kLaneS = 4;    // ring slots
-
-// Shared memory of one CTA: the eta ring, the temperature ring (high and
-// low parts), the barriers.
-static size_t lane_smem(int n, int tx, int slots) {
-  const int ty = kLaneNC / tx;
-  const size_t slot = (size_t)(ty + 2) * (tx + 2) * n * 4;
-  const size_t tslot = (size_t)(((tx + 2) * (ty + 2) + 3) / 4 * 4) * 4;
-  return (size_t)slots * (slot + 2 * tslot) + (size_t)slots * sizeof(uint64_t);
+// Calls f(std::integral_constant<int, n>) for the orientation counts that have a
+// kernel; false for the others.
+template <class F>
+static bool with_count(int n, F&& f) {
+  switch (n) {
+    case 10: f(std::integral_constant<int, 10>()); return true;
+    case 12: f(std::integral_constant<int, 12>()); return true;
+    case 14: f(std::integral_constant<int, 14>()); return true;
+    case 16: f(std::integral_constant<int, 16>()); return true;
+    case 18: f(std::integral_constant<int, 18>()); return true;
+    case 20: f(std::integral_constant<int, 20>()); return true;
+    case 22: f(std::integral_constant<int, 22>()); return true;
+    case 24: f(std::integral_constant<int, 24>()); return true;
+    default: return false;
+  }
 }
 
-bool plan_lane_tiles(int nx, int ny, int nz, int n, int sm_count, int max_smem_per_sm,
+// Cells from which the counts other than 20 take this kernel: at 6,000 cells
+// it and the TMA-fed kernel are level (isotropic 5.3 to 6.3 us a step against
+// 5.2 to 7.8, anisotropic 5.3 to 6.2 against 5.7 to 9.7, by count), at 32,768
+// it takes 5.6 to 6.5 us against 9.8 to 21, at 1M 30 to 86 against 49 to 91.
+constexpr int64_t kLaneMinCells = 1 << 13;
+
+// With a compensated heat state (comp) only 20 orientations do: the split step
+// (heat kernel, then the TMA-fed kernel) is level with it for the others
+// (20 steps of 200 x 100 x 50 cells: n = 12 1551 us here and 1466 split, n = 24
+// 2031 and 1908, n = 10 1529 and 1565).
+bool plan_lane_tiles(int nx, int ny, int nz, int n, int bcx, bool comp, int sm_count, int max_smem_per_sm,
                      int max_smem_per_block, int zchunks_override, TilePlan* out) {
-  if (n != 4 * kLaneNV) return false;
   // ghosted temperature offsets are 32-bit in this kernel
   if ((int64_t)(nx + 2) * (ny + 2) * (nz + 2) >= ((int64_t)1 << 31)) return false;
-  const int tx = kLaneTX, ty = kLaneNC / tx, S = kLaneS;
-  const size_t smem = lane_smem(n, tx, S);
-  // kLaneCTAs CTAs per SM: the dynamic shared memory plus the static variables and
-  // the per-CTA reservation
-  if (kLaneCTAs * (smem + 1024 + 128) > (size_t)max_smem_per_sm ||
-      smem > (size_t)max_smem_per_block)
-    return false;
+  if (n != 20 && comp) return false;
+  if (n != 20 && (int64_t)nx * ny * nz < kLaneMinCells) return false;
   TilePlan t{};
-  t.vec = 4;
+  if (!with_count(n, [&](auto c) {
+        using LP = LanePlan<decltype(c)::value>;
+        t.vec = 2 * LP::VP;
+        t.tx = LP::TX;
+        t.ty = LP::NC / LP::TX;
+        t.rs = LP::NC;
+        t.stages = LP::S;
+        t.pitch = LP::pitch;
+        t.tslot = LP::tslot;
+        t.smem = LP::S * (LP::slot + 2 * LP::tslot * sizeof(float));
+      }))
+    return false;
+  if (t.vec == 2 && (nx % 2 != 0 || bcx != PFG_BC_NEUMANN)) return false;
+  // two CTAs per SM: the dynamic shared memory plus the static variables and
+  // the per-CTA reservation
+  if (2 * (t.smem + 1024 + 256) > (size_t)max_smem_per_sm || t.smem > (size_t)max_smem_per_block)
+    return false;
   t.tpc = 1;
-  t.tx = tx;
-  t.ty = ty;
   t.cpw = 8;        // a warp owns 8 x 4 cells
-  t.wx = tx / 8;
+  t.wx = t.tx / 8;
   t.rpw = 4;
-  t.rs = kLaneNC;
-  t.stages = S;
-  t.pitch = (tx + 2) * n;
-  t.tslot = ((tx + 2) * (ty + 2) + 3) / 4 * 4;
-  t.tiles_x = (nx + tx - 1) / tx;
-  t.tiles_y = (ny + ty - 1) / ty;
+  t.tiles_x = (nx + t.tx - 1) / t.tx;
+  t.tiles_y = (ny + t.ty - 1) / t.ty;
   const long tiles = (long)t.tiles_x * t.tiles_y;
   int best_zc = plan_planes(tiles, nz, sm_count);
   if (zchunks_override > 0) best_zc = (nz + std::min(zchunks_override, nz) - 1) /
@@ -494,37 +566,47 @@ bool plan_lane_tiles(int nx, int ny, int nz, int n, int sm_count, int max_smem_p
   t.zc = best_zc;
   t.zchunks = (nz + t.zc - 1) / t.zc;
   t.units = tiles * t.zchunks;
-  t.smem = smem;
   if (t.units >= (1L << 31)) return false;
   *out = t;
   return true;
 }
 
-template <bool ANISO, int TSRC, bool COMP>
+template <int N, bool ANISO, int TSRC, bool COMP>
 static cudaError_t launch_lane_t(const StepArgs& a, const TilePlan& t, cudaStream_t s) {
-  auto k = pf_lane_kernel<kLaneNV, ANISO, TSRC, kLaneNC, kLaneCTAs, kLaneTX, kLaneS, COMP>;
+  using LP = LanePlan<N>;
+  auto k = pf_lane_kernel<N, ANISO, TSRC, COMP>;
+  // the temperature planes are staged with the fused heat state only
+  const int smem = (int)(TSRC == kTHeat ? t.smem : LP::S * LP::slot);
   static int configured[64] = {0};
   const int dev = device_info().device;
-  if (dev < 0 || dev >= 64 || configured[dev] < (int)t.smem) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)t.smem);
+  if (dev < 0 || dev >= 64 || configured[dev] < smem) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) configured[dev] = (int)t.smem;
+    if (dev >= 0 && dev < 64) configured[dev] = smem;
   }
-  k<<<(unsigned)t.units, kLaneNC, t.smem, s>>>(a);
+  k<<<(unsigned)t.units, LP::NC, smem, s>>>(a);
   return cudaGetLastError();
 }
 
 template <int TSRC>
 cudaError_t launch_lane_kernel(const StepArgs& a, const TilePlan& t, cudaStream_t s) {
-  if (a.n != 4 * kLaneNV || t.tx != kLaneTX || t.stages != kLaneS) return cudaErrorInvalidValue;
-  if constexpr (TSRC == kTHeat) {
-    if (a.T_lo)
-      return (a.pc.aniso > 0.f) ? launch_lane_t<true, TSRC, true>(a, t, s)
-                                : launch_lane_t<false, TSRC, true>(a, t, s);
-  }
-  return (a.pc.aniso > 0.f) ? launch_lane_t<true, TSRC, false>(a, t, s)
-                            : launch_lane_t<false, TSRC, false>(a, t, s);
+  cudaError_t e = cudaErrorInvalidValue;
+  with_count(a.n, [&](auto c) {
+    constexpr int N = decltype(c)::value;
+    if (t.tx != LanePlan<N>::TX || t.stages != LanePlan<N>::S) return;
+    const bool an = a.pc.aniso > 0.f;
+    if constexpr (TSRC == kTHeat) {
+      if (a.T_lo) {
+        if constexpr (N == 20)
+          e = an ? launch_lane_t<N, true, TSRC, true>(a, t, s)
+                 : launch_lane_t<N, false, TSRC, true>(a, t, s);
+        return;
+      }
+    }
+    e = an ? launch_lane_t<N, true, TSRC, false>(a, t, s)
+           : launch_lane_t<N, false, TSRC, false>(a, t, s);
+  });
+  return e;
 }
 
 template cudaError_t launch_lane_kernel<kTArray>(const StepArgs&, const TilePlan&, cudaStream_t);

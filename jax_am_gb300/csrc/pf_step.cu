@@ -497,13 +497,13 @@ TilePlan plan_for_current_device(const pfg_pf_params& p) {
   return plan_tiles(p.nx, p.ny, p.nz, p.num_oris, d.sm_count, d.smem_per_sm, d.smem_per_block);
 }
 
-static bool plan_lane(const pfg_pf_params& p, TilePlan* t) {
+static bool plan_lane(const pfg_pf_params& p, TilePlan* t, bool comp = false) {
   const DeviceInfo& d = device_info();
-  return plan_lane_tiles(p.nx, p.ny, p.nz, p.num_oris, d.sm_count, d.smem_per_sm,
+  return plan_lane_tiles(p.nx, p.ny, p.nz, p.num_oris, p.bc_x, comp, d.sm_count, d.smem_per_sm,
                          d.smem_per_block, g_tune_zchunks, t);
 }
 
-// Plan and launch one step: the cell-per-lane kernel (num_oris = 20), else
+// Plan and launch one step: the cell-per-lane kernel (plan_lane_tiles), else
 // the TMA-fed kernel, else the warp-per-cells kernel when the orientation
 // count allows it (num_oris / VEC <= 32), otherwise the generic kernel.
 template <int TSRC>
@@ -799,7 +799,7 @@ extern "C" int pfg_heat_pf_step_comp_supported(const pfg_pf_params* p) {
   const DeviceInfo& d = device_info();
   TilePlan t;
   const int v = g_kernel_variant;
-  if (v == 0 && plan_lane(*p, &t)) return 1;
+  if (v == 0 && plan_lane(*p, &t, true)) return 1;
   return ((v == 0 || v == 3) && plan_tma_tiles(p->nx, p->ny, p->nz, p->num_oris, p->bc_x,
                                                d.sm_count, d.smem_per_sm, &t))
              ? 1
@@ -837,7 +837,7 @@ extern "C" int pfg_heat_pf_step_comp(const pfg_pf_params* p, const pfg_heat_para
   a.hp = *h;
   const cudaStream_t cs = static_cast<cudaStream_t>(stream);
   TilePlan t;
-  if (v == 0 && plan_lane(*p, &t)) {  // the heat update inside the stencil
+  if (v == 0 && plan_lane(*p, &t, true)) {  // the heat update inside the stencil
     fill_common(a, *p, t, dt);
     a.cpw = t.cpw; a.wx = t.wx; a.rpw = t.rpw;
     return record_cuda(launch_lane_kernel<kTHeat>(a, t, cs));

@@ -78,9 +78,9 @@ template <int TSRC>
 cudaError_t launch_tma_kernel(const StepArgs& a, const TilePlan& t, cudaStream_t s);
 // Which compile-time plan of the TMA-fed kernel (1 or 2) a TMA plan uses, or 0.
 int fixed_plan_index(int n, const TilePlan& t);
-// Cell-per-lane TMA kernel (pf_lane.cu), num_oris = 20.
-bool plan_lane_tiles(int nx, int ny, int nz, int n, int sm_count, int max_smem_per_sm,
-                     int max_smem_per_block, int zchunks_override, TilePlan* out);
+// Cell-per-lane TMA kernel (pf_lane.cu), even num_oris from 10 to 24.
+bool plan_lane_tiles(int nx, int ny, int nz, int n, int bcx, bool comp, int sm_count,
+                     int max_smem_per_sm, int max_smem_per_block, int zchunks_override, TilePlan* out);
 template <int TSRC>
 cudaError_t launch_lane_kernel(const StepArgs& a, const TilePlan& t, cudaStream_t s);
 // Compensated heat step alone (heat_comp.cu): a.T, a.T_lo -> a.T_out,
