@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 pf_batch_kernel(BatchHeader* __restrict__ hdr, int k) {
   extern __shared__ __align__(128) float smem[];
   __shared__ __align__(16) StepArgs s_args;
+  __shared__ TempCoef s_Tc[kTmaMaxPlanes];  // of a TMA-fed unit's planes
   __shared__ int s_job;
   __shared__ long long s_unit;
   __shared__ int s_begin[kBatchCachedJobs];  // the jobs' first units (host keeps them < 2^31)
@@ -107,10 +108,10 @@ pf_batch_kernel(BatchHeader* __restrict__ hdr, int k) {
       float* eout = J.eta[(step + 1) & 1];
       if (J.aniso)
         tma_unit<true, kTQuench, kThreads, 4, 0, true>(s_args, unit, ein, eout, t0, tma_barriers,
-                                                       &g_batch_device_error);
+                                                       &g_batch_device_error, s_Tc);
       else
         tma_unit<false, kTQuench, kThreads, 4, 0, true>(s_args, unit, ein, eout, t0, tma_barriers,
-                                                        &g_batch_device_error);
+                                                        &g_batch_device_error, s_Tc);
       tma_barriers = true;
     } else if (step < J.target_steps) {  // uniform over the CTA
       // the job's arguments into shared memory, then this step's buffers
@@ -162,7 +163,8 @@ __global__ void pf_batch_advance_kernel(BatchHeader* __restrict__ hdr, int k_ste
 // Dynamic shared memory of every batch launch: two CTAs per SM, less the
 // kernel's static shared memory.
 static size_t batch_smem_budget(const DeviceInfo& d) {
-  return (size_t)d.smem_per_sm / 2 - 2048 - sizeof(StepArgs) - 64 - kBatchCachedJobs * sizeof(int);
+  return (size_t)d.smem_per_sm / 2 - 2048 - sizeof(StepArgs) - 64 -
+         kBatchCachedJobs * sizeof(int) - kTmaMaxPlanes * sizeof(TempCoef);
 }
 
 }  // namespace pfg

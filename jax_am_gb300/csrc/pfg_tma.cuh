@@ -68,7 +68,8 @@ template <> struct FixedPlan<2> {
 // err: the device error flag of the calling kernel.
 template <bool ANISO, int TSRC, int NC, int VEC, int FIX, bool BATCH>
 __device__ __forceinline__ void tma_unit(const StepArgs& a, int unit, const float* eta_in,
-                                         float* eta_out, double t_batch, bool reinit, int* err) {
+                                         float* eta_out, double t_batch, bool reinit, int* err,
+                                         TempCoef* s_Tc = nullptr) {
   static_assert(VEC == 4 || VEC == 2, "16- or 8-byte vectors");
   using FP = FixedPlan<FIX == 0 ? 1 : FIX>;
   static_assert(FIX == 0 || (FP::vec == VEC && NC == 256), "a fixed plan is a 256-thread plan");
@@ -136,14 +137,14 @@ __device__ __forceinline__ void tma_unit(const StepArgs& a, int unit, const floa
   }
   __syncthreads();
   const double t0 = s_t0;
-  // batched units (moving gradient): the temperature of each of the unit's
-  // planes, evaluated once (float64 arithmetic is slow on this GPU) rather
-  // than by every thread at every plane
-  __shared__ float s_Tq[kTmaMaxPlanes];
+  // batched units (moving gradient): a plane has one temperature, so the
+  // temperature coefficients of the unit's planes are worked out once (into
+  // s_Tc), a thread per plane, rather than by every thread at every plane
   if constexpr (BATCH && TSRC == kTQuench) {
     for (int j = threadIdx.x; j < nplanes; j += NC) {
       const double zc = a.q.z_first + (double)(zb - 1 + j) * (double)a.h_z;
-      s_Tq[j] = (float)(a.q.T_base + a.q.grad * (zc - a.q.z0) - a.q.grad * a.q.vel * t0);
+      const float Tz = (float)(a.q.T_base + a.q.grad * (zc - a.q.z0) - a.q.grad * a.q.vel * t0);
+      s_Tc[j] = temp_coefficients_fast(a.pc, Tz, a.dt);
     }
     __syncthreads();
   }
@@ -300,14 +301,13 @@ __device__ __forceinline__ void tma_unit(const StepArgs& a, int unit, const floa
     float4* cb = cc + (size_t)buf * P_ty * P_tx;
     TempCoef plane{};
     if constexpr (TSRC == kTQuench) {
-      float Tz;
       if constexpr (BATCH) {
-        Tz = s_Tq[pz - zb + 1];
+        plane = s_Tc[pz - zb + 1];
       } else {
         const double zc = a.q.z_first + (double)pz * (double)a.h_z;
-        Tz = (float)(a.q.T_base + a.q.grad * (zc - a.q.z0) - a.q.grad * a.q.vel * t0);
+        plane = temp_coefficients_fast(
+            a.pc, (float)(a.q.T_base + a.q.grad * (zc - a.q.z0) - a.q.grad * a.q.vel * t0), a.dt);
       }
-      plane = temp_coefficients_fast(a.pc, Tz, a.dt);
     }
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
