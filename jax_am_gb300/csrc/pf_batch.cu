@@ -190,6 +190,43 @@ extern "C" int64_t pfg_batch_table_bytes(int num_jobs) {
   return (int64_t)sizeof(BatchHeader) + (int64_t)num_jobs * (int64_t)sizeof(BatchJobDev);
 }
 
+// What a unit of zc planes costs: the bytes of its tile and planes with halo.
+static double unit_cost(const TilePlan& t, const pfg_batch_job& J, int zc) {
+  return (double)(t.tx + 2) * (t.ty + 2) * (zc + 2) * J.params.num_oris;
+}
+
+// Planes per unit, at most, of a table: whole z columns up to 64 planes read
+// the fewest halo planes, but with few units the launch waits for its last
+// ones.  Units are handed out largest first, so once those of at least some
+// cost are out, the slots are at their mean load and finish about half such a
+// unit apart; the launch takes no less than its largest unit.  (Six jobs of 32
+// to 160 cells a side: 127 us a launch with whole columns, 87 split; sixteen
+// 245 either way.)
+static int unit_planes(const pfg_batch_job* jobs, const std::vector<TilePlan>& plans, int slots) {
+  int best = 64;
+  double least = 0.0;
+  std::vector<std::pair<double, double>> costs(plans.size());  // a unit's, the job's
+  for (int c : {64, 48, 40, 32, 28, 24, 20, 16, 12, 8}) {
+    for (size_t j = 0; j < plans.size(); ++j) {
+      const TilePlan& t = plans[j];
+      const int zch = (jobs[j].params.nz + c - 1) / c;
+      const double cost = unit_cost(t, jobs[j], (jobs[j].params.nz + zch - 1) / zch);
+      costs[j] = {cost, cost * (double)t.tiles_x * t.tiles_y * zch};
+    }
+    std::sort(costs.begin(), costs.end());
+    double span = costs.empty() ? 0.0 : costs.back().first, out = 0.0;
+    for (auto it = costs.rbegin(); it != costs.rend(); ++it) {
+      out += it->second;
+      span = std::max(span, out / slots + 0.5 * it->first);
+    }
+    if (c == 64 || span < least) {
+      least = span;
+      best = c;
+    }
+  }
+  return best;
+}
+
 extern "C" int pfg_batch_encode(const pfg_batch_job* jobs, int num_jobs, void* table,
                                 int64_t table_bytes, int64_t* total_units) {
   if (num_jobs < 0) return PFG_ERR_PARAM;
@@ -228,15 +265,16 @@ extern "C" int pfg_batch_encode(const pfg_batch_job* jobs, int num_jobs, void* t
       return PFG_ERR_SHAPE;  // orientation count the warp-per-cells body cannot take
     }
     bodies[(size_t)j] = tma ? 1 : 0;
-    // units of whole z columns (or 64-plane chunks), so that few halo planes
-    // are read twice
-    const int zch = std::max(1, (J.params.nz + 63) / 64);
+  }
+  const int planes = unit_planes(jobs, plans, 2 * d.sm_count);
+  for (int j = 0; j < num_jobs; ++j) {
+    TilePlan& t = plans[(size_t)j];
+    const pfg_batch_job& J = jobs[j];
+    const int zch = (J.params.nz + planes - 1) / planes;
     t.zc = (J.params.nz + zch - 1) / zch;
     t.zchunks = (J.params.nz + t.zc - 1) / t.zc;
     t.units = (long)t.tiles_x * t.tiles_y * t.zchunks;
-    // bytes a unit moves: its tile with halo, its planes with halo, n floats
-    const double cost = (double)(t.tx + 2) * (t.ty + 2) * (t.zc + 2) * J.params.num_oris;
-    order[(size_t)j] = {-cost, j};
+    order[(size_t)j] = {-unit_cost(t, J, t.zc), j};
   }
   // largest units first (stable: equal costs keep the caller's order)
   std::stable_sort(order.begin(), order.end(),

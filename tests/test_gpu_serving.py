@@ -83,6 +83,27 @@ def test_batch_bodies_match_plain_solver(pad):
     assert _lib.device_error() == 0
 
 
+@pytest.mark.parametrize("n", [8, 13])
+def test_unit_splits_leave_a_job_unchanged(n):
+    """The planes per unit depend on the table (a lone job's columns are
+    split, also into chunks of unequal size; among many they are whole): the
+    same job alone and among large ones is bit-identical, with more planes
+    than a unit takes, in both unit bodies."""
+    from jax_am_gb300 import _lib
+    from jax_am_gb300.serving import BatchServer
+    out = []
+    for others in (0, 9):
+        jobs = [make_job((21, 18, 131), n, 11, 3)]
+        jobs += [make_job((96, 96, 62), 20, 8, 10 + k) for k in range(others)]
+        srv = BatchServer(max_jobs=16, graph_steps=4, pad_oris=n % 4 == 0)
+        for j in jobs:
+            srv.submit(j)
+        srv.run(realtime=False)
+        out.append(jobs[0].result)
+    assert torch.equal(out[0], out[1])
+    assert _lib.device_error() == 0
+
+
 def test_graph_replay_equals_eager():
     from jax_am_gb300.serving import BatchServer
     res = []
