@@ -35,7 +35,7 @@ PF_KEYS = dict(T_liquidus=1623.0, gas_const=8.3, Qg=1.4e5, L0=3.5e3, kappa_g=2.7
                ad_hoc=1.0)
 METRIC = "cell_orientation_updates_per_s"
 UNIT = "cell*ori/s"
-KERNEL = ("pf_lane_kernel<NV=5, ANISO=true, TSRC=heat, TX=16, S=4, COMP=true> (fused "
+KERNEL = ("pf_lane_kernel<N=20, ANISO=true, TSRC=heat, COMP=true> (fused "
           "compensated heat + anisotropic phase field, one cell per thread, 16x16 tiles, "
           "4-slot TMA ring)")
 

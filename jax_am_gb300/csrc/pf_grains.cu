@@ -21,14 +21,15 @@
 // increasing index order (a block-wise scan), and one pass adds each tile's
 // count and first and second coordinate moments into its grains' records
 // (exact integers: per run in closed form, per tile in shared memory, then one
-// 64-bit atomic per grain of the tile and moment).  The caller orders the
-// records by (orientation, first cell) to obtain the reference's order, and
-// computes volumes and aspect ratios from the moments.
+// 64-bit atomic per grain of the tile and moment); a thread per grain takes its
+// PCA aspect ratio from the moments.  The caller orders the records by
+// (orientation, first cell) to obtain the reference's order, and the volumes
+// from the cell counts.
 //
 // Bound: latency and L2.  A cell-by-cell merge in global memory took 2306 us of
 // 2946 us at 8M cells (1,500 grains: every cell of a grain chases and updates
 // the same few roots); within a tile the chains are short and in shared memory:
-// 330 us in all (tiles 168, faces 47, roots 33, moments 48).
+// 357 us in all (tiles 148, shapes 49, faces 48, moments 48, roots 33).
 //
 // Termination: a label only ever decreases and never drops below its own
 // root's index, and a non-root always points to a smaller index, so every find
