@@ -26,11 +26,11 @@
 // the CTA waits for its copies in flight (each with the full bound) and
 // returns.
 //
-// Bound: issue slots and chains of dependent instructions at 16 warps an SM.
-// Against the TMA-fed kernel, whose lanes share a cell (its per-cell work goes
+// Bound: issue slots and chains of dependent instructions at 16 warps an SM (24
+// for n = 10 and 12).  Against the TMA-fed kernel, whose lanes share a cell (its per-cell work goes
 // through shared memory, and no vector of zeros is skipped), a moving-gradient
-// step at 128 x 128 x 64 cells, isotropic: n = 10 49 -> 33 us, 12 62 -> 30,
-// 16 49 -> 39, 20 64 -> 43, 24 79 -> 49; anisotropic 51 -> 37, 69 -> 36,
+// step at 128 x 128 x 64 cells, isotropic: n = 10 49 -> 31 us, 12 62 -> 25,
+// 16 49 -> 39, 20 64 -> 43, 24 79 -> 49; anisotropic 51 -> 31, 69 -> 29,
 // 51 -> 43, 65 -> 46, 86 -> 52.
 #include <cuda_runtime.h>
 
@@ -111,8 +111,13 @@ struct LanePlan {
       (VP == 1 || XB < 8) ? row + ((want - row) % 32 + 32) % 32 : row;  // floats
   static constexpr size_t slot = (size_t)(NC / TX + 2) * pitch * 4;
   static constexpr int tslot = ((TX + 2) * (NC / TX + 2) + 3) / 4 * 4;
-  // ring slots: four where two CTAs then fit an SM
-  static constexpr int S = 4 * (slot + 2 * tslot * 4) <= 114304 ? 4 : 3;
+  // CTAs per SM.  Three take at most 80 registers a thread and a third of
+  // shared memory: n = 10 34 -> 31 us a step at 128 x 128 x 64, n = 12 30 -> 25
+  // (anisotropic 37 -> 31, 36 -> 29); n = 14 and 16 gain at some sizes and lose
+  // 5 to 7 % at others, and 16 spills.
+  static constexpr int CTAS = N <= 12 ? 3 : 2;
+  // ring slots: four where that many CTAs then fit an SM
+  static constexpr int S = 4 * (slot + 2 * tslot * 4) <= (CTAS == 3 ? 76544 : 114304) ? 4 : 3;
 };
 // COMP: the fused heat state is compensated (T = T + T_lo, double-float
 // update).
@@ -123,7 +128,7 @@ struct LanePlan {
 // above); plane m was last read in iteration m - 1, so right after the
 // barrier that opens iteration m its slot takes plane m + S.
 template <int N, bool ANISO, int TSRC, bool COMP>
-__global__ void __launch_bounds__(LanePlan<N>::NC, 2)
+__global__ void __launch_bounds__(LanePlan<N>::NC, LanePlan<N>::CTAS)
 pf_lane_kernel(const __grid_constant__ StepArgs a) {
   using LP = LanePlan<N>;
   constexpr int NC = LP::NC, TX = LP::TX, TY = NC / TX, S = LP::S;
@@ -536,6 +541,7 @@ bool plan_lane_tiles(int nx, int ny, int nz, int n, int bcx, bool comp, int sm_c
   if (n != 20 && comp) return false;
   if (n != 20 && (int64_t)nx * ny * nz < kLaneMinCells) return false;
   TilePlan t{};
+  int ctas = 2;
   if (!with_count(n, [&](auto c) {
         using LP = LanePlan<decltype(c)::value>;
         t.vec = 2 * LP::VP;
@@ -546,12 +552,13 @@ bool plan_lane_tiles(int nx, int ny, int nz, int n, int bcx, bool comp, int sm_c
         t.pitch = LP::pitch;
         t.tslot = LP::tslot;
         t.smem = LP::S * (LP::slot + 2 * LP::tslot * sizeof(float));
+        ctas = LP::CTAS;
       }))
     return false;
   if (t.vec == 2 && (nx % 2 != 0 || bcx != PFG_BC_NEUMANN)) return false;
-  // two CTAs per SM: the dynamic shared memory plus the static variables and
+  // the CTAs of an SM: the dynamic shared memory plus the static variables and
   // the per-CTA reservation
-  if (2 * (t.smem + 1024 + 256) > (size_t)max_smem_per_sm || t.smem > (size_t)max_smem_per_block)
+  if (ctas * (t.smem + 1024 + 256) > (size_t)max_smem_per_sm || t.smem > (size_t)max_smem_per_block)
     return false;
   t.tpc = 1;
   t.cpw = 8;        // a warp owns 8 x 4 cells
@@ -560,7 +567,7 @@ bool plan_lane_tiles(int nx, int ny, int nz, int n, int bcx, bool comp, int sm_c
   t.tiles_x = (nx + t.tx - 1) / t.tx;
   t.tiles_y = (ny + t.ty - 1) / t.ty;
   const long tiles = (long)t.tiles_x * t.tiles_y;
-  int best_zc = plan_planes(tiles, nz, sm_count);
+  int best_zc = plan_planes(tiles, nz, sm_count * ctas / 2);
   if (zchunks_override > 0) best_zc = (nz + std::min(zchunks_override, nz) - 1) /
                                       std::min(zchunks_override, nz);
   t.zc = best_zc;
