@@ -8,6 +8,7 @@ uniform).  The step runs in ``libpfgb300.so``; the kernel reads the reference
 layout directly through its strides, so no transpose is made.
 """
 import ctypes
+import weakref
 
 import numpy as np
 import torch
@@ -44,7 +45,42 @@ def make_heat_params(gamma_args, nx, ny, nz, dx, dy, dz, x_first=None, y_first=N
     return h
 
 
-_coord_cache = {}
+# The coordinates of the last call that were found uniform and their first
+# centre: (weak references to x and y, what was checked, (x_first, y_first)).
+# One entry, replaced as a whole.
+_checked = None
+
+
+def _contents(a):
+    """What tells whether an array that was looked at before still holds the
+    same coordinates: a CUDA tensor's storage and version counter (no copy to
+    the host), otherwise the corners of its top plane."""
+    if torch.is_tensor(a) and a.is_cuda and not a.is_inference():
+        return a.data_ptr(), a._version, a.dtype, a.shape, a.stride()
+    return tuple(a.shape), [float(a[i, i, -1]) for i in (0, -1)]
+
+
+def _first_centre(x, y, nx, ny, dx, dy):
+    """(x_first, y_first) of cell-centre grids that must be uniform with
+    spacing dx, dy.  The check copies the top plane to the host, so its outcome
+    is kept for the next call -- for the same objects (not the same ids: a
+    freed array's id is given to another), contents, extents and spacings."""
+    global _checked
+    x, y = (a if torch.is_tensor(a) else np.asarray(a) for a in (x, y))
+    key = (nx, ny, dx, dy, _contents(x), _contents(y))
+    last = _checked
+    if last is not None and last[0]() is x and last[1]() is y and last[2] == key:
+        return last[3]
+    xt, yt = (a[:, :, -1].detach().cpu().numpy() if torch.is_tensor(a) else a[:, :, -1]
+              for a in (x, y))
+    ex = xt[0, 0] + dx * np.arange(nx)[:, None]
+    ey = yt[0, 0] + dy * np.arange(ny)[None, :]
+    if not (np.allclose(xt, ex, rtol=1e-6, atol=1e-12) and np.allclose(yt, ey, rtol=1e-6,
+                                                                      atol=1e-12)):
+        raise ValueError("x and y must be uniform cell-centre grids with spacing dx, dy")
+    first = (float(xt[0, 0]), float(yt[0, 0]))
+    _checked = (weakref.ref(x), weakref.ref(y), key, first)
+    return first
 
 
 def update_T(T, xl, yl, x, y, P, dx, dy, dz, dt, gamma_args, out=None):
@@ -57,18 +93,7 @@ def update_T(T, xl, yl, x, y, P, dx, dy, dz, dt, gamma_args, out=None):
     if T.dim() != 3:
         raise ValueError("T must be the ghosted (nx+2, ny+2, nz+2) field")
     nx, ny, nz = (s - 2 for s in T.shape)
-    key = (id(x), id(y), float(dx), float(dy))
-    if key not in _coord_cache:
-        xt, yt = (a[:, :, -1].detach().cpu().numpy() if torch.is_tensor(a)
-                  else np.asarray(a)[:, :, -1] for a in (x, y))
-        ex = xt[0, 0] + float(dx) * np.arange(nx)[:, None]
-        ey = yt[0, 0] + float(dy) * np.arange(ny)[None, :]
-        if not (np.allclose(xt, ex, rtol=1e-6, atol=1e-12) and np.allclose(yt, ey, rtol=1e-6,
-                                                                          atol=1e-12)):
-            raise ValueError("x and y must be uniform cell-centre grids with spacing dx, dy")
-        _coord_cache.clear()
-        _coord_cache[key] = (float(xt[0, 0]), float(yt[0, 0]))
-    x_first, y_first = _coord_cache[key]
+    x_first, y_first = _first_centre(x, y, nx, ny, float(dx), float(dy))
     h = make_heat_params(gamma_args, nx, ny, nz, dx, dy, dz, x_first, y_first,
                          layout=_lib.LAYOUT_XYZ)
     step = lib.pfg_heat_step

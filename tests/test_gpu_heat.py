@@ -255,3 +255,33 @@ def test_graph_replay_equals_eager():
     assert torch.equal(runs[0].state, runs[1].state)
     assert torch.equal(runs[0].T_ghosted, runs[1].T_ghosted)
     assert runs[0].steps_taken == runs[1].steps_taken == 47
+
+
+def test_update_T_places_the_beam_by_the_coordinates_given():
+    """Grids of equal spacing and different origins, each freed before the next
+    is made, and one moved in place: the result is that of the same call with
+    arrays that were never used before."""
+    from jax_am_gb300.cfd.gamma import update_T
+    nx, ny, nz, h = 24, 16, 8, 1e-5
+    T = torch.full((nx + 2, ny + 2, nz + 2), 300.0, device="cuda")
+
+    def grid(k):
+        return torch.meshgrid(*((torch.arange(m, device="cuda", dtype=torch.float32) + 0.5 + o) * h
+                                for m, o in ((nx, 3 * k), (ny, -2 * k), (nz, 0))),
+                              indexing="ij")[:2]
+
+    def step(x, y):
+        return update_T(T, 12 * h, 8 * h, x, y, 50.0, h, h, h, 1e-7, GAMMA_DEFAULTS)
+    held = [grid(k) for k in range(8)]
+    expected = [step(*g) for g in held]
+    assert not torch.equal(expected[0], expected[1])
+    for k in range(8):
+        x, y = grid(k)
+        assert torch.equal(step(x, y), expected[k]), k
+        assert torch.equal(step(x, y), expected[k]), k
+        del x, y
+    x, y = (a.clone() for a in held[0])
+    assert torch.equal(step(x, y), expected[0])
+    x.copy_(held[1][0])
+    y.copy_(held[1][1])
+    assert torch.equal(step(x, y), expected[1])
