@@ -134,3 +134,49 @@ def test_adjoint_tile_edges(shape, n, ckpt, aniso):
     assert abs(J - Jt.item()) <= 1e-5 * abs(Jt.item())
     assert abs(gP - rP) <= 1e-3 * abs(rP) and abs(gv - rv) <= 1e-3 * abs(rv)
     assert np.linalg.norm(ge.double().cpu().numpy() - re) <= 1e-3 * np.linalg.norm(re)
+
+
+@pytest.mark.parametrize("shape,n", [((1, 1, 1), 1), ((5, 3, 2), 3), ((13, 7, 5), 10),
+                                     ((37, 31, 23), 64), ((80, 75, 64), 7)])
+def test_objective_in_float64(shape, n):
+    """J of values over float32's whole range against the exact sum; the bound
+    is one rounding of 2^-53 per addition of the longest chain (a thread's
+    elements, the trees, the blocks).  A diverged state's J is infinite."""
+    import ctypes
+    import math
+    from jax_am_gb300 import _lib
+    from jax_am_gb300.phase_field.allen_cahn import make_pf_params
+    lib = _lib.load()
+    nx, ny, nz = shape
+    N = nx * ny * nz
+    poly, _, _, pf_args, _, _ = pf_case(shape, n, 0.0, seed=2, h=(1e-6,) * 3)
+    p = make_pf_params(pf_args, poly)
+    rng = np.random.default_rng(n)
+    eta, w = f32(rng.standard_normal((N, n))), f32(rng.random(n) - 0.2)
+    w = np.where(np.abs(w) < 1e-3, 0.5, w)
+
+    def J_of(eta):
+        e = torch.tensor(eta, dtype=torch.float32, device="cuda")
+        J = torch.zeros(1, dtype=torch.float64, device="cuda")
+        lam = torch.empty_like(e)
+        wd = torch.tensor(w, dtype=torch.float32, device="cuda")
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        for seed in (None, lam):
+            J.zero_()
+            _lib.check(lib.pfg_objective(ctypes.byref(p), _lib.ptr(e), _lib.ptr(wd), _lib.ptr(J),
+                                         _lib.ptr(seed), stream), "pfg_objective")
+        return J.item(), lam
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    threads = min(N * n, sms * 8 * 256) // 2
+    roundings = N * n / max(1, threads) + 16 + 8 * sms
+    for scale in (1.0, 1e18, 1e25, 1e-25):
+        x = f32(eta * scale)
+        J, lam = J_of(x)
+        terms = (w * x * x).reshape(-1)
+        exact, size = math.fsum(terms), math.fsum(np.abs(terms))
+        assert abs(J - exact / N) <= roundings * 2.0 ** -53 * size / N, scale
+        ref = np.float32(2) * np.float32(w) * np.float32(x) * (np.float32(1) / np.float32(N))
+        with np.errstate(over="ignore"):
+            np.testing.assert_array_equal(lam.cpu().numpy(), ref)
+    eta[N // 2, n // 2] = np.inf
+    assert J_of(eta)[0] == math.copysign(math.inf, w[n // 2])
