@@ -394,7 +394,8 @@ int pfg_batch_advance(void* device_table, int k_steps, void* stream);
  * and Tb_out = dJ/d Tg^k (interior and the six ghost faces; the caller zeroes
  * edge/corner entries once) and adds this step's contributions to grads[0]
  * (dJ/d beam power) and grads[1] (dJ/d scan speed, with dxl_dv = d x_beam / d v
- * at the mid-step time).  scratch: pfg_adjoint_scratch_bytes(p) bytes. */
+ * at the mid-step time).  scratch: pfg_adjoint_scratch_bytes(p) bytes.  lam_out
+ * may be lam_in or eta (slower without anisotropy); Tb_out not Tb_in or Tg. */
 int64_t pfg_adjoint_scratch_bytes(const pfg_pf_params* p);
 int pfg_adjoint_step(const pfg_pf_params* p, const pfg_heat_params* h, const float* eta,
                      const float* Tg, double t, float dt, const float* lam_in, const float* Tb_in,

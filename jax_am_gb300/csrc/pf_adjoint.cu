@@ -20,8 +20,8 @@
 // cell, so one launch per cell (heat transpose and the cell coefficients) and
 // one per order parameter do the step and no (N, n) field is written but
 // lam_out: at 1M cells, n = 10, 63 us against 230 us with the fields written and
-// gathered.  With anisotropy the fields u, v and loc go through memory (kernels
-// A, B, then C).
+// gathered.  With anisotropy, or with an output in the place of an input, the
+// fields u, v and loc go through memory (kernels A, B, then C).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -573,6 +573,11 @@ objective_kernel(const float* __restrict__ eta, const float* __restrict__ w, lon
 
 using namespace pfg;
 
+// Whether [a, a + na) and [b, b + nb) share an element.
+static bool overlap(const float* a, int64_t na, const float* b, int64_t nb) {
+  return a < b + nb && b < a + na;
+}
+
 extern "C" int64_t pfg_adjoint_scratch_bytes(const pfg_pf_params* p) {
   if (check_pf_params(p)) return -1;
   const int64_t N = (int64_t)p->nx * p->ny * p->nz;
@@ -631,9 +636,16 @@ extern "C" int pfg_adjoint_step(const pfg_pf_params* p, const pfg_heat_params* h
   const DeviceInfo& d = device_info();
   const int cpw = 32 / ((p->num_oris + 1) / 2);  // cells per warp of the element kernels
   const int cell_blocks = (int)std::min<int64_t>((N + 255) / 256, (int64_t)d.sm_count * 16);
-  // the isotropic kernel's in-plane offsets are 32-bit (a plane of 2^31 elements
-  // takes the other kernels)
-  if (!(a.pc.aniso > 0.f) && (int64_t)p->nx * p->ny * p->num_oris < ((int64_t)1 << 31)) {
+  // The isotropic kernel reads eta and lam_in at neighbours while others write
+  // lam_out, and after Tb_out is written.  Kernels A and B read lam_in at the
+  // element that they write and have read eta before, and C writes Tb_out last,
+  // so outputs there may take the place of eta or lam_in.
+  const int64_t Ng = (int64_t)(p->nx + 2) * (p->ny + 2) * (p->nz + 2);
+  const bool in_place = overlap(lam_out, Nn, lam_in, Nn) || overlap(lam_out, Nn, eta, Nn) ||
+                        overlap(Tb_out, Ng, lam_in, Nn) || overlap(Tb_out, Ng, eta, Nn);
+  // its in-plane offsets are 32-bit (a plane of 2^31 elements takes the others)
+  if (!(a.pc.aniso > 0.f) && !in_place &&
+      (int64_t)p->nx * p->ny * p->num_oris < ((int64_t)1 << 31)) {
     a.q = sc;
     a.g = sc + N;
     a.om2 = sc + 2 * N;

@@ -180,3 +180,52 @@ def test_objective_in_float64(shape, n):
             np.testing.assert_array_equal(lam.cpu().numpy(), ref)
     eta[N // 2, n // 2] = np.inf
     assert J_of(eta)[0] == math.copysign(math.inf, w[n // 2])
+
+
+def _adjoint_step_inputs(shape, n, aniso, force=False, seed=6):
+    """One adjoint step's arguments on random fields, and the call."""
+    import ctypes
+    from jax_am_gb300 import _lib
+    from jax_am_gb300.cfd.gamma import make_heat_params
+    from jax_am_gb300.phase_field.allen_cahn import make_pf_params
+    lib = _lib.load()
+    nx, ny, nz = shape
+    poly, eta, _, pf_args, _, _ = pf_case(shape, n, aniso, seed=seed, h=(1e-6,) * 3, force=force)
+    p = make_pf_params(pf_args, poly)
+    h = make_heat_params(dict(GAMMA_DEFAULTS, r=8e-6), nx, ny, nz, 1e-6, 1e-6, 1e-6,
+                         path=[(0.0, 1.0, 2e-6, 3e-6, 1.0, 3e-6, 2.0)])
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    eta = torch.tensor(eta, dtype=torch.float32, device="cuda")
+    lam = torch.randn(eta.shape, generator=g, device="cuda")
+    Tg = 1000.0 + 1100.0 * torch.rand((nz + 2, ny + 2, nx + 2), generator=g, device="cuda")
+    Tb = torch.randn(Tg.shape, generator=g, device="cuda")
+    scratch = torch.empty(int(lib.pfg_adjoint_scratch_bytes(ctypes.byref(p))), dtype=torch.uint8,
+                          device="cuda")
+
+    def step(eta, lam, lam_out, Tb_out):
+        grads = torch.zeros(2, dtype=torch.float64, device="cuda")
+        st = lib.pfg_adjoint_step(ctypes.byref(p), ctypes.byref(h), _lib.ptr(eta), _lib.ptr(Tg),
+                                  0.0, 3e-8, _lib.ptr(lam), _lib.ptr(Tb), _lib.ptr(lam_out),
+                                  _lib.ptr(Tb_out), _lib.ptr(scratch), scratch.numel(),
+                                  _lib.ptr(grads), 1e-3,
+                                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        _lib.check(st, "pfg_adjoint_step")
+        return grads
+    return eta, lam, Tg, Tb, step
+
+
+@pytest.mark.parametrize("aniso", [0.0, 0.15])
+@pytest.mark.parametrize("shape,n", [((33, 21, 12), 10), ((14, 9, 5), 7)])
+def test_adjoint_step_in_place(shape, n, aniso):
+    """lam_out in the place of lam_in or of eta: the isotropic step's two forms
+    round alike, so equal bit for bit to separate buffers."""
+    eta, lam, Tg, Tb, step = _adjoint_step_inputs(shape, n, aniso)
+    ref, Tref = torch.empty_like(lam), torch.zeros_like(Tb)
+    gref = step(eta, lam, ref, Tref)
+    for out in ("lam", "eta"):
+        e, l, T = eta.clone(), lam.clone(), torch.zeros_like(Tb)
+        o = l if out == "lam" else e
+        grads = step(e, l, o, T)
+        assert torch.equal(o, ref), out
+        assert torch.equal(T, Tref), out
+        assert torch.allclose(grads, gref, rtol=1e-12)  # the blocks' order of atomics
