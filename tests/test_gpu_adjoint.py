@@ -217,8 +217,10 @@ def _adjoint_step_inputs(shape, n, aniso, force=False, seed=6):
 @pytest.mark.parametrize("aniso", [0.0, 0.15])
 @pytest.mark.parametrize("shape,n", [((33, 21, 12), 10), ((14, 9, 5), 7)])
 def test_adjoint_step_in_place(shape, n, aniso):
-    """lam_out in the place of lam_in or of eta: the isotropic step's two forms
-    round alike, so equal bit for bit to separate buffers."""
+    """lam_out in the place of lam_in or of eta against separate buffers: the
+    same kernels with anisotropy, so equal; without it the one-pass kernel's
+    results, whose terms (no larger than the largest result) a compiler may
+    contract otherwise: 16 roundings of 2^-24."""
     eta, lam, Tg, Tb, step = _adjoint_step_inputs(shape, n, aniso)
     ref, Tref = torch.empty_like(lam), torch.zeros_like(Tb)
     gref = step(eta, lam, ref, Tref)
@@ -226,6 +228,7 @@ def test_adjoint_step_in_place(shape, n, aniso):
         e, l, T = eta.clone(), lam.clone(), torch.zeros_like(Tb)
         o = l if out == "lam" else e
         grads = step(e, l, o, T)
-        assert torch.equal(o, ref), out
-        assert torch.equal(T, Tref), out
+        for got, want in ((o, ref), (T, Tref)):
+            tol = 0.0 if aniso else 2.0 ** -20 * float(want.abs().max())
+            assert float((got - want).abs().max()) <= tol, out
         assert torch.allclose(grads, gref, rtol=1e-12)  # the blocks' order of atomics
