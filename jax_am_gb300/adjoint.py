@@ -43,10 +43,6 @@ class LaserTrackProblem:
         self.C = max(1, int(checkpoint_every))
         self.x_start, self.y = float(x_start), float(y)
         self.t_end = self.steps * self.dt * 2.0 + 1.0  # the track outlasts the run
-        # the device clock at each step: float32 dt summed in float64, in order
-        self.times = [0.0]
-        for _ in range(self.steps):
-            self.times.append(self.times[-1] + self.dt)
         p = self.p
         self.N = p.nx * p.ny * p.nz
         self.n = p.num_oris
@@ -56,6 +52,13 @@ class LaserTrackProblem:
             T_init = torch.full(self.gshape, float(gamma_args["T0"]), dtype=torch.float32)
         self.T_init = T_init.to("cuda", torch.float32).reshape(self.gshape).contiguous()
         self._ckpt = None
+
+    def _times(self):
+        """The device clock at each step: float32 dt summed in float64, in order."""
+        times = [0.0]
+        for _ in range(self.steps):
+            times.append(times[-1] + float(np.float32(self.dt)))
+        return times
 
     def heat_params(self, P, v):
         x1 = self.x_start + v * self.t_end
@@ -69,14 +72,13 @@ class LaserTrackProblem:
                                        _lib.ptr(clk_in), _lib.ptr(clk_out), self.dt, _stream())
         _lib.check(st, "pfg_heat_pf_step")
 
-    def _advance(self, h, eta, T, k0, steps, keep_every):
-        """Advance (eta, T), the state of step ``k0``, by ``steps`` steps;
-        returns the final state and the kept ones, steps ``k0``, ``k0 +
-        keep_every``, ...  The states that are not kept alternate between two
+    def _advance(self, h, eta, T, t, steps, keep_every):
+        """Advance (eta, T), the state at time ``t``, by ``steps`` steps;
+        returns the final state and every ``keep_every``-th one, the first
+        among them.  The states that are not kept alternate between two
         buffers; nothing is copied and the inputs are not written."""
         clk = torch.empty((2, 2), dtype=torch.int64, device="cuda")
-        _lib.check(self.lib.pfg_clock_set(_lib.ptr(clk[0]), self.times[k0], k0, _stream()),
-                   "pfg_clock_set")
+        _lib.check(self.lib.pfg_clock_set(_lib.ptr(clk[0]), t, 0, _stream()), "pfg_clock_set")
         kept, free = [], []
         state, own = (eta, T), False  # own: the state's buffers may be written again
         for k in range(steps):
@@ -103,7 +105,8 @@ class LaserTrackProblem:
         h = self.heat_params(self.P, self.v)
         eta = eta0.to("cuda", torch.float32).reshape(self.N, self.n).contiguous()
         # the first checkpoint is a copy: the caller may write eta0 before gradient()
-        (eta_f, _), ckpt = self._advance(h, eta.clone(), self.T_init.clone(), 0, self.steps, self.C)
+        (eta_f, _), ckpt = self._advance(h, eta.clone(), self.T_init.clone(), 0.0, self.steps,
+                                         self.C)
         self._ckpt = ckpt
         self._eta_final = eta_f
         return float(self.objective(eta_f).item())
@@ -120,15 +123,15 @@ class LaserTrackProblem:
         grads = torch.zeros(2, dtype=torch.float64, device="cuda")
         nbytes = int(self.lib.pfg_adjoint_scratch_bytes(ctypes.byref(self.p)))
         scratch = torch.empty(nbytes // 4 + 1, dtype=torch.float32, device="cuda")
-        dt = self.dt
+        dt, times = self.dt, self._times()
         for seg in reversed(range(len(self._ckpt))):
             k0 = seg * self.C
             nseg = min(self.C, self.steps - k0)
             # the segment's states again (its last step's result is not needed)
-            last, states = self._advance(h, *self._ckpt[seg], k0, nseg - 1, 1)
+            last, states = self._advance(h, *self._ckpt[seg], times[k0], nseg - 1, 1)
             states.append(last)
             for j in reversed(range(nseg)):
-                t = self.times[k0 + j]
+                t = times[k0 + j]
                 e_k, T_k = states.pop()
                 st = self.lib.pfg_adjoint_step(
                     ctypes.byref(self.p), ctypes.byref(h), _lib.ptr(e_k), _lib.ptr(T_k), t, dt,

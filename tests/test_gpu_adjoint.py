@@ -232,3 +232,26 @@ def test_adjoint_step_in_place(shape, n, aniso):
             tol = 0.0 if aniso else 2.0 ** -20 * float(want.abs().max())
             assert float((got - want).abs().max()) <= tol, out
         assert torch.allclose(grads, gref, rtol=1e-12)  # the blocks' order of atomics
+
+
+def test_steps_and_dt_of_a_problem_may_change():
+    """``steps`` and ``dt`` are read at each run: a problem made with others and
+    then changed gives what one made with them gives."""
+    from jax_am_gb300.adjoint import LaserTrackProblem
+    shape, n = (9, 7, 5), 4
+    poly, eta, Tg, pf_args, oargs, g, w = _setup(0.0, 7, 3, shape, n)
+    e0 = torch.tensor(eta, dtype=torch.float32, device="cuda")
+
+    def problem(steps, dt):
+        return LaserTrackProblem(pf_args, poly, g, w, dt, steps, 1e-6, 2e-6, checkpoint_every=3,
+                                 T_init=torch.tensor(Tg))
+    want, got = problem(7, 3e-8), problem(2, 1e-8)
+    got.steps, got.dt, got.t_end = want.steps, want.dt, want.t_end
+    res = []
+    for p in (want, got):
+        J = p.forward(2.0, 0.8, e0)
+        res.append((J, *p.gradient()))
+    a, b = res
+    assert abs(a[0] - b[0]) <= 1e-14 * abs(a[0])
+    assert abs(a[1] - b[1]) <= 1e-12 * abs(a[1]) and abs(a[2] - b[2]) <= 1e-12 * abs(a[2])
+    assert torch.equal(a[3], b[3])
