@@ -52,7 +52,7 @@ struct AdjArgs {
   float* loc;          // (N, n)
   float* muPF;         // (N) dt * sum_i lam_i dR_i/dT
   float* mask;         // (N) 0 where liquid forcing zeroed the cell, else 1
-  // isotropic step, per cell: Lg kappa' (0 where liquid), Lg m_g / ad_hoc,
+  // isotropic step, per cell: Lg kappa' (-0 where liquid), Lg m_g / ad_hoc,
   // 2 (1 - zeta)^2 (-1 where liquid) and d Lg / dT
   float* q;
   float* g;
@@ -311,7 +311,11 @@ adj_pf_iso_kernel(const __grid_constant__ AdjArgs a) {
   const int cxm = y * a.nx + nbr(x, -1, a.nx, a.bcx), cxp = y * a.nx + nbr(x, 1, a.nx, a.bcx);
   const int cym = nbr(y, -1, a.ny, a.bcy) * a.nx + x, cyp = nbr(y, 1, a.ny, a.bcy) * a.nx + x;
   const float mg = a.pc.mg_ad, kap = a.pc.kappa_ad;
-  auto u_of = [](float2 l, float q) { return make_float2(__fmul_rn(l.x, q), __fmul_rn(l.y, q)); };
+  // u of a cell: 0 where liquid (q = -0), whatever its lam
+  auto u_of = [](float2 l, float q) {
+    const bool off = __float_as_uint(q) == 0x80000000u;
+    return make_float2(off ? 0.f : __fmul_rn(l.x, q), off ? 0.f : __fmul_rn(l.y, q));
+  };
   const int64_t first = (int64_t)c0 * n + i0;
   const float* eta = a.eta + first;
   const float* lam = a.lam_in + first;
@@ -373,7 +377,7 @@ adj_pf_iso_kernel(const __grid_constant__ AdjArgs a) {
       mu += lamm * (dLg * (-mg * gg + kap * L) + Lgm * 4.f * om * e * dz);
       const float lapu = a.pc.wx * (u0 + u1 - 2.f * u) + a.pc.wy * (u2 + u3 - 2.f * u) +
                          a.pc.wz * (u4 + u5 - 2.f * u);
-      return __fadd_rn(liquid ? 0.f : l, __fmul_rn(a.dt, loc + lapu));
+      return fmaf(liquid ? 0.f : 1.f, l, __fmul_rn(a.dt, loc + lapu));
     };
     float2 out;
     out.x = element(ec.x, exm.x, exp_.x, eym.x, eyp.x, em.x, ep.x, lc.x, uc.x, uxm.x, uxp.x, uym.x,
@@ -433,7 +437,7 @@ __global__ void __launch_bounds__(256) adj_cell_kernel(const __grid_constant__ A
     a.alpha[c] = heat_local(a.hc, T).alpha;
     if constexpr (ISO) {
       const AdjTemp tq = adj_temp(a.pc, T);
-      a.q[c] = tq.liquid ? 0.f : tq.Lg * a.pc.kappa_ad;
+      a.q[c] = tq.liquid ? -0.f : tq.Lg * a.pc.kappa_ad;
       a.g[c] = tq.Lg * a.pc.mg_ad;
       a.om2[c] = tq.liquid ? -1.f : 2.f * tq.om * tq.om;
       a.dLg[c] = tq.dLg;

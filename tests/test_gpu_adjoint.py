@@ -255,3 +255,25 @@ def test_steps_and_dt_of_a_problem_may_change():
     assert abs(a[0] - b[0]) <= 1e-14 * abs(a[0])
     assert abs(a[1] - b[1]) <= 1e-12 * abs(a[1]) and abs(a[2] - b[2]) <= 1e-12 * abs(a[2])
     assert torch.equal(a[3], b[3])
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_adjoint_step_non_finite_at_liquid_cells(value):
+    """A non-finite adjoint at cells that liquid forcing zeroed stays there: the
+    one-pass kernel's other cells hold what the kernels that go through
+    scratch (lam_out in the place of lam_in) give, finite and equal to 16
+    roundings of the largest."""
+    from tests.cases import PF_DEFAULTS
+    eta, lam, Tg, Tb, step = _adjoint_step_inputs((19, 13, 9), 10, 0.0, force=True)
+    T = Tg[1:-1, 1:-1, 1:-1].reshape(-1)
+    liquid = T > PF_DEFAULTS["T_liquidus"] + 1.0
+    assert 0.2 < float(liquid.float().mean()) < 0.8
+    lam[liquid, 3] = value
+    out, T_out = torch.empty_like(lam), torch.zeros_like(Tb)
+    step(eta, lam, out, T_out)
+    ref, T_ref = lam.clone(), torch.zeros_like(Tb)
+    step(eta, ref, ref, T_ref)
+    assert bool(ref[~liquid].isfinite().all()) and bool(T_ref.isfinite().all())
+    assert torch.equal(out.isfinite(), ref.isfinite())
+    for got, want in ((out[ref.isfinite()], ref[ref.isfinite()]), (T_out, T_ref)):
+        assert float((got - want).abs().max()) <= 2.0 ** -20 * float(want.abs().max())
