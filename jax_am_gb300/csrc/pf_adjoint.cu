@@ -311,11 +311,7 @@ adj_pf_iso_kernel(const __grid_constant__ AdjArgs a) {
   const int cxm = y * a.nx + nbr(x, -1, a.nx, a.bcx), cxp = y * a.nx + nbr(x, 1, a.nx, a.bcx);
   const int cym = nbr(y, -1, a.ny, a.bcy) * a.nx + x, cyp = nbr(y, 1, a.ny, a.bcy) * a.nx + x;
   const float mg = a.pc.mg_ad, kap = a.pc.kappa_ad;
-  // u of a cell: 0 where liquid (q = -0), whatever its lam
-  auto u_of = [](float2 l, float q) {
-    const bool off = __float_as_uint(q) == 0x80000000u;
-    return make_float2(off ? 0.f : __fmul_rn(l.x, q), off ? 0.f : __fmul_rn(l.y, q));
-  };
+  auto u_of = [](float2 l, float q) { return make_float2(__fmul_rn(l.x, q), __fmul_rn(l.y, q)); };
   const int64_t first = (int64_t)c0 * n + i0;
   const float* eta = a.eta + first;
   const float* lam = a.lam_in + first;
@@ -333,14 +329,14 @@ adj_pf_iso_kernel(const __grid_constant__ AdjArgs a) {
     const bool wraps = z + 1 == a.nz;  // the plane above: the next, this one or the first
     const int64_t up_at = wraps ? (a.bcz ? -(int64_t)(a.nz - 1) * sz : 0) : sz;
     const float2 ep = load_two<VEC>(eta + up_at, second), lp = load_two<VEC>(lam + up_at, second);
-    const float2 up = u_of(lp, a.q[cz + (wraps ? (a.bcz ? -(a.nz - 1) * xy : 0) : xy)]);
+    float2 up = u_of(lp, a.q[cz + (wraps ? (a.bcz ? -(a.nz - 1) * xy : 0) : xy)]);
     const float2 exm = load_two<VEC>(eta + nxm, second), exp_ = load_two<VEC>(eta + nxp, second);
     const float2 eym = load_two<VEC>(eta + nym, second), eyp = load_two<VEC>(eta + nyp, second);
     const float* qz = a.q + (cz - c0);
-    const float2 uxm = u_of(load_two<VEC>(lam + nxm, second), qz[cxm]);
-    const float2 uxp = u_of(load_two<VEC>(lam + nxp, second), qz[cxp]);
-    const float2 uym = u_of(load_two<VEC>(lam + nym, second), qz[cym]);
-    const float2 uyp = u_of(load_two<VEC>(lam + nyp, second), qz[cyp]);
+    float2 uxm = u_of(load_two<VEC>(lam + nxm, second), qz[cxm]);
+    float2 uxp = u_of(load_two<VEC>(lam + nxp, second), qz[cxp]);
+    float2 uym = u_of(load_two<VEC>(lam + nym, second), qz[cym]);
+    float2 uyp = u_of(load_two<VEC>(lam + nyp, second), qz[cyp]);
     const float Lgm = a.g[cz], o2 = a.om2[cz], dLg = a.dLg[cz];
     const bool liquid = o2 < 0.f;
     // per-cell sums
@@ -380,11 +376,32 @@ adj_pf_iso_kernel(const __grid_constant__ AdjArgs a) {
       return fmaf(liquid ? 0.f : 1.f, l, __fmul_rn(a.dt, loc + lapu));
     };
     float2 out;
-    out.x = element(ec.x, exm.x, exp_.x, eym.x, eyp.x, em.x, ep.x, lc.x, uc.x, uxm.x, uxp.x, uym.x,
-                    uyp.x, um.x, up.x);
-    if (second)
-      out.y = element(ec.y, exm.y, exp_.y, eym.y, eyp.y, em.y, ep.y, lc.y, uc.y, uxm.y, uxp.y,
-                      uym.y, uyp.y, um.y, up.y);
+    auto both = [&] {
+      mu = 0.f;
+      out.x = element(ec.x, exm.x, exp_.x, eym.x, eyp.x, em.x, ep.x, lc.x, uc.x, uxm.x, uxp.x,
+                      uym.x, uyp.x, um.x, up.x);
+      if (second)
+        out.y = element(ec.y, exm.y, exp_.y, eym.y, eyp.y, em.y, ep.y, lc.y, uc.y, uxm.y, uxp.y,
+                        uym.y, uyp.y, um.y, up.y);
+    };
+    both();
+    // A liquid cell has no u (q = -0) whatever its lam, but 0 times a non-finite
+    // lam is NaN: looked at where a result shows it (as a test at every u, 85
+    // -> 94 us a step at 1M cells, n = 10).
+    if (!isfinite(out.x) || (second && !isfinite(out.y))) {
+      auto clear = [&](float2& u, int64_t cell) {
+        if (__float_as_uint(a.q[cell]) == 0x80000000u) u = make_float2(0.f, 0.f);
+      };
+      const int64_t below = (int64_t)nbr(z, -1, a.nz, a.bcz) * xy + c0;
+      clear(uc, cz);
+      clear(um, below);
+      clear(up, (int64_t)nbr(z, 1, a.nz, a.bcz) * xy + c0);
+      clear(uxm, cz - c0 + cxm);
+      clear(uxp, cz - c0 + cxp);
+      clear(uym, cz - c0 + cym);
+      clear(uyp, cz - c0 + cyp);
+      both();
+    }
     if (valid) {
       float* o = a.lam_out + (lam - a.lam_in);
       if constexpr (VEC) {
@@ -538,11 +555,18 @@ __global__ void __launch_bounds__(256) adj_heat_kernel(const __grid_constant__ A
 }
 
 // ---- objective J = mean over cells of sum_i w_i eta_i^2 and its seed ----------
-// Float64 throughout.  A thread keeps to one orientation (the launch's threads,
-// less a remainder, are a whole number of cells), so its weight is applied once
-// and an element costs one conversion and one fused multiply-add of the float64
-// pipe, which bounds this kernel, instead of two conversions and three
-// operations.
+// Float64 throughout.  The float64 pipe bounds this kernel (two lanes a clock an
+// SM), so an element takes one instruction of it: a thread keeps to one
+// orientation (the launch's threads, less a remainder, are a whole number of
+// cells) and applies its weight once, and integer instructions widen the values
+// (1M cells, n = 10: 28 us a launch; with conversions 46, with a product and a
+// weight an element 85).
+
+// |v| as a double, of a value that is zero or normal: the exponent's bias and
+// place change.
+__device__ __forceinline__ double widened_abs(unsigned m) {
+  return __hiloint2double((int)((m >> 3) + (m ? 0x38000000u : 0u)), (int)(m << 29));
+}
 template <bool SEED>
 __global__ void __launch_bounds__(256)
 objective_kernel(const float* __restrict__ eta, const float* __restrict__ w, long long ncell, int n,
@@ -554,10 +578,22 @@ objective_kernel(const float* __restrict__ eta, const float* __restrict__ w, lon
   double sum = 0.0;
   if (first < stride && first < total) {
     const float wi = __ldg(w + (int)(first % n));
+    bool other = false;  // a denormal, infinite or NaN value
+#pragma unroll 4
     for (long long e = first; e < total; e += stride) {
       const float v = __ldg(eta + e);
-      sum = fma((double)v, (double)v, sum);
+      const unsigned m = __float_as_uint(v) & 0x7fffffffu;
+      other |= m - 1u < 0x007fffffu || m >= 0x7f800000u;
+      const double d = widened_abs(m);
+      sum = fma(d, d, sum);
       if (SEED) lam[e] = 2.f * wi * v * inv;
+    }
+    if (other) {
+      sum = 0.0;
+      for (long long e = first; e < total; e += stride) {
+        const double d = (double)__ldg(eta + e);
+        sum = fma(d, d, sum);
+      }
     }
     sum *= (double)wi;
   }
