@@ -135,9 +135,15 @@ static int heat_step(const pfg_heat_params* h, const float* Tg_in, float* Tg_out
   if ((int64_t)(h->nx + 2) * (h->ny + 2) * (h->nz + 2) >= ((int64_t)1 << 31)) return PFG_ERR_SHAPE;
   const HeatConsts H = make_heat_consts(*h);
   const bool xyz = h->layout == PFG_LAYOUT_XYZ;
-  if (((xyz ? h->nx : h->nz) + kHeatChunk - 1) / kHeatChunk > 65535 - (edges ? 1 : 0))
-    return PFG_ERR_SHAPE;
+  const int chunks = ((xyz ? h->nx : h->nz) + kHeatChunk - 1) / kHeatChunk;
+  if (chunks > 65535) return PFG_ERR_SHAPE;
   cudaError_t e;
+  if (edges && chunks == 65535) {  // no grid row left for the edges: the whole field first
+    const size_t bytes = sizeof(float) * (h->nx + 2) * (h->ny + 2) * (h->nz + 2);
+    e = cudaMemcpyAsync(Tg_out, Tg_in, bytes, cudaMemcpyDeviceToDevice, s);
+    if (e != cudaSuccess) return record_cuda(e);
+    edges = false;
+  }
   if (xyz) e = edges ? launch_heat<true, true>(H, Tg_in, Tg_out, xl, yl, power, dt, s)
                      : launch_heat<true, false>(H, Tg_in, Tg_out, xl, yl, power, dt, s);
   else e = edges ? launch_heat<false, true>(H, Tg_in, Tg_out, xl, yl, power, dt, s)

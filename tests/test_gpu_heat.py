@@ -285,3 +285,30 @@ def test_update_T_places_the_beam_by_the_coordinates_given():
     x.copy_(held[1][0])
     y.copy_(held[1][1])
     assert torch.equal(step(x, y), expected[1])
+
+
+@pytest.mark.parametrize("nx", [8 * 65534, 8 * 65535])
+def test_update_T_longest_grids(nx):
+    """The grid's longest slow axis, with and without a row of blocks left for
+    the edges: a new field is a copy of the old one that the step then wrote."""
+    from jax_am_gb300.cfd.gamma import update_T
+    h, ny, nz = 1e-6, 2, 1
+    g = torch.Generator(device="cuda").manual_seed(1)
+    T = 300.0 + 1500.0 * torch.rand((nx + 2, ny + 2, nz + 2), generator=g, device="cuda")
+    x, y = torch.meshgrid(*((torch.arange(m, device="cuda", dtype=torch.float64) + 0.5) * h
+                            for m in (nx, ny, nz)), indexing="ij")[:2]
+    args = (0.5 * nx * h, h, x, y, 50.0, h, h, h, 1e-9, GAMMA_DEFAULTS)
+    ref = T.clone()
+    update_T(T, *args, out=ref)
+    assert torch.equal(update_T(T, *args), ref)
+
+
+def test_update_T_refuses_longer_grids():
+    from jax_am_gb300.cfd.gamma import update_T
+    h, nx = 1e-6, 8 * 65535 + 1
+    x, y = np.meshgrid((np.arange(nx) + 0.5) * h, [0.5 * h], indexing="ij")
+    T = torch.full((nx + 2, 3, 3), 300.0, device="cuda")
+    for out in (None, T.clone()):
+        with pytest.raises(ValueError):
+            update_T(T, 0.0, 0.0, x[..., None], y[..., None], 50.0, h, h, h, 1e-9,
+                     GAMMA_DEFAULTS, out=out)
