@@ -544,6 +544,9 @@ __device__ __forceinline__ bool solve_reduce(const SolveArgs& a, SolveShared& sh
                                              bool& late) {
   bar_wait<kSolveThreads>(kBarSums);
   if (sh.late) late = true;
+  // The first partial also says that this block's words of phat and shat are
+  // cleared: a release of what its working threads wrote before the barrier.
+  if (seq == 1) __threadfence();
   if (i < D) {
     Posted* part = a.board->part[PART + i];
     const int half = (lane >> 3) & 1, vb = 2 * (int)blockIdx.x + half;
