@@ -214,7 +214,9 @@ int pfg_device_error(int clear);
  * TMA-fed and cell-per-lane kernels first waits that long on a barrier that
  * nothing completes, so the launch takes its timeout path (the CTA waits for
  * its copies in flight and returns; PFG_ERR_TIMEOUT in pfg_device_error)
- * without any fault; its output is then invalid.  Process-wide; the stencil
+ * without any fault; its output is then invalid, and the CFD solver's resident
+ * solves wait that long for a partial sum that nothing posts (PFG_ERR_TIMEOUT
+ * from the call).  Process-wide; the stencil
  * steps' results do not change; the CFD solver's dot products are summed in
  * another order (float64 rounding only). */
 int pfg_tune(int key, int value);
@@ -584,7 +586,8 @@ int pfg_cfd_solid_update(const pfg_cfd_grid* g, double Ts, double Tl, const doub
  * 287-323) followed by update_convective_terms (cfd_am.py:254-259): reads T
  * and the box's vel, conv and grad_p0 from the global arrays, writes the
  * box's vel, grad_p0, conv and conv_T back.  The convective terms use the
- * global cell size, the solves the local box's (as the reference does). */
+ * global cell size, the solves the local box's (as the reference does).  With
+ * PFG_ERR_TIMEOUT (a wait of a solve ran out) the arrays are as they were. */
 int pfg_cfd_flow_step(const pfg_cfd_grid* global, const pfg_cfd_grid* local,
                       const pfg_cfd_flow* f, const double* T, double* vel, double* conv,
                       double* grad_p0, double* conv_T, void* ws, int64_t ws_bytes,

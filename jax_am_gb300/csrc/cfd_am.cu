@@ -29,6 +29,7 @@
 
 namespace pfg {
 int g_cfd_cells_per_thread = 4;  // pfg_tune key 6
+extern long long g_probe_wait;   // pfg_tune key 8
 
 namespace cfd {
 
@@ -412,7 +413,9 @@ __global__ void k_e(long long n, KState* st, double* P, double* x, double* r, co
 //
 // The blocks wait on one another, so the launch is cooperative (all of them
 // resident, at most one per SM), and each wait is bounded: one that runs out
-// sets the abort word, and every block returns.
+// sets the abort word and its block returns, as do the others when their waits
+// for it run out.  The launches behind an aborted solve leave the caller's
+// fields as they are.
 constexpr int kSolveCells = 4;      // cells per thread, at most
 constexpr int kSolveWork = 512;     // working threads: two 256-thread blocks of the kernels above
 constexpr int kSolveThreads = kSolveWork + 96;
@@ -457,6 +460,7 @@ struct SolveArgs {
   long long* k_out;
   double tol, atol;
   long long maxiter;
+  long long probe;     // > 0: the wait probe, cycles
 };
 
 // One level of a packed tree: value a goes on in the lanes without bit o, b in
@@ -525,10 +529,11 @@ struct SolveShared {
   double alpha, omega, beta;
   int stop, early;
   int late;  // a working warp's wait ran out
+  int off;   // an earlier solve of the step was aborted
 };
 
 __device__ __forceinline__ bool solve_late(const SolveArgs& a, bool& late, long long t0) {
-  if (clock64() - t0 < kSolveWaitCycles) return false;
+  if (clock64() - t0 < (a.probe > 0 ? a.probe : kSolveWaitCycles)) return false;
   atomicExch(&a.tail->abort, 1);
   late = true;
   return true;
@@ -554,6 +559,8 @@ __device__ __forceinline__ bool solve_reduce(const SolveArgs& a, SolveShared& sh
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((lane & 23) == 0 && vb < a.nb) post(part + vb, s, seq);
+    // the wait probe: a number that nothing posts
+    const unsigned long long awaited = a.probe > 0 ? ~0ull : seq;
     constexpr int kParts = kSolveBlocks / 32;
     static_assert(kParts >= 8 && kParts <= 16, "a thread of 256 takes one or two partials");
     double v[kParts];
@@ -564,7 +571,7 @@ __device__ __forceinline__ bool solve_reduce(const SolveArgs& a, SolveShared& sh
 #pragma unroll
       for (int w = 0; w < kParts; ++w) {
         v[w] = 0.0;
-        if (w * 32 + lane < a.nb) all &= posted(part + w * 32 + lane, seq, v[w]);
+        if (w * 32 + lane < a.nb) all &= posted(part + w * 32 + lane, awaited, v[w]);
       }
     } while (!__all_sync(0xffffffffu, all || solve_late(a, late, t0)));
 #pragma unroll
@@ -658,8 +665,12 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(const __grid_constan
   // off the critical path, and 19 warps leave a thread 96 registers
   __shared__ double x[kSolveCells][kSolveWork], rhat[kSolveCells][kSolveWork];
   const int lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) sh.late = 0;
+  if (threadIdx.x == 0) {
+    sh.late = 0;
+    sh.off = *(volatile const int*)&a.tail->abort;
+  }
   __syncthreads();
+  if (sh.off) return;
   if (threadIdx.x >= kSolveWork) {
     solve_wait(a, sh, (threadIdx.x - kSolveWork) >> 5, lane);
     return;
@@ -930,6 +941,7 @@ static int solve_resident(const Dims& d, const double* diag, double diag0, const
   a.tol = tol;
   a.atol = atol;
   a.maxiter = maxiter;
+  a.probe = g_probe_wait;
   cudaError_t e = cudaMemsetAsync(a.board, 0, sizeof(SolveBoard), s);
   if (e != cudaSuccess) return record_cuda(e);
   void* args[] = {&a};
@@ -1079,7 +1091,8 @@ __global__ void k_energy_jacobian(Dims d, EnergyK K, const double* U, const doub
 __global__ void k_copy(long long n, const double* a, double* b) {
   GRID_LOOP(c, n) b[c] = a[c];
 }
-__global__ void k_axpy(long long n, double* U, const double* inc) {
+__global__ void k_axpy(long long n, double* U, const double* inc, const SolveTail* tail) {
+  if (tail->abort) return;
   GRID_LOOP(c, n) U[c] = U[c] + inc[c];
 }
 __global__ void k_norm(const double* P, int nb, double* out) {
@@ -1191,7 +1204,8 @@ __global__ void k_pressure_rhs(Dims d, FlowK F, const double* velL, double* b, d
 // gradient of p (zero-gradient ghosts, cfd_am.py:82-91), projection and
 // pressure-gradient update written into the global arrays
 __global__ void k_project(Dims d, FlowK F, const double* p, const double* velL, double* vel,
-                          double* grad_p0, double ldz) {
+                          double* grad_p0, double ldz, const SolveTail* tail) {
+  if (tail->abort) return;
   const long long sx = (long long)d.ny * d.nz, sy = d.nz;
   GRID_LOOP(c, d.n) {
     int i, j, k;
@@ -1224,7 +1238,9 @@ __device__ __forceinline__ double upwind_face(double l2, double l1, double r1, d
 // div(f, vel_f) on the box for f = T and the three velocity components
 // (update_convective_terms, cfd_am.py:254-259), global cell size
 __global__ void k_convective(Dims d, FlowK F, double gdx, double gdy, double gdz, const double* T,
-                             const double* vel, double* conv_T, double* conv) {
+                             const double* vel, double* conv_T, double* conv,
+                             const SolveTail* tail) {
+  if (tail->abort) return;
   GRID_LOOP(c, d.n) {
     int i, j, k;
     ijk(d, c, i, j, k);
@@ -1375,7 +1391,7 @@ extern "C" int pfg_cfd_energy_solve(const pfg_cfd_grid* g, const pfg_cfd_energy*
     else
       st = krylov(d, w.vals, w.diag, w.b, w.x, 1e-5, 0.0, 10 * n, w, s, &k);
     if (st) return st;
-    k_axpy<<<nb, kThreads, 0, s>>>(n, T_out, w.x);
+    k_axpy<<<nb, kThreads, 0, s>>>(n, T_out, w.x, w.tail);
     k_energy_residual<<<nb, kThreads, 0, s>>>(d, K, T_out, T0, conv_T, w.b, w.P);
     k_norm<<<1, kThreads, 0, s>>>(w.P, nb, norm);
     ce = cudaGetLastError();
@@ -1463,9 +1479,9 @@ extern "C" int pfg_cfd_flow_step(const pfg_cfd_grid* global, const pfg_cfd_grid*
     st = krylov(d, w.vals, nullptr, w.b, w.x, 1e-10, 0.0, 10000, w, s, &h.k[3]);
   }
   if (st) return st;
-  k_project<<<nb, kThreads, 0, s>>>(d, F, w.x, w.velL, vel, grad_p0, local->dz);
+  k_project<<<nb, kThreads, 0, s>>>(d, F, w.x, w.velL, vel, grad_p0, local->dz, w.tail);
   k_convective<<<nb, kThreads, 0, s>>>(d, F, global->dx, global->dy, global->dz, T, vel, conv_T,
-                                       conv);
+                                       conv, w.tail);
   ce = cudaGetLastError();
   if (ce != cudaSuccess) return record_cuda(ce);
   if (resident) {  // the one host wait of the step

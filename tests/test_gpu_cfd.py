@@ -257,3 +257,57 @@ def test_am3d_solver_block_edges(N, NL, cells_per_thread):
                 assert ok, (N, NL, step, f, err, scale)
     finally:
         lib.pfg_tune(6, 0)
+
+
+def _box_case(N, NL, seed=0, **more):
+    """A solver on N cells with a box of NL, a melt pool and a flow in it."""
+    h = 5e-6
+    args = dict(CASES["surface"], P=60.0, speed=2.5,
+                X0=[0.3 * N[0] * h, 0.5 * N[1] * h, N[2] * h], **more)
+    s = gpu_solver(args, N, NL, h, (0.2441, 338.39, 300.0, 1563.0),
+                   (0.0163105, 4.5847, 300.0, 1563.0))
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x, y, z = torch.meshgrid(*((torch.arange(n, device="cuda", dtype=torch.float64) + 0.5) * h - b
+                               for n, b in zip(N, args["X0"])), indexing="ij")
+    w = 0.25 * N[1] * h
+    T = 300.0 + 2300.0 * torch.exp(-(x * x + y * y) / w ** 2 + 2.0 * z / w)
+    s.T.copy_(T[..., None])
+    s.vel.copy_(0.05 * torch.randn(s.vel.shape, generator=g, device="cuda", dtype=torch.float64) *
+                (T > 1623.0)[..., None])
+    return s
+
+
+def _fields(s):
+    return {f: getattr(s, f).clone() for f in FIELDS}
+
+
+def test_timed_out_solves_leave_the_fields():
+    """The wait probe makes the waits of the solves that run in one launch run
+    out (10 us): an error, fields as they were, and the next step without the
+    probe gives what a solver that never timed out gives.  In the second case
+    the energy solve takes the launches of each iteration, which wait for
+    nothing, so that the flow solves' waits run out."""
+    from jax_am_gb300 import _lib
+    lib = _lib.load()
+    for N, NL in (([24, 14, 9], [14, 9, 6]), ([120, 60, 50], [30, 20, 12])):
+        s, clean = _box_case(N, NL), _box_case(N, NL)
+        clean.time_integration()
+        before = _fields(s)
+        assert lib.pfg_tune(8, 20000) == 0
+        try:
+            with pytest.raises(_lib.PFGError, match="TIMEOUT"):
+                s.time_integration()
+            torch.cuda.synchronize()
+        finally:
+            assert lib.pfg_tune(8, 0) == 0
+        flow = ("vel", "conv_T", "conv", "grad_p0")
+        energy_done = N[0] == 120
+        for f in flow if energy_done else FIELDS:
+            assert torch.equal(getattr(s, f), before[f]), f
+        if energy_done:
+            assert torch.equal(s.T, clean.T)
+            s.T, s.solidID = before["T"], before["solidID"]
+        s.time_integration()
+        for f in FIELDS:
+            assert torch.equal(getattr(s, f), getattr(clean, f)), f
+        assert s.iterations() == clean.iterations()
