@@ -216,9 +216,12 @@ int pfg_device_error(int clear);
  * its copies in flight and returns; PFG_ERR_TIMEOUT in pfg_device_error)
  * without any fault; its output is then invalid, and the CFD solver's resident
  * solves wait that long for a partial sum that nothing posts (PFG_ERR_TIMEOUT
- * from the call).  Process-wide; the stencil
- * steps' results do not change; the CFD solver's dot products are summed in
- * another order (float64 rounding only). */
+ * from the call), 9 = the CFD solver's small systems (1: the launches of each
+ * iteration, as for large ones; 2: their one launch is asked for with more
+ * blocks than a device holds, which the call refuses, as a context with few
+ * SMs would, and the launches of each iteration follow).  Process-wide; the
+ * stencil steps' results do not change; key 6 makes the CFD solver sum its dot
+ * products in another order (float64 rounding only), key 9 does not. */
 int pfg_tune(int key, int value);
 
 /* The launch plan a step with these parameters would use on the current

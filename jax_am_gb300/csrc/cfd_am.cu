@@ -29,6 +29,7 @@
 
 namespace pfg {
 int g_cfd_cells_per_thread = 4;  // pfg_tune key 6
+int g_cfd_solves = 0;            // pfg_tune key 9: 1 never resident, 2 resident launches refused
 extern long long g_probe_wait;   // pfg_tune key 8
 
 namespace cfd {
@@ -908,10 +909,16 @@ static cudaGraphExec_t chunk_graph(const Dims& d, const double* vals, const doub
 // Above that the per-iteration launches are the better ones: the vectors no
 // longer fit the registers of one wave of blocks.
 static bool solve_fits(long long n) {
+  if (g_cfd_solves == 1) return false;
   const long long nb = nblocks(n);
   return nb <= std::min(2LL * device_info().sm_count, (long long)kSolveBlocks) &&
          n <= nb * kThreads * kSolveCells;
 }
+
+// The launch of k_solve was refused: fewer SMs than the device's may take it
+// (a partitioned context), or something else holds what a CTA needs on each.
+// The launches of each iteration run in any context.
+constexpr int kRefused = -1;
 
 // Enqueue k_solve: x = 0 start, k lands in tail->k[slot] (no host wait).
 static int solve_resident(const Dims& d, const double* diag, double diag0, const double* rows,
@@ -948,8 +955,14 @@ static int solve_resident(const Dims& d, const double* diag, double diag0, const
   const void* fn = rows ? (const void*)k_solve<true, true>
                    : dinv ? (const void*)k_solve<false, true>
                           : (const void*)k_solve<false, false>;
-  e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)((a.nb + 1) / 2)), dim3(kSolveThreads), args,
-                                  0, s);
+  // (key 9 = 2: a grid that no device holds at once, which the call refuses)
+  const unsigned blocks = (unsigned)((a.nb + 1) / 2) * (g_cfd_solves == 2 ? 4096u : 1u);
+  e = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kSolveThreads), args, 0, s);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported ||
+      e == cudaErrorLaunchOutOfResources) {
+    cudaGetLastError();
+    return kRefused;
+  }
   return e == cudaSuccess ? PFG_OK : record_cuda(e);
 }
 
@@ -1367,7 +1380,7 @@ extern "C" int pfg_cfd_energy_solve(const pfg_cfd_grid* g, const pfg_cfd_energy*
   K.Lz = g->lz;
   const int nb = nblocks(n);
   double* norm = &w.tail->norm;
-  const bool resident = solve_fits(n);
+  bool resident = solve_fits(n);
   cudaError_t ce = cudaMemsetAsync(w.tail, 0, sizeof(SolveTail), s);
   if (ce != cudaSuccess) return record_cuda(ce);
   k_copy<<<nb, kThreads, 0, s>>>(n, T0, T_out);
@@ -1385,11 +1398,12 @@ extern "C" int pfg_cfd_energy_solve(const pfg_cfd_grid* g, const pfg_cfd_energy*
   while (std::sqrt(bb) / res_init > e->newton_tol && it < e->max_newton) {
     k_energy_jacobian<<<nb, kThreads, 0, s>>>(d, K, T_out, T0, w.vals, w.diag);
     long long k = 0;
-    if (resident)
+    if (resident) {
       st = solve_resident(d, w.vals, 0.0, w.vals + n, nullptr, w.diag, w.b, w.x, 1e-5, 0.0, 10 * n,
                           w, 0, s);
-    else
-      st = krylov(d, w.vals, w.diag, w.b, w.x, 1e-5, 0.0, 10 * n, w, s, &k);
+      resident = st != kRefused;
+    }
+    if (!resident) st = krylov(d, w.vals, w.diag, w.b, w.x, 1e-5, 0.0, 10 * n, w, s, &k);
     if (st) return st;
     k_axpy<<<nb, kThreads, 0, s>>>(n, T_out, w.x, w.tail);
     k_energy_residual<<<nb, kThreads, 0, s>>>(d, K, T_out, T0, conv_T, w.b, w.P);
@@ -1448,7 +1462,7 @@ extern "C" int pfg_cfd_flow_step(const pfg_cfd_grid* global, const pfg_cfd_grid*
   F.ldx = local->dx;
   F.ldy = local->dy;
   const int nb = nblocks(nl);
-  const bool resident = solve_fits(nl);
+  bool resident = solve_fits(nl);
   // the neighbour coefficients are the same in every cell
   double off_m[6], off_p[6], diag_p = 0.0;
   for (int q = 0; q < 6; ++q) {
@@ -1459,22 +1473,42 @@ extern "C" int pfg_cfd_flow_step(const pfg_cfd_grid* global, const pfg_cfd_grid*
   cudaError_t ce = cudaMemsetAsync(w.tail, 0, sizeof(SolveTail), s);
   if (ce != cudaSuccess) return record_cuda(ce);
   SolveTail h{};
+  // What the resident solves left, on the host: the one wait of a step whose
+  // solves all are; before the first launch of an iteration otherwise.
+  auto solved = [&] {
+    ce = read_tail(w.tail, &h, s);
+    if (ce != cudaSuccess) return record_cuda(ce);
+    return h.abort ? (int)PFG_ERR_TIMEOUT : (int)PFG_OK;
+  };
   for (int comp = 0; comp < 3; ++comp) {
     double* u = w.velL + comp * nl;
-    k_momentum<<<nb, kThreads, 0, s>>>(d, F, comp, T, vel, conv, grad_p0, w.b, w.vals, w.diag,
-                                       !resident);
-    if (resident)
+    auto momentum = [&] {
+      k_momentum<<<nb, kThreads, 0, s>>>(d, F, comp, T, vel, conv, grad_p0, w.b, w.vals, w.diag,
+                                         !resident);
+    };
+    momentum();
+    if (resident) {
       st = solve_resident(d, w.vals, 0.0, nullptr, off_m, w.diag, w.b, u, 1e-10, 0.0, 10000, w,
                           comp, s);
-    else
-      st = krylov(d, w.vals, w.diag, w.b, u, 1e-10, 0.0, 10000, w, s, &h.k[comp]);
+      if (st == kRefused) {
+        if ((st = solved())) return st;
+        resident = false;
+        momentum();  // with the rows of neighbour coefficients
+      }
+    }
+    if (!resident) st = krylov(d, w.vals, w.diag, w.b, u, 1e-10, 0.0, 10000, w, s, &h.k[comp]);
     if (st) return st;
   }
   k_pressure_rhs<<<nb, kThreads, 0, s>>>(d, F, w.velL, w.b, local->dz);
   if (resident) {
     st = solve_resident(d, nullptr, diag_p, nullptr, off_p, nullptr, w.b, w.x, 1e-10, 0.0, 10000,
                         w, 3, s);
-  } else {
+    if (st == kRefused) {
+      if ((st = solved())) return st;
+      resident = false;
+    }
+  }
+  if (!resident) {
     k_pressure_vals<<<nb, kThreads, 0, s>>>(d, w.vals);
     st = krylov(d, w.vals, nullptr, w.b, w.x, 1e-10, 0.0, 10000, w, s, &h.k[3]);
   }
@@ -1484,11 +1518,7 @@ extern "C" int pfg_cfd_flow_step(const pfg_cfd_grid* global, const pfg_cfd_grid*
                                        conv, w.tail);
   ce = cudaGetLastError();
   if (ce != cudaSuccess) return record_cuda(ce);
-  if (resident) {  // the one host wait of the step
-    ce = read_tail(w.tail, &h, s);
-    if (ce != cudaSuccess) return record_cuda(ce);
-    if (h.abort) return PFG_ERR_TIMEOUT;
-  }
+  if (resident && (st = solved())) return st;
   if (stats) {
     for (int comp = 0; comp < 3; ++comp) stats->momentum_krylov[comp] = h.k[comp];
     stats->pressure_krylov = h.k[3];

@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(kThreads, 2) pf_warp_kernel(const __grid_const
 // ---------------------------------------------------------------------------
 
 extern int g_tma_consumers;
-extern int g_cfd_cells_per_thread;
+extern int g_cfd_cells_per_thread, g_cfd_solves;
 extern int g_fixed_plans;
 // Plan overrides for tuning sweeps (0 = automatic).
 static int g_tune_wx = 0, g_tune_rpw = 0, g_tune_stages = 0;
@@ -67,6 +67,8 @@ int set_tune(int key, int value) {
     case 7: if (value > 1) return PFG_ERR_PARAM;
             g_fixed_plans = value ? 0 : 1; return PFG_OK;
     case 8: g_probe_wait = value; return PFG_OK;
+    case 9: if (value > 2) return PFG_ERR_PARAM;
+            g_cfd_solves = value; return PFG_OK;
     default: return PFG_ERR_PARAM;
   }
 }

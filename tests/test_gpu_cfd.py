@@ -311,3 +311,59 @@ def test_timed_out_solves_leave_the_fields():
         for f in FIELDS:
             assert torch.equal(getattr(s, f), getattr(clean, f)), f
         assert s.iterations() == clean.iterations()
+
+
+@pytest.mark.parametrize("form", [1, 2], ids=["launches", "refused"])
+@pytest.mark.parametrize("N,NL", [([7, 5, 3], [5, 3, 2]), ([37, 19, 13], [23, 17, 11]),
+                                  ([60, 41, 15], [45, 31, 14]),
+                                  ([101, 60, 50], [96, 56, 50])])
+def test_both_forms_of_a_solve_agree(N, NL, form):
+    """Two steps with the solves in one launch each (pfg_tune key 9 = 0) and in
+    five launches an iteration, asked for (1) or because the one launch is
+    refused (2): the same fields bit for bit and the same iteration counts, for
+    systems of one 256-thread block to more than 256 (303,000 and 268,800
+    cells)."""
+    from jax_am_gb300 import _lib
+    lib = _lib.load()
+    a, b = _box_case(N, NL), _box_case(N, NL)
+    for _ in range(2):
+        a.time_integration()
+        assert lib.pfg_tune(9, form) == 0
+        try:
+            b.time_integration()
+        finally:
+            assert lib.pfg_tune(9, 0) == 0
+        assert a.iterations() == b.iterations()
+        for f in FIELDS:
+            assert torch.equal(getattr(a, f), getattr(b, f)), f
+    assert a.iterations()["pressure_krylov"] > 2 and float(a.vel.abs().max()) > 1e-4
+
+
+def test_solves_of_several_threads():
+    """Two threads with a stream each, their solves' launches wanting every SM:
+    each gives what it gives alone."""
+    import threading
+    N, NL = [101, 60, 50], [96, 56, 50]
+    alone = [_box_case(N, NL, seed=k) for k in range(2)]
+    for s in alone:
+        s.time_integration()
+    both = [_box_case(N, NL, seed=k) for k in range(2)]
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(s):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                s.time_integration()
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(s,)) for s in both]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for s, r in zip(both, alone):
+        for f in FIELDS:
+            assert torch.equal(getattr(s, f), getattr(r, f)), f
