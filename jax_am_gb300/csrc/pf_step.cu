@@ -360,9 +360,6 @@ HeatDF make_heat_df(const pfg_heat_params& h, float dt) {
   HeatDF d;
   d.k1 = df_split(0.0163);
   d.k0 = df_split(4.5847);
-  d.c1 = df_split(0.2441);
-  d.c0 = df_split(338.39);
-  d.latent = df_split((double)h.latent);
   const double r = (double)h.beam_radius;
   d.beam_coef = df_split(2.0 * (double)h.absorptivity / 3.14159265358979323846 / (r * r));
   d.two_over_r2 = df_split(2.0 / (r * r));

@@ -50,13 +50,6 @@ __device__ __forceinline__ DF df_add(DF x, DF y) {
   s.l += t.l;
   return fast_two_sum(s.h, s.l);
 }
-// The same sum with the low parts added in float32 (error below 2^-46 of the
-// larger operand, not of a cancelled result): 11 operations instead of 20.
-__device__ __forceinline__ DF df_add_fast(DF x, DF y) {
-  DF s = two_sum(x.h, y.h);
-  s.l += x.l + y.l;
-  return fast_two_sum(s.h, s.l);
-}
 __device__ __forceinline__ DF df_add_f(DF x, float b) {
   DF s = two_sum(x.h, b);
   s.l += x.l;
@@ -85,15 +78,17 @@ __device__ __forceinline__ DF df_div(DF x, DF y) {
   return df_add_f(q, __fdiv_rn(r2.h, y.h));
 }
 
-// x / y from two quotient digits, each off the approximate reciprocal of y.h
-// (the first remainder is exact): relative error about 2^-44, 13 operations
-// and one reciprocal instead of three float32 divisions and two remainders.
-// Operands in the normal range.
-__device__ __forceinline__ DF df_div_fast(DF x, DF y, float rcp_yh) {
+// x / y from three quotient digits off one approximate reciprocal of y.h (within
+// an ulp): each digit's remainder of the leading parts is exact, so the third
+// digit leaves the pair's own rounding.  About 25 operations against 75 for
+// df_div and its three IEEE quotients.  Operands in the normal range.
+__device__ __forceinline__ DF df_div_rcp(DF x, DF y, float rcp_yh) {
   const float q1 = x.h * rcp_yh;
-  const DF p = two_prod(q1, y.h);
-  const float rem = ((x.h - p.h) - p.l) + fmaf(-q1, y.l, x.l);
-  return fast_two_sum(q1, rem * rcp_yh);
+  const DF r = two_sum(fmaf(-q1, y.h, x.h), fmaf(-q1, y.l, x.l));
+  const float q2 = r.h * rcp_yh;
+  const float r2 = fmaf(-q2, y.h, r.h) + fmaf(-q2, y.l, r.l);
+  const DF q = fast_two_sum(q1, q2);
+  return fast_two_sum(q.h, fmaf(r2, rcp_yh, q.l));
 }
 
 // x > c and x < c for a float c (h + l compared exactly: |l| <= ulp(h) / 2)

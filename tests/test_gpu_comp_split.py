@@ -86,3 +86,119 @@ def test_multi_track_n30_long_run():
                            compensated=True)
     assert Tmax >= T_LIQ, f"the laser never melted the surface (T max {Tmax:.1f} K)"
     torch.cuda.empty_cache()
+
+
+# ---- one step's rounding -----------------------------------------------------
+# Pair arithmetic in which every sum, difference, product and quotient is a
+# normalised pair of its own, in NumPy float32 (a fused multiply-add is the
+# longdouble value rounded once).
+_f, _L = np.float32, np.longdouble
+
+
+def _two_sum(a, b):
+    s = a + b
+    bb = s - a
+    return s, (a - (s - bb)) + (b - bb)
+
+
+def _fast(a, b):
+    s = a + b
+    return s, b - (s - a)
+
+
+def _fma(a, b, c):
+    return (_L(a) * _L(b) + _L(c)).astype(_f)
+
+
+def _add(x, y):
+    s, e = _two_sum(x[0], y[0])
+    t, u = _two_sum(x[1], y[1])
+    s, e = _fast(s, e + t)
+    return _fast(s, e + u)
+
+
+def _sub(x, y):
+    return _add(x, (-y[0], -y[1]))
+
+
+def _mul(x, y):
+    p = x[0] * y[0]
+    return _fast(p, _fma(x[0], y[1], _fma(x[1], y[0], _fma(x[0], y[0], -p))))
+
+
+def _div(x, y):
+    z = np.zeros_like(x[0])
+    q1 = x[0] / y[0]
+    r = _sub(x, _mul(y, (q1, z)))
+    q = _fast(q1, r[0] / y[0])
+    r = _sub(x, _mul(y, q))
+    return _add(q, (r[0] / y[0], z))
+
+
+def _pair(v, like=None):
+    v = np.asarray(v, dtype=np.float64)
+    h = v.astype(_f)
+    p = h, (v - h).astype(_f)
+    return p if like is None else tuple(np.broadcast_to(a, like.shape).astype(_f) for a in p)
+
+
+@pytest.mark.parametrize("n", [20, 12], ids=["lane", "split"])
+@pytest.mark.parametrize("lo,hi", [(400.0, 1540.0), (1575.0, 1610.0), (1640.0, 3000.0),
+                                   (3000.0, 9000.0)])
+def test_compensated_step_rounds_as_full_pairs(n, lo, hi):
+    """One compensated heat step of random temperature pairs against extended
+    precision: the root mean square and the largest error of the cells away from
+    the faces are those of full pair arithmetic on the same values (2 % and a
+    quarter for the sample's spread; low parts summed in float32 add a fifth to
+    the former)."""
+    from jax_am_gb300.phase_field.allen_cahn import PFSolver
+    from jax_am_gb300.runner import HeatPFRun, single_track
+    from tests.cases import GAMMA_DEFAULTS, pf_case
+    nx, ny, nz = 96, 64, 48
+    hx, dt = float(_f(1e-6)), float(_f(2e-8))
+    poly, eta, _, pf_args, _, _ = pf_case((nx, ny, nz), n, 0.0, seed=4, h=(hx,) * 3)
+    g = dict(GAMMA_DEFAULTS)
+    rng = np.random.default_rng(int(lo) + n)
+    base = rng.uniform(lo, hi, (nz // 8 + 1, ny // 8 + 1, nx // 8 + 1))
+    T = np.kron(base, np.ones((8, 8, 8)))[: nz + 2, : ny + 2, : nx + 2]
+    T = T + rng.uniform(-10.0, 10.0, T.shape)
+    h, l = _pair(T)
+    run = HeatPFRun(PFSolver(pf_args, poly), g, single_track(1e-6, 2e-6, 0.8, 0.0, 1.0), dt=dt,
+                    eta0=torch.tensor(eta, dtype=torch.float32, device="cuda"),
+                    T_init=torch.tensor(h), compensated=True)
+    run.Tl[run.cur].copy_(torch.tensor(l))
+    run.run(1, graph=False)
+    got = run.T_ghosted_f64.cpu().numpy()[2:-2, 2:-2, 2:-2]
+
+    def at(a, d=(0, 0, 0)):
+        return a[tuple(slice(2 + k, m - 2 + k) for k, m in zip(d, a.shape))]
+    dirs = [(0, 0, 1), (0, 1, 0), (1, 0, 0)]
+    rho, L, Ts, Tl = (float(_f(g[k])) for k in ("rho", "L", "Ts", "Tl"))
+    x = _L(h) + _L(l)
+    c = at(x)
+    clip = np.clip(c, 300.0, _L(Tl))
+    k = _L(0.0163) * clip + _L(4.5847)
+    cp = _L(0.2441) * clip + _L(338.39) + np.where((c > Ts) & (c < Tl), _L(L), _L(0))
+    lap = sum((at(x, d) - c) + (at(x, tuple(-v for v in d)) - c) for d in dirs) / (_L(hx) * _L(hx))
+    exact = c + k * _L(dt) / (cp * _L(rho)) * lap
+
+    C = at(h), at(l)
+    z = np.zeros_like(C[0])
+    cl = tuple(np.where(clip == c, v, w) for v, w in zip(C, (clip.astype(_f), z)))
+    kk = _add(_mul(_pair(0.0163, z), cl), _pair(4.5847, z))
+    cc = _add(_mul(_pair(0.2441, z), cl), _pair(338.39, z))
+    cm = _add(cc, _pair(L, z))
+    cc = tuple(np.where((c > Ts) & (c < Tl), a, b) for a, b in zip(cm, cc))
+    ll = z, z
+    for d in dirs:
+        m, p = ((at(h, e), at(l, e)) for e in (tuple(-v for v in d), d))
+        ll = _add(ll, _mul(_add(_sub(m, C), _sub(p, C)), _pair(1.0 / (hx * hx), z)))
+    coef = _div(_mul(kk, (np.full_like(z, dt), z)), _mul(cc, (np.full_like(z, rho), z)))
+    full = _add(C, _mul(coef, ll))
+    e_full = np.abs((_L(full[0]) + _L(full[1]) - exact).astype(np.float64))
+    e_got = np.abs((_L(got) - exact).astype(np.float64))
+    rms = [float(np.sqrt(np.mean(e * e))) for e in (e_got, e_full)]
+    print(f"n = {n}, {lo} .. {hi} K: rms {rms[0]:.3e} (full pairs {rms[1]:.3e}), largest "
+          f"{e_got.max():.3e} ({e_full.max():.3e}) K")
+    assert rms[0] <= 1.02 * rms[1]
+    assert e_got.max() <= 1.25 * e_full.max()
