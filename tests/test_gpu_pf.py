@@ -363,3 +363,34 @@ def test_start_by_value_matches_device_clock(shape, n, source):
     torch.cuda.synchronize()
     assert int(clk[1, 1]) == step + 1
     assert float(clk[1, :1].view(torch.float64)) == t + float(np.float32((t + dt) - t))
+
+
+@pytest.mark.parametrize("source", ["array", "quench"])
+def test_warp_kernel_on_the_largest_odd_grid(source):
+    """125 x 90 x 60 cells, n = 30: odd nx with 8-byte vectors, so the
+    warp-per-cells kernel, 560 units of 16 x 9 tiles and nine planes; against
+    the generic kernel as above."""
+    from jax_am_gb300 import _lib
+    from jax_am_gb300.phase_field.allen_cahn import Quench
+    lib = _lib.load()
+    shape, n = (125, 90, 60), 30
+    poly, _, _, pf_args, _, _ = pf_case((2, 2, 2), n, 0.15, seed=n)
+    s = _solver(dict(pf_args, Nx=shape[0], Ny=shape[1], Nz=shape[2]), poly)
+    plan = _lib.describe_plan(s.params)
+    assert (plan["kernel"], plan["vec"], plan["tile_x"], plan["tile_y"]) == (2, 2, 16, 9), plan
+    g = torch.Generator(device="cuda").manual_seed(n)
+    eta = torch.rand((s.N, n), generator=g, device="cuda")
+    T = 1400.0 + 700.0 * torch.rand(s.N, generator=g, device="cuda")
+    if source == "quench":
+        T = Quench(1623.0, 5e6, 0.1, z0=3e-5)
+    outs = []
+    for v in (0, 1):
+        lib.pfg_set_kernel_variant(v)
+        state, t = (eta, 0.0), 0.0
+        for _ in range(4):
+            t += 1e-8
+            state, _ = s.stepper(state, t, [T])
+        outs.append(state[0])
+    lib.pfg_set_kernel_variant(0)
+    assert float((outs[0] - outs[1]).abs().max()) <= 1e-5
+    assert _lib.device_error() == 0
