@@ -99,9 +99,8 @@ def update_T(T, xl, yl, x, y, P, dx, dy, dz, dt, gamma_args, out=None):
     step = lib.pfg_heat_step
     if out is None:  # edge/corner ghosts are carried over unchanged
         out, step = torch.empty_like(T), lib.pfg_heat_step_whole
-    st = step(ctypes.byref(h), _lib.ptr(T), _lib.ptr(out), float(xl), float(yl),
-                           float(P), float(dt),
-                           ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    st = step(ctypes.byref(h), _lib.ptr(T), _lib.ptr(out), float(xl), float(yl), float(P),
+              float(dt), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
     _lib.check(st, "pfg_heat_step")
     return out
 

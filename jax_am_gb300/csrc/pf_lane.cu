@@ -64,14 +64,6 @@ __device__ __forceinline__ float add_squares(F2 u, float s) {
   return fmaf(f2_lo(u), f2_lo(u), fmaf(f2_hi(u), f2_hi(u), s));
 }
 
-// Per-cell folded coefficients from the temperature part and S.
-__device__ __forceinline__ float4 lane_fold(const PFConsts& c, const TempCoef& tc, float S) {
-  if (tc.liquid != 0.f) return make_float4(0.f, 0.f, 0.f, 0.f);
-  const float K = 4.f * S + tc.om2 - 1.f;
-  const float clw = tc.cl * c.wx;
-  return make_float4(1.f + tc.cg * K, -3.f * tc.cg, clw * (1.f + c.aniso), 2.f * c.aniso * clw);
-}
-
 // A vector of VP pairs (16 or 8 bytes).
 template <int VP>
 __device__ __forceinline__ void load_pairs(F2* v, const float* p) {
@@ -438,7 +430,7 @@ pf_lane_kernel(const __grid_constant__ StepArgs a) {
       TempCoef tcf;
       if constexpr (COMP) tcf = temp_coefficients_pair(a.pc, Tcell, Lc, a.dt);
       else tcf = temp_coefficients_fast(a.pc, Tcell, a.dt);
-      const float4 k = lane_fold(a.pc, tcf, s_a + s_b);
+      const float4 k = pair_fold(a.pc, tcf, s_a + s_b);
       // the skip below needs finite coefficients in every cell of the warp
       const bool kfinite = __all_sync(0xffffffffu, !valid || (isfinite(k.x) && isfinite(k.y) &&
                                                                isfinite(k.z) && isfinite(k.w)));

@@ -709,7 +709,9 @@ extern "C" int pfg_pf_step_interp_at(const pfg_pf_params* p, const pfg_interp* w
   return step_from<kTInterp>(a, p, eta_in, eta_out, nullptr, nullptr, pfg_clock{t, 0}, dt, stream);
 }
 
+namespace pfg {
 __global__ void clock_set_kernel(pfg_clock* clk, pfg_clock v) { *clk = v; }
+}  // namespace pfg
 
 extern "C" int pfg_clock_set(pfg_clock* clk, double t, int64_t step, void* stream) {
   if (!clk) return PFG_ERR_NULL;

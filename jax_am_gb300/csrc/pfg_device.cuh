@@ -251,6 +251,13 @@ struct CoefPair {
 __device__ __forceinline__ CoefPair coef_pair(const float4& k) {
   return CoefPair{f2_pack(k.x, k.x), f2_pack(k.y, k.y), f2_pack(k.z, k.z), f2_pack(k.w, k.w)};
 }
+// Its per-cell coefficients from the temperature part and S.
+__device__ __forceinline__ float4 pair_fold(const PFConsts& c, const TempCoef& tc, float S) {
+  if (tc.liquid != 0.f) return make_float4(0.f, 0.f, 0.f, 0.f);
+  const float K = 4.f * S + tc.om2 - 1.f;
+  const float clw = tc.cl * c.wx;
+  return make_float4(1.f + tc.cg * K, -3.f * tc.cg, clw * (1.f + c.aniso), 2.f * c.aniso * clw);
+}
 template <bool ANISO, class Dot>
 __device__ __forceinline__ F2 elem_pair(const LapPair& L, F2 e, F2 xm, F2 xp, F2 ym, F2 yp, F2 zm,
                                         F2 zp, const CoefPair& k, Dot&& dot) {

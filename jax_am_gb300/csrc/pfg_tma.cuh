@@ -25,14 +25,6 @@ __device__ __forceinline__ bool tma_wait(uint64_t* bar, unsigned parity, int* er
   return false;
 }
 
-// Per-cell folded coefficients (see elem_pair).
-__device__ __forceinline__ float4 tma_fold(const PFConsts& c, const TempCoef& tc, float S) {
-  if (tc.liquid != 0.f) return make_float4(0.f, 0.f, 0.f, 0.f);
-  const float K = 4.f * S + tc.om2 - 1.f;
-  const float clw = tc.cl * c.wx;
-  return make_float4(1.f + tc.cg * K, -3.f * tc.cg, clw * (1.f + c.aniso), 2.f * c.aniso * clw);
-}
-
 // NC threads (256: two CTAs per SM, or 512: one CTA per SM with a tile
 // twice as large).  VEC = 4 when num_oris % 4 == 0 (a cell is whole 16-byte
 // vectors); VEC = 2 for other even num_oris with an even nx, even tile
@@ -354,7 +346,7 @@ __device__ __forceinline__ void tma_unit(const StepArgs& a, int unit, const floa
                     : temp_coefficients_fast(a.pc, ts[c_toff[q]], a.dt);
       }
       else tc = temp_coefficients_fast(a.pc, ts[c_toff[q]], a.dt);
-      cb[c_cc[q]] = tma_fold(a.pc, tc, s0 + s1);
+      cb[c_cc[q]] = pair_fold(a.pc, tc, s0 + s1);
     }
     if (pz + 1 < ze) load_lo(pz + 1);
   };

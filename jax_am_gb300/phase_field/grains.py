@@ -53,34 +53,6 @@ def _cell_volume(pf_args):
     return hx * hy * hz
 
 
-def aspect_ratios(records):
-    """Aspect ratios of grains given as (cells, sums, sums2) records of their
-    integer moments: the covariance of the cell centres (ddof = 1, exact
-    integer numerators), its eigenvalues in descending order, 2 sqrt(ev0) /
-    (sqrt(ev1) + sqrt(ev2)); 1 below 5 cells (utils.py:286-310).  Cell-centre
-    scaling (h, the volume weights) cancels.  ``segment_grains`` takes them from
-    the GPU (``pfg_grain_shapes``)."""
-    ar = np.ones(len(records))
-    big = [k for k in range(len(records)) if records[k][0] >= 5]
-    if not big:
-        return ar
-    cov = np.zeros((len(big), 3, 3))
-    pairs = ((0, 0, 0), (1, 1, 1), (2, 2, 2), (0, 1, 3), (0, 2, 4), (1, 2, 5))
-    for j, k in enumerate(big):
-        c, s, s2 = records[k]
-        c = int(c)
-        den = c * (c - 1)
-        for a, b, m in pairs:
-            # exact: (c * sum(ab) - sum(a) sum(b)) / (c (c - 1)), big Python ints
-            v = (c * int(s2[m]) - int(s[a]) * int(s[b])) / den
-            cov[j, a, b] = cov[j, b, a] = v
-    ev = np.linalg.eigvalsh(cov)[:, ::-1]
-    ln = np.sqrt(np.maximum(ev, 0.0))
-    with np.errstate(divide="ignore", invalid="ignore"):
-        ar[big] = 2.0 * ln[:, 0] / (ln[:, 1] + ln[:, 2])
-    return ar
-
-
 _FIRST_ROWS = 4096  # grains that the first copy to the host has room for
 
 
