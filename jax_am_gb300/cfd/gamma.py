@@ -46,18 +46,21 @@ def make_heat_params(gamma_args, nx, ny, nz, dx, dy, dz, x_first=None, y_first=N
 
 
 # The coordinates of the last call that were found uniform and their first
-# centre: (weak references to x and y, what was checked, (x_first, y_first)).
-# One entry, replaced as a whole.
+# centre: (weak references to x and y, extents and spacings, what x and y held,
+# (x_first, y_first)).  One entry, replaced as a whole.
 _checked = None
 
 
 def _contents(a):
     """What tells whether an array that was looked at before still holds the
-    same coordinates: a CUDA tensor's storage and version counter (no copy to
+    same coordinates: a CUDA tensor's version counter and storage (no copy to
     the host), otherwise the corners of its top plane."""
-    if torch.is_tensor(a) and a.is_cuda and not a.is_inference():
-        return a.data_ptr(), a._version, a.dtype, a.shape, a.stride()
-    return tuple(a.shape), [float(a[i, i, -1]) for i in (0, -1)]
+    if torch.is_tensor(a) and a.is_cuda:
+        try:
+            return a._version, a.data_ptr(), a.shape, a.stride()
+        except RuntimeError:  # an inference tensor has no version counter
+            pass
+    return a.shape, float(a[0, 0, -1]), float(a[-1, -1, -1])
 
 
 def _first_centre(x, y, nx, ny, dx, dy):
@@ -66,11 +69,12 @@ def _first_centre(x, y, nx, ny, dx, dy):
     is kept for the next call -- for the same objects (not the same ids: a
     freed array's id is given to another), contents, extents and spacings."""
     global _checked
+    grid, last = (nx, ny, dx, dy), _checked
+    if (last is not None and last[0]() is x and last[1]() is y and last[2] == grid
+            and last[3] == _contents(x) and last[4] == _contents(y)):
+        return last[5]
     x, y = (a if torch.is_tensor(a) else np.asarray(a) for a in (x, y))
-    key = (nx, ny, dx, dy, _contents(x), _contents(y))
-    last = _checked
-    if last is not None and last[0]() is x and last[1]() is y and last[2] == key:
-        return last[3]
+    held = _contents(x), _contents(y)
     xt, yt = (a[:, :, -1].detach().cpu().numpy() if torch.is_tensor(a) else a[:, :, -1]
               for a in (x, y))
     ex = xt[0, 0] + dx * np.arange(nx)[:, None]
@@ -79,7 +83,7 @@ def _first_centre(x, y, nx, ny, dx, dy):
                                                                       atol=1e-12)):
         raise ValueError("x and y must be uniform cell-centre grids with spacing dx, dy")
     first = (float(xt[0, 0]), float(yt[0, 0]))
-    _checked = (weakref.ref(x), weakref.ref(y), key, first)
+    _checked = (weakref.ref(x), weakref.ref(y), grid, *held, first)
     return first
 
 
