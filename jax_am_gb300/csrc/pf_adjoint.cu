@@ -562,11 +562,15 @@ __global__ void __launch_bounds__(256) adj_heat_kernel(const __grid_constant__ A
 // (1M cells, n = 10: 28 us a launch; with conversions 46, with a product and a
 // weight an element 85).
 
-// |v| as a double, of a value that is zero or normal: the exponent's bias and
-// place change.
-__device__ __forceinline__ double widened_abs(unsigned m) {
-  return __hiloint2double((int)((m >> 3) + (m ? 0x38000000u : 0u)), (int)(m << 29));
+// |v| as a double, of a finite value: the exponent's bias and place change.  Far
+// fields are full of denormals, which are scaled by 2^64 first.
+__device__ __forceinline__ double widened_abs(float v) {
+  const bool tiny = fabsf(v) < 1e-30f;
+  const unsigned m = __float_as_uint(fabsf(tiny ? v * 0x1p64f : v));
+  const unsigned bias = m == 0u ? 0u : tiny ? 0x34000000u : 0x38000000u;
+  return __hiloint2double((int)((m >> 3) + bias), (int)(m << 29));
 }
+
 template <bool SEED>
 __global__ void __launch_bounds__(256)
 objective_kernel(const float* __restrict__ eta, const float* __restrict__ w, long long ncell, int n,
@@ -578,13 +582,12 @@ objective_kernel(const float* __restrict__ eta, const float* __restrict__ w, lon
   double sum = 0.0;
   if (first < stride && first < total) {
     const float wi = __ldg(w + (int)(first % n));
-    bool other = false;  // a denormal, infinite or NaN value
+    bool other = false;  // an infinite or NaN value
 #pragma unroll 4
     for (long long e = first; e < total; e += stride) {
       const float v = __ldg(eta + e);
-      const unsigned m = __float_as_uint(v) & 0x7fffffffu;
-      other |= m - 1u < 0x007fffffu || m >= 0x7f800000u;
-      const double d = widened_abs(m);
+      other |= !isfinite(v);
+      const double d = widened_abs(v);
       sum = fma(d, d, sum);
       if (SEED) lam[e] = 2.f * wi * v * inv;
     }

@@ -169,7 +169,7 @@ def test_objective_in_float64(shape, n):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     threads = min(N * n, sms * 8 * 256) // 2
     roundings = N * n / max(1, threads) + 16 + 8 * sms
-    for scale in (1.0, 1e18, 1e25, 1e-25):
+    for scale in (1.0, 1e18, 1e25, 1e-25, 1e-37):
         x = f32(eta * scale)
         J, lam = J_of(x)
         terms = (w * x * x).reshape(-1)
