@@ -753,9 +753,13 @@ pf_diag_cells_kernel(const __grid_constant__ DiagArgs a) {
   }
 }
 
+// Dynamic shared memory up to which a launch needs no attribute: 48 KB less room
+// for the kernels' static arrays.
+constexpr size_t kPlainSmem = 44 * 1024;
+
 template <int NV>
 static cudaError_t launch_diag_cells_t(const DiagArgs& a, int nb, size_t smem, cudaStream_t s) {
-  if (smem > 48 * 1024) {
+  if (smem > kPlainSmem) {
     cudaError_t e = cudaFuncSetAttribute(pf_diag_cells_kernel<NV>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -810,7 +814,7 @@ int launch_diag(const pfg_pf_params* p, const float* eta, const float* T, int T_
     const size_t smem = (size_t)w * 32 * a.n * sizeof(float);
     const void* fn = (a.n % 4 == 0) ? (const void*)pf_inspect_kernel<true>
                                     : (const void*)pf_inspect_kernel<false>;
-    if (smem > 48 * 1024) {
+    if (smem > kPlainSmem) {
       cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem);
       if (e != cudaSuccess) return record_cuda(e);

@@ -171,3 +171,28 @@ def test_diag_non_finite_values(n):
     m = O.inspect(np.nan_to_num(eta), eta, T, oargs["T_liquidus"])
     assert d["max_T"] == m["max_T"]
 
+
+@pytest.mark.parametrize("n", [4, 8, 11, 12, 13, 20, 24, 64])
+def test_first_call_of_a_process(n):
+    """The records of a process's first call, when no larger launch has raised
+    the kernels' shared-memory limit (12 orientations take exactly 48 KB
+    beside the static arrays)."""
+    import os
+    import subprocess
+    import sys
+    code = f"""
+import torch
+from tests.cases import pf_case
+from jax_am_gb300.phase_field.allen_cahn import PFSolver
+poly, eta, T, a, _, _ = pf_case((40, 30, 20), {n}, 0.15, seed=1)
+s = PFSolver(a, poly)
+e = torch.tensor(eta, dtype=torch.float32, device="cuda")
+Td = torch.tensor(T, dtype=torch.float32, device="cuda")
+i, d = s.inspect(e, Td, e), s.diagnostics(e, Td, e)
+assert torch.equal(s.argmax(e).long(), e.argmax(1))
+assert i["n_liquid"] == d["n_liquid"] == int((T >= 1623.0).sum())
+assert i["n_ori_changed"] == d["n_ori_changed"] == i["n_nonfinite"] == 0
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
